@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "internal.h"
 
 #include "devmath.cuh"
@@ -95,6 +97,27 @@ __device__ __forceinline__ void fast_bounds_of(const FrameConst& f, float3 g0, f
     }
 }
 
+// ---------------------------------------------------------------- fast decisions (GPS): position bound
+// gps_fast computes a particle's image position with the MUFU forms. r = sqrt(-2 log(1 - u1)) is
+// within kErMax of the exact path's (checked over every uniform); the radius table is continuous
+// and piecewise linear in w = r 128 / (4.123 sqrt 2), its largest step 0.04874 <= kLutSlope, and w is
+// within 1.3e-4 (kErMax and the roundings of both paths at w <= 127), so the radius is within
+// kLutSlope 1.3e-4 + 4e-6 (the interpolation's roundings in both paths); times sine or cosine, with
+// radii up to 5.84, within kGpsEw.
+constexpr float kLutSlope = 0.049f;
+constexpr float kGpsEw = kLutSlope * 1.3e-4f + 4e-6f + 5.84f * (kSinCos + 2.0f * kU) + 6e-7f;
+constexpr float kCellBias = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest whole number
+// Half a subpixel minus the bound of |position - exact position| in subpixels, along x and y; a
+// sample nearer than that to a subpixel edge is undecided. Per unit of the factor's row sum S:
+// kGpsEw and the products' roundings (below 6e-6); the sums' roundings at the magnitude of the
+// mean and of the grid coordinate; 2e-6 for the subpixel arithmetic.
+__device__ __forceinline__ float2 gps_limits(const FrameConst& f, float mx, float my, float l00, float l10, float l11) {
+    const float side = (float)f.side, sx = fabsf(l00), sy = fabsf(l10) + fabsf(l11);
+    const float ex = (sx * (kGpsEw + 6e-6f) + F_(3e-7) * fabsf(mx)) * side * F_(1.02) + F_(2e-6);
+    const float ey = (sy * (kGpsEw + 6e-6f) + F_(3e-7) * fabsf(my)) * side * F_(1.02) + F_(2e-6);
+    return make_float2(F_(0.5) - ex, F_(0.5) - ey);  // not positive, or NaN: never decides
+}
+
 // ============================================================================ geometry
 // Once per camera: projection, opacity clamp, per-method count descriptor and particle record,
 // and the view-dependent SH colour (prepare/prepare_gps/prepare_pbvr without the seed-dependent
@@ -133,6 +156,8 @@ __global__ void __launch_bounds__(128) k_geometry(FrameConst f, const float4* __
                 R[0] = r0;
                 R[1] = make_float4(l00, l10, l11, a);
                 R[2] = make_float4(__uint_as_float(i0), li2, F_(0.0), F_(0.0));
+                const float2 lim = gps_limits(f, pr.mx, pr.my, l00, l10, l11);
+                R[3] = make_float4(lim.x, lim.y, F_(0.0), F_(0.0));
             }
         } else if (method == 0u) {
             // footprint-subpixel mode (render_monte_carlo, oracle.rs:240-310): footprint s per splat
@@ -199,7 +224,7 @@ __global__ void __launch_bounds__(128) k_geometry(FrameConst f, const float4* __
                     R[0] = r0;
                     R[1] = make_float4(lo_x, lo_y, sz_x, sz_y);
                     R[2] = make_float4(pr.c * invdet, -pr.b * invdet, pr.a * invdet, peak_tau);
-                    R[3] = make_float4(F_(0.0), F_(0.0), F_(0.0), sparse ? F_(1.0) : F_(0.0));
+                    R[3] = make_float4(__uint_as_float(0xFFFFFFFFu / f2u(sz_x)), F_(0.0), F_(0.0), sparse ? F_(1.0) : F_(0.0));
                 }
             }
         } else {
@@ -474,23 +499,41 @@ __device__ __forceinline__ void splat_write(ull* sub, uint32_t idx, float depth_
     if (packed < cur) atomicMin(sub + idx, packed);
 }
 
-// emit_particle (gps_splat.wgsl:259-282) with the packed winner rule
-__device__ __forceinline__ uint32_t emit_gps(const FrameConst& f, const FTabs& T, const float* lut, uint32_t i, uint32_t& rs,
-                                             float4 r0, float4 r1, float4 r2, ull* sub) {
+constexpr uint32_t kNoCell = 0xFFFFFFFFu;  // "not written" of the locate functions
+
+// emit_particle (gps_splat.wgsl:259-282): the image position of a GPS particle, its random numbers
+// taken from rs (kIter: the iterated radius and footprint blocks may be asked for)
+template <bool kIter>
+__device__ __forceinline__ float2 gps_position(const FrameConst& f, const FTabs& T, const float* lut, uint32_t& rs, float4 r0,
+                                               float4 r1, float4 r2) {
     float u = gx::next_u(&rs);
-    float r = f.exact_radius ? corrected_radius_exact(r0.w, r2.y, u)
-                             : corrected_radius_lut(lut, __float_as_uint(r2.x), r1.w, u, T.lg);
+    float r = kIter && f.exact_radius ? corrected_radius_exact(r0.w, r2.y, u)
+                                      : corrected_radius_lut(lut, __float_as_uint(r2.x), r1.w, u, T.lg);
     float th = gxc::kTwoPi * gx::next_u(&rs);
     float sn, cs;
     gx::sincos_t(th, T.sc, &sn, &cs);
     float wx = r * cs, wy = r * sn;
-    float px_ = r0.x + r1.x * wx;
-    float py_ = r0.y + (r1.y * wx + r1.z * wy);
-    if (r2.z > F_(1.0)) {
+    return make_float2(r0.x + r1.x * wx, r0.y + (r1.y * wx + r1.z * wy));
+}
+// subpixel of an image position, kNoCell off screen
+__device__ __forceinline__ uint32_t subpixel_of(const FrameConst& f, float2 q) {
+    if (q.x < F_(0.0) || q.x >= (float)f.W || q.y < F_(0.0) || q.y >= (float)f.H) return kNoCell;
+    uint32_t px = f2u(q.x), py = f2u(q.y);
+    uint32_t sx = min(f.side - 1u, f2u((q.x - (float)px) * (float)f.side));
+    uint32_t sy = min(f.side - 1u, f2u((q.y - (float)py) * (float)f.side));
+    return (py * f.W + px) * f.S + sy * f.side + sx;
+}
+
+// a GPS particle with the packed winner rule; returns whether it was written
+template <bool kIter = true>
+__device__ __forceinline__ uint32_t emit_gps(const FrameConst& f, const FTabs& T, const float* lut, uint32_t i, uint32_t& rs,
+                                             float4 r0, float4 r1, float4 r2, ull* sub) {
+    const float2 q = gps_position<kIter>(f, T, lut, rs, r0, r1, r2);
+    if (kIter && r2.z > F_(1.0)) {
         // footprint block (write_block, oracle.rs:156-173): the s x s subpixels around the sample
         const int s = (int)r2.z, side = (int)f.side;
-        const int gx0 = (int)floorf(px_ * (float)side - F_(0.5) * (float)s + F_(0.5));
-        const int gy0 = (int)floorf(py_ * (float)side - F_(0.5) * (float)s + F_(0.5));
+        const int gx0 = (int)floorf(q.x * (float)side - F_(0.5) * (float)s + F_(0.5));
+        const int gy0 = (int)floorf(q.y * (float)side - F_(0.5) * (float)s + F_(0.5));
         const int gw = (int)f.W * side, gh = (int)f.H * side;
         uint32_t wrote = 0u;
         for (int gy = max(gy0, 0); gy < min(gy0 + s, gh); ++gy)
@@ -501,11 +544,9 @@ __device__ __forceinline__ uint32_t emit_gps(const FrameConst& f, const FTabs& T
             }
         return wrote;
     }
-    if (px_ < F_(0.0) || px_ >= (float)f.W || py_ < F_(0.0) || py_ >= (float)f.H) return 0u;
-    uint32_t px = f2u(px_), py = f2u(py_);
-    uint32_t sx = min(f.side - 1u, f2u((px_ - (float)px) * (float)f.side));
-    uint32_t sy = min(f.side - 1u, f2u((py_ - (float)py) * (float)f.side));
-    splat_write(sub, (py * f.W + px) * f.S + sy * f.side + sx, r0.z, i);
+    const uint32_t cell = subpixel_of(f, q);
+    if (cell == kNoCell) return 0u;
+    splat_write(sub, cell, r0.z, i);
     return 1u;
 }
 
@@ -732,42 +773,155 @@ void launch_fast_bounds(uint32_t* out, cudaStream_t st) {
     k_fast_bounds<<<148 * 8, 256, 0, st>>>(out);
 }
 
+// The subpixel a ScreenOccupancy particle tests, its offset from the splat's centre and the acceptance
+// draw's squared distance (particle_pass, gps_splat.wgsl:686-703): integer arithmetic and single
+// roundings in the shader's order, shared by the exact and the fast decision. Divisions by the
+// rectangle's width and by the subpixel count are multiplications by their reciprocals: R[3].x
+// holds floor((2^32 - 1) / width), whose quotient is at most one too small.
+struct SoCell {
+    uint32_t cell;  // subpixel index
+    float r2;       // squared Mahalanobis distance of the jittered sample
+};
+__device__ __forceinline__ SoCell so_cell(const FrameConst& f, uint32_t k, uint32_t& rs, const float4* R) {
+    const float4 r0 = R[0], b = R[1], inv = R[2], r3 = R[3];
+    const uint32_t side = f.side, samples = f.S;
+    const uint32_t bz = f2u(b.z);
+    uint32_t cell = k;
+    if (r3.w > F_(0.0))
+        cell = min(f2u(gx::next_u(&rs) * b.z * b.w * (float)samples), bz * f2u(b.w) * samples - 1u);
+    uint32_t pixel = cell, sub_i = 0u;
+    if (side > 1u) {
+        pixel = side == 2u ? cell >> 2 : side == 4u ? cell >> 4 : cell / 9u;
+        sub_i = cell - pixel * samples;
+    }
+    uint32_t row = __umulhi(pixel, __float_as_uint(r3.x)), col = pixel - row * bz;
+    if (col >= bz) {
+        col -= bz;
+        ++row;
+    }
+    const uint32_t xx = f2u(b.x) + col, yy = f2u(b.y) + row;
+    const float n1 = gx::next_u(&rs);
+    const float n2 = gx::next_u(&rs);
+    float uvx = n1, uvy = n2;
+    if (side > 1u) {
+        const uint32_t sy = side == 2u ? sub_i >> 1 : side == 4u ? sub_i >> 2 : sub_i / 3u;
+        uvx = (float)(sub_i - sy * side) + n1;
+        uvy = (float)sy + n2;
+        if (side == 3u) {
+            uvx = div_(uvx, F_(3.0));
+            uvy = div_(uvy, F_(3.0));
+        } else {  // a division by a power of two is exact
+            const float h = side == 2u ? F_(0.5) : F_(0.25);
+            uvx = uvx * h;
+            uvy = uvy * h;
+        }
+    }
+    const float dx = (float)xx + uvx - r0.x, dy = (float)yy + uvy - r0.y;
+    SoCell c;
+    c.r2 = fmax_(inv.x * dx * dx + F_(2.0) * inv.y * dx * dy + inv.z * dy * dy, F_(0.0));
+    c.cell = (yy * f.W + xx) * samples + sub_i;
+    return c;
+}
+// whether the particle is a hit, u its acceptance draw (gps_splat.wgsl:700-706)
+__device__ __forceinline__ bool so_hit(const FrameConst& f, const FTabs& T, const float4* R, float r2, float u) {
+    const float alpha = fmin_(R[0].w * gx::exp_t(-F_(0.5) * r2, T.ex), gxc::kOneMinus1e6);
+    const float l = gx::log_t(F_(1.0) - alpha, T.lg);
+    const float coverage = R[3].w > F_(0.0) ? div_(-l, R[2].w) : F_(1.0) - gx::exp_t(f.density * l, T.ex);
+    return !(u >= coverage);
+}
 // ScreenOccupancy branch of particle_pass (gps_splat.wgsl:686-708); returns 1 on a hit
 __device__ __forceinline__ uint32_t emit_so(const FrameConst& f, const FTabs& T, uint32_t i, uint32_t k, uint32_t& rs,
                                             const float4* R, ull* sub) {
-    float4 r0 = R[0], b = R[1];
-    const uint32_t side = f.side, samples = f.S;
-    bool sparse = R[3].w > F_(0.0);
-    uint32_t cell = k;
-    uint32_t bz = f2u(b.z), bw = f2u(b.w);
-    if (sparse) cell = min(f2u(gx::next_u(&rs) * b.z * b.w * (float)samples), bz * bw * samples - 1u);
-    uint32_t pixel = cell / samples, sub_i = cell % samples;
-    uint32_t xx = f2u(b.x) + pixel % bz, yy = f2u(b.y) + pixel / bz;
-    float n1 = gx::next_u(&rs);
-    float n2 = gx::next_u(&rs);
-    float uvx = div_((float)(sub_i % side) + n1, (float)side);
-    float uvy = div_((float)(sub_i / side) + n2, (float)side);
-    float dx = (float)xx + uvx - r0.x, dy = (float)yy + uvy - r0.y;
-    float4 inv = R[2];
-    float r2 = fmax_(inv.x * dx * dx + F_(2.0) * inv.y * dx * dy + inv.z * dy * dy, F_(0.0));
-    float alpha = fmin_(r0.w * gx::exp_t(-F_(0.5) * r2, T.ex), gxc::kOneMinus1e6);
-    float coverage;
-    if (sparse) coverage = div_(-gx::log_t(F_(1.0) - alpha, T.lg), inv.w);
-    else coverage = F_(1.0) - gx::exp_t(f.density * gx::log_t(F_(1.0) - alpha, T.lg), T.ex);
-    if (gx::next_u(&rs) >= coverage) return 0u;
-    splat_write(sub, (yy * f.W + xx) * samples + sub_i, r0.z, i);
+    const SoCell c = so_cell(f, k, rs, R);
+    if (!so_hit(f, T, R, c.r2, gx::next_u(&rs))) return 0u;
+    splat_write(sub, c.cell, R[0].z, i);
     return 1u;
 }
 
+// ---------------------------------------------------------------- fast decisions (ScreenOccupancy, GPS)
+// Both methods write a depth that is constant per splat, so a particle's whole effect is the
+// subpixel it hits: once approximate maths with an error bound settles that, the exact path is not
+// needed at all. The answers are the exact path's: 0 not written, 1 written, 2 undecided.
+
+// so_hit with the MUFU forms. r2 is exact here, so the only errors are those of exp and log:
+// y = o exp(-r2/2) within y rel (approximation, the exact exp's 2 ulp, both products' roundings),
+// v = 1 - min(y, 1 - 1e-6) within ev, log v within el (its argument's error ev / v, 1.07 for
+// ev / v <= 1/16, the approximation's and the exact log's own errors). Sparse splats compare u tau
+// with -log v (one division and one product rounding), dense ones u with 1 - exp(density log v).
+__device__ __forceinline__ uint32_t so_fast(const FrameConst& f, const float4* R, float r2, float u) {
+    const float y = R[0].w * mufu(r2 * (-F_(0.5) * kLog2e), 1);
+    const float rel = __fmaf_rn(F_(0.5) * kExpB, r2, kExpA + F_(5.4e-7) + F_(2.0) * kU);
+    const float ev = __fmaf_rn(y, rel, F_(2.0) * kU + F_(2.0) * kExpTiny);
+    const float v = F_(1.0) - fmin_(y, gxc::kOneMinus1e6);
+    const float rv = ev * mufu(v, 3);
+    const float l2 = mufu(v, 0);  // log2 v <= 0
+    const float nl = l2 * -kLn2;
+    const float el = __fmaf_rn(kLogRel + F_(5e-7), nl, __fmaf_rn(F_(1.08), rv, (kLogAbs + F_(4e-7)) * F_(1.01)));
+    float a, e;  // the draw against a, within e
+    bool sure = rv <= F_(0.0625);
+    if (R[3].w > F_(0.0)) {
+        u = u * R[2].w;
+        a = nl;
+        e = __fmaf_rn(F_(8.0) * kU, u, el);
+    } else {
+        const float x2 = f.density * l2;  // density log v, in powers of two
+        const float ea = f.density * el;  // of density log v
+        const float q = mufu(x2, 1);
+        a = F_(1.0) - q;
+        e = __fmaf_rn(q, __fmaf_rn(kExpB + F_(2.0) * kU, -x2, __fmaf_rn(ea, F_(1.1), kExpA + F_(5.4e-7))), F_(4.0) * kU + F_(2.0) * kExpTiny);
+        sure = sure && ea >= F_(0.0) && ea <= F_(0.0625);
+    }
+    e = e * kSafe;
+    const bool miss = u >= a + e, hit = u < a - e;
+    return !sure ? 2u : miss ? 0u : hit ? 1u : 2u;
+}
+
+// A GPS particle's subpixel (bounds: gps_limits). At a node of the radius table either neighbouring
+// cell gives the same value, so the cell may come from rounding w - 1/2.
+__device__ __forceinline__ uint32_t gps_fast(const FrameConst& f, const float* lut, uint32_t rs, float4 r0, float4 r1,
+                                             uint32_t row, float2 lim, uint32_t& cell) {
+    const float a = fmax_(F_(1.0) - gx::next_u(&rs), gxc::kUMin);
+    rs = gx::pcg(rs);
+    const float x = mufu(a, 0) * (-F_(2.0) * kLn2);
+    const float w = (x * mufu(x, 2)) * (gxc::kLutFv * F_(0.70710678));  // < 126.7
+    const float t = (float)(rs >> 8u) * (gxc::kTwoPi * (F_(1.0) / F_(16777216.0)));
+    const float wb = (w - F_(0.5)) + kCellBias;
+    const float b = w - (wb - kCellBias);
+    const float* L = lut + row + (__float_as_uint(wb) & 0xFFu);
+    const bool far = x >= kXMin;  // else the radius bound does not hold (and w may be NaN)
+    float ra = F_(0.0);
+    if (far) {
+        const float q00 = L[0], q01 = L[1], q10 = L[129], q11 = L[130];
+        const float p0 = __fmaf_rn(b, q01 - q00, q00), p1 = __fmaf_rn(b, q11 - q10, q10);
+        ra = __fmaf_rn(r1.w, p1 - p0, p0);
+    }
+    const float wx = ra * mufu(t, 5), wy = ra * mufu(t, 4);
+    const float px = __fmaf_rn(r1.x, wx, r0.x), py = __fmaf_rn(r1.z, wy, __fmaf_rn(r1.y, wx, r0.y));
+    const float side = (float)f.side;
+    const float hx = __fmaf_rn(px, side, -F_(0.5)), hy = __fmaf_rn(py, side, -F_(0.5));
+    const float bx = hx + kCellBias, by = hy + kCellBias;
+    const bool sure = far && fabsf(hx - (bx - kCellBias)) < lim.x && fabsf(hy - (by - kCellBias)) < lim.y;
+    const uint32_t cx = __float_as_uint(bx) - 0x4B400000u, cy = __float_as_uint(by) - 0x4B400000u;
+    const bool on = cx < f.W * f.side && cy < f.H * f.side;
+    if (f.side == 1u) {
+        cell = cy * f.W + cx;
+    } else {
+        const uint32_t m = f.side == 2u ? 0x80000000u : f.side == 4u ? 0x40000000u : 0x55555556u;
+        const uint32_t qx = __umulhi(cx, m), qy = __umulhi(cy, m);
+        cell = qy * ((f.W - 1u) * f.S) + cy * f.side + qx * (f.S - f.side) + cx;
+    }
+    return sure ? (on ? 1u : 0u) : 2u;
+}
+
 constexpr int kPT = 256;               // threads per particle block
-constexpr uint32_t kRing = 64;         // per-warp ring of undecided PBVR particles (uint2 entries)
+constexpr uint32_t kRing = 64;         // per-warp ring of undecided particles (uint2 entries)
 #ifndef GPSB_FAST_GIVE_UP
 #define GPSB_FAST_GIVE_UP 10
 #endif
-// undecided lanes of one step above which a warp stops the fast test for the rest of its tile
+// undecided lanes of one step above which a warp stops the PBVR fast test for the rest of its unit
 // (measured on the bench views: 10 beats 4, 7, 16, 24 and never giving up)
 constexpr uint32_t kFastGiveUp = GPSB_FAST_GIVE_UP;
-static_assert(kTabFloats % 2 == 0, "the ring after the entry lists needs 8-byte alignment");
+static_assert(kTabFloats % 2 == 0, "the unit table after the maths tables needs 8-byte alignment");
 
 // Largest j in [lo, hi) with off(j) <= v, by a 32-ary warp search (off(lo) <= v must hold).
 __device__ __forceinline__ uint32_t warp_last_le(const uint2* __restrict__ L, uint32_t lo, uint32_t hi, uint64_t v, int lane) {
@@ -785,256 +939,253 @@ __device__ __forceinline__ uint32_t warp_last_le(const uint2* __restrict__ L, ui
     return lo;
 }
 
-// Persistent particle kernel: every block repeatedly takes a tile of kPTile consecutive
-// particles of one ensemble (dynamic work counter), maps each particle to (splat i, k) through
-// the compact list, regenerates it from its own stream particle_seed(i, k + 1, seed) and writes it
-// with one 64-bit atomicMin of (depth key << 32 | i), which equals the reference's depth pass
-// followed by the colour pass (gps_splat.wgsl:276-281). Ensembles flagged skipped get no work.
-// MC: 0 GPS, 1 PBVR, 2 ScreenOccupancy; kPIPT: particles per thread per tile; FM: PBVR fast decisions
-// (0 off, 1 on, 2 validate), a template parameter so each variant gets its own register allocation
-template <int MC, int kPIPT, int FM>
-__global__ void __launch_bounds__(kPT, FM == 1 ? GPSB_FAST_MIN_BLOCKS : GPSB_PARTICLE_MIN_BLOCKS) k_particles(FrameConst f, const float4* __restrict__ rec,
-                                                   const float* __restrict__ lut, const uint2* __restrict__ clist,
-                                                   const EnsTotal* __restrict__ etot, uint32_t first_seed, uint32_t E,
-                                                   ull* sub, uint32_t* unit_counter, ull* stats) {
-    constexpr int kPTile = kPT * kPIPT;  // particles per tile
-    // dynamic shared memory: [fmath tables (kTabFloats)] [first unit of each ensemble (E + 1)]
-    // [entry offsets (kPTile + 2)] [entry ids (kPTile + 2)] [radius table (GPS) | rings (PBVR fast)]
+// Whether variant (MC, FM) keeps the maths tables in shared memory: the variants whose particles
+// mostly run the exact path. The fast GPS and ScreenOccupancy variants reach it for well under one
+// particle in a hundred and read the global tables, which leaves the space to more blocks.
+template <int MC, int FM>
+constexpr bool kStageTabs = MC == 1 || FM != 1;
+
+// Persistent particle kernel. A unit of work is up to steps * 32 consecutive particles of one
+// ensemble; every warp by itself takes the next unit from a device counter, finds its first list
+// entry with a 32-ary search and steps through it 32 particles at a time, lane l on particle
+// p + l. Each particle is mapped to (splat i, k) through the compact list, regenerated from its own
+// stream particle_seed(i, k + 1, seed) and written with one 64-bit atomicMin of (depth key << 32 | i),
+// which equals the reference's depth pass followed by the colour pass (gps_splat.wgsl:276-281).
+// Ensembles flagged skipped get no work.
+//
+// Bound: instruction issue (PBVR, ScreenOccupancy) or the scattered reads of the subpixel words
+// (GPS). Consecutive lanes hold consecutive particles, so a step of a splat with 32 or more particles
+// left is one warp-uniform comparison, and where splats change within a step the lanes share the
+// records they load: the list entries of the step are one coalesced 256-byte read, the boundaries
+// within it a __reduce_or_sync of one bit each. No list staging in shared memory, no block barrier.
+// Measured against tiles of 4096 particles per block, 16 consecutive ones per thread, staged lists
+// and the exact path for GPS and ScreenOccupancy (B200): GPS, 560k splats, 1280x720, 2x2 subpixels, 4
+// ensembles (773M particles) 9.14 -> 4.9 ms, 252 -> 190 instructions per particle; ScreenOccupancy,
+// 2M splats, 1920x1080, 2 ensembles (4.9G particles) 56.4 -> 34 ms, 379 -> 220 instructions.
+//
+// MC: 0 GPS, 1 PBVR, 2 ScreenOccupancy; FM: fast decisions (0 off, 1 on, 2 validate: exact always,
+// disagreements counted), template parameters so each variant gets its own register allocation.
+template <int MC, int FM>
+__global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS : GPSB_PARTICLE_MIN_BLOCKS)
+    k_particles(FrameConst f, const float4* __restrict__ rec, const float* __restrict__ lut, const uint2* __restrict__ clist,
+                const EnsTotal* __restrict__ etot, uint32_t first_seed, uint32_t E, uint32_t max_steps, ull* sub,
+                uint32_t* unit_counter, ull* stats) {
+    // dynamic shared memory: [maths tables (kTabFloats)] [first unit of each ensemble (E + 1, 64-bit)]
+    // [rings (FM == 1)] [radius table (GPS)]
     extern __shared__ __align__(16) uint32_t s_dyn[];
-    const FTabs T = stage_tabs(reinterpret_cast<float*>(s_dyn));
-    uint64_t* s_ubase = reinterpret_cast<uint64_t*>(s_dyn + kTabFloats);
-    uint32_t* s_off = s_dyn + kTabFloats + 2 * (E + 1);
-    uint32_t* s_id = s_off + (kPTile + 2);
-    float* s_lut = reinterpret_cast<float*>(s_id + (kPTile + 2));
-    __shared__ uint32_t s_unit, s_j0, s_w, s_claim;
+    constexpr bool kTabs = kStageTabs<MC, FM>;
+    uint64_t* s_ubase = reinterpret_cast<uint64_t*>(s_dyn + (kTabs ? kTabFloats : 0));
+    uint2* s_ring = reinterpret_cast<uint2*>(s_ubase + (E + 1));
+    float* s_lut = reinterpret_cast<float*>(s_ring + (FM == 1 ? (kPT / 32) * kRing : 0));
+    __shared__ uint32_t s_steps;
     const int tid = threadIdx.x, lane = tid & 31;
-    const bool use_lut = MC == 0 && !f.exact_radius;
-    if (use_lut)
-        for (int k = tid; k < kLutN; k += kPT) s_lut[k] = __ldg(&lut[k]);
-    if (tid == 0) {
-        uint64_t acc = 0;
-        for (uint32_t e = 0; e < E; ++e) {
-            s_ubase[e] = acc;
-            EnsTotal t = etot[e];
-            if (t.flags == 0u && t.particles) acc += (t.particles + kPTile - 1) / kPTile;
+    // particles per unit: max_steps * 32, fewer when the call is so small that warps would get none
+    if (tid < 32) {
+        uint64_t total = 0;
+        for (uint32_t e = lane; e < E; e += 32) {
+            const EnsTotal t = etot[e];
+            total += t.flags == 0u ? t.particles : 0ull;
         }
-        s_ubase[E] = acc;
+        for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        const uint64_t want = total / ((uint64_t)gridDim.x * kPT);
+        const uint32_t steps = want >= max_steps ? max_steps : want < 1u ? 1u : (uint32_t)want;
+        uint64_t acc = 0;
+        for (uint32_t e0 = 0; e0 < E; e0 += 32) {
+            const uint32_t e = e0 + lane;
+            uint64_t n = 0;
+            if (e < E) {
+                const EnsTotal t = etot[e];
+                n = t.flags == 0u ? (t.particles + steps * 32u - 1u) / (steps * 32u) : 0ull;
+            }
+            uint64_t incl = n;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (e < E) s_ubase[e] = acc + incl - n;
+            acc += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) {
+            s_ubase[E] = acc;
+            s_steps = steps;
+        }
     }
     __syncthreads();
     const uint64_t total_units = s_ubase[E];
-    const uint64_t PS = (uint64_t)f.W * f.H * f.S;
-    uint32_t points = 0, writes = 0, exact_runs = 0, mismatch = 0;
-    // next tile: its unit number and list window, found by one warp (lane 0 writes s_unit, s_j0, s_w)
-    auto find_unit = [&]() {
-        uint32_t un = 0u;
-        if (lane == 0) un = atomicAdd(unit_counter, 1u);
-        un = __shfl_sync(0xffffffffu, un, 0);
-        uint32_t j0 = 0u, j1 = 0u;
-        if ((uint64_t)un < total_units) {
-            uint32_t lo = 0, hi = E;
-            while (hi - lo > 1u) {
-                uint32_t mid = (lo + hi) >> 1;
-                if (s_ubase[mid] <= un) lo = mid; else hi = mid;
-            }
-            const EnsTotal et = etot[lo];
-            const uint64_t q0 = ((uint64_t)un - s_ubase[lo]) * kPTile;
-            const uint64_t q1 = q0 + kPTile < et.particles ? q0 + kPTile : et.particles;
-            const uint2* Lq = clist + (size_t)lo * f.N;
-            j0 = warp_last_le(Lq, 0u, et.nonzero, q0, lane);
-            j1 = warp_last_le(Lq, j0, et.nonzero, q1 - 1, lane);
-        }
-        if (lane == 0) {
-            s_unit = un;
-            s_j0 = j0;
-            s_w = j1 - j0 + 1u;
-        }
-    };
-    if (tid < 32) find_unit();
+    // a block whose warps could not get a unit each leaves before it stages anything
+    if ((uint64_t)blockIdx.x * (kPT / 32) >= total_units) return;
+    FTabs T{gx::tab_log(), gx::tab_exp(), gx::tab_sc()};
+    if (kTabs) T = stage_tabs(reinterpret_cast<float*>(s_dyn));
+    if (MC == 0 && !f.exact_radius)
+        for (int k = tid; k < kLutN; k += kPT) s_lut[k] = __ldg(&lut[k]);
     __syncthreads();
+    const uint32_t unit = s_steps * 32u;
+    const uint64_t PS = (uint64_t)f.W * f.H * f.S;
+    const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);  // lanes up to this one
+    uint2* ring = s_ring + (size_t)(tid >> 5) * kRing;
+    uint32_t points = 0, writes = 0, exact_runs = 0, mismatch = 0;
+    uint32_t next = 0u;
+    if (lane == 0) next = atomicAdd(unit_counter, 1u);
     for (;;) {
-        const uint64_t u = s_unit;
-        if (u >= total_units) break;
-        const uint32_t j0 = s_j0, w = s_w;
-        // ensemble of unit u: largest e with s_ubase[e] <= u
-        uint32_t lo = 0, hi = E;
-        while (hi - lo > 1u) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (s_ubase[mid] <= u) lo = mid; else hi = mid;
+        const uint32_t un = __shfl_sync(0xffffffffu, next, 0);
+        if ((uint64_t)un >= total_units) break;
+        if (lane == 0) next = atomicAdd(unit_counter, 1u);  // the next unit; its latency is covered by this one
+        // ensemble of the unit: largest e with s_ubase[e] <= un
+        uint32_t e = 0, eh = E;
+        while (eh - e > 1u) {
+            const uint32_t mid = (e + eh) >> 1;
+            if (s_ubase[mid] <= un) e = mid; else eh = mid;
         }
-        const uint32_t e = lo;
-        const EnsTotal et = etot[e];
-        const uint64_t p0 = (u - s_ubase[e]) * kPTile;
-        const uint64_t p1 = p0 + kPTile < et.particles ? p0 + kPTile : et.particles;
+        const uint32_t n_part = (uint32_t)etot[e].particles;  // below 2^32: the ensemble is not skipped
+        const uint32_t nz = etot[e].nonzero;
+        const uint32_t p0 = (uint32_t)((uint64_t)un - s_ubase[e]) * unit;
+        const uint32_t left = n_part - p0 < unit ? n_part - p0 : unit;  // particles of the unit
         const uint2* L = clist + (size_t)e * f.N;
-        for (uint32_t q = tid; q <= w; q += kPT) {
-            uint32_t j = j0 + q;
-            if (q < w) {
-                uint2 ent = __ldg(&L[j]);
-                s_id[q] = ent.x;
-                s_off[q] = ent.y;
-            } else {
-                s_off[q] = j < et.nonzero ? __ldg(&L[j].y) : (uint32_t)et.particles;
-            }
-        }
-        if (tid == 0) s_claim = 0u;
-        __syncthreads();  // window staged, unit read by every thread, claim open
         const uint32_t seed = first_seed + e;
         ull* S = sub + (size_t)e * PS;
-        uint64_t p = p0 + (uint64_t)tid * kPIPT;
-        if (MC == 1 && FM == 1) {
-            // Converged warp loop over the fast decisions: the particles pbvr_fast leaves undecided
-            // go to a per-warp ring in shared memory and run the exact path 32 at a time with the
-            // whole warp, instead of once for every divergent lane. A warp whose lanes are mostly
-            // undecided (on-screen work) drops the fast test for the rest of the tile.
-            uint2* ring = reinterpret_cast<uint2*>(s_lut) + (size_t)(tid >> 5) * kRing;
-            const uint32_t below = (1u << lane) - 1u;
-            uint32_t head = 0u, count = 0u, pp = 0u, pend = 0u, jj = 0u, cur = 0xFFFFFFFFu;
-            bool fast = true;
-            float4 R[kRecF4];
-            if (p < p1) {
-                pp = (uint32_t)p;
-                uint32_t a = 0, b = w;
-                while (b - a > 1u) {
-                    uint32_t m = (a + b) >> 1;
-                    if (s_off[m] <= pp) a = m; else b = m;
-                }
-                jj = a;
-                pend = (uint32_t)(p + kPIPT < p1 ? p + kPIPT : p1);
-            }
-            auto load_rec = [&](uint32_t i) {
-                const float4* Rg = rec + (size_t)i * kRecF4;
+        // the entry of the step's first particle: index ej, splat ci, offset co; nx the next offset
+        uint32_t ej = warp_last_le(L, 0u, nz, p0, lane);
+        uint32_t ci, co, nx;
+        {
+            const uint2 en = __ldg(&L[ej]);
+            ci = en.x;
+            co = en.y;
+            nx = ej + 1u < nz ? __ldg(&L[ej + 1u].y) : n_part;
+        }
+        uint32_t cur = 0xFFFFFFFFu;
+        float4 R[kRecF4];
+        auto load_rec = [&](uint32_t i) {
+            const float4* Rg = rec + (size_t)i * kRecF4;
+            constexpr int n = MC == 1 ? kRecF4 : FM == 1 || MC == 2 ? 4 : 3;
 #pragma unroll
-                for (int c = 0; c < kRecF4; ++c) R[c] = __ldg(&Rg[c]);
-                cur = i;
-            };
-            auto run_exact = [&](uint32_t i, uint32_t k) {
-                if (i != cur) load_rec(i);
-                uint32_t rs = gx::particle_seed(i, k + 1u, seed);
-                const uint32_t r = emit_pbvr(f, T, i, rs, R, S);
+            for (int c = 0; c < n; ++c) R[c] = __ldg(&Rg[c]);
+            cur = i;
+        };
+        auto run_exact = [&](uint32_t i, uint32_t k) {
+            if (i != cur) load_rec(i);
+            uint32_t rs = gx::particle_seed(i, k + 1u, seed);
+            uint32_t r;
+            if (MC == 0) {
+                writes += emit_gps<FM == 0>(f, T, s_lut, i, rs, R[0], R[1], R[2], S);
+            } else if (MC == 1) {
+                r = emit_pbvr(f, T, i, rs, R, S);
                 points += r & 1u;
                 writes += r >> 1;
-            };
-            uint32_t nxt = 0u, ci = 0u, ck = 0u;  // next entry boundary, current splat and index
-            if (pp < pend) {
-                ci = s_id[jj];
-                ck = pp - s_off[jj];
-                nxt = s_off[jj + 1];
+            } else {
+                r = emit_so(f, T, i, k, rs, R, S);
+                points += r;
+                writes += r;
             }
-            // fast steps: every lane evaluates a particle (a lane past its range evaluates one it
-            // does not own and ignores the answer; pbvr_fast only reads registers), so the step
-            // body has no divergent branch but the list boundary; a warp whose splat changed in
-            // any lane reloads every lane's record
-            int it = 0;
-            for (; it < kPIPT && fast; ++it) {
-                const bool act = pp < pend;
-                if (act && pp >= nxt) {
-                    while (pp >= s_off[jj + 1]) ++jj;
-                    ci = s_id[jj];
-                    ck = pp - s_off[jj];
-                    nxt = s_off[jj + 1];
+        };
+        uint32_t head = 0u, count = 0u;
+        bool fast = true;  // warp-uniform
+        for (uint32_t d0 = 0; d0 < left; d0 += 32u) {
+            const uint32_t pp0 = p0 + d0;  // first particle of the step
+            const bool act = d0 + (uint32_t)lane < left;
+            uint32_t i = ci, k = pp0 + (uint32_t)lane - co;
+            const uint32_t room = nx - pp0;  // particles of the current entry from pp0 on
+            if (room <= 32u) {
+                // entries that begin within the step, in list order, one per lane; offsets are distinct
+                const uint32_t j = ej + 1u + (uint32_t)lane;
+                const uint2 en = j < nz ? __ldg(&L[j]) : make_uint2(0u, 0u);
+                const uint32_t d = j < nz ? en.y - pp0 : 64u;
+                const uint32_t starts = __reduce_or_sync(0xffffffffu, d < 32u ? 1u << d : 0u);
+                const uint32_t c = (uint32_t)__popc(starts & upto);  // entries begun by this lane
+                const uint32_t src = c - 1u;
+                const uint32_t wi = __shfl_sync(0xffffffffu, en.x, src & 31u), wo = __shfl_sync(0xffffffffu, en.y, src & 31u);
+                if (c) {
+                    i = wi;
+                    k = pp0 + (uint32_t)lane - wo;
                 }
-                const uint32_t i = ci, k = ck;
-                ck += act ? 1u : 0u;
-                pp += act ? 1u : 0u;
+                // the entry of the next step's first particle
+                const uint32_t adv = (uint32_t)__popc(__ballot_sync(0xffffffffu, d <= 32u));
+                if (adv) {
+                    ej += adv;
+                    ci = __shfl_sync(0xffffffffu, en.x, adv - 1u);
+                    co = __shfl_sync(0xffffffffu, en.y, adv - 1u);
+                    nx = ej + 1u < nz ? (adv < 32u ? __shfl_sync(0xffffffffu, en.y, adv & 31u) : __ldg(&L[ej + 1u].y)) : n_part;
+                }
+            }
+            if (FM == 1 && (MC != 1 || fast)) {
+                // converged fast step: every lane evaluates a particle (a lane past the unit one it does
+                // not own, whose answer is ignored); where any lane's splat changed all lanes reload
                 if (__any_sync(0xffffffffu, i != cur)) load_rec(i);
-                const uint32_t q = pbvr_fast(f, gx::particle_seed(i, k + 1u, seed), R);
-                const uint32_t need = (act && q == 2u) ? 1u : 0u;
-                points += (act && q != 2u) ? q : 0u;
+                uint32_t rs = gx::particle_seed(i, k + 1u, seed);
+                uint32_t q;
+                if (MC == 0) {
+                    uint32_t cell;
+                    q = gps_fast(f, s_lut, rs, R[0], R[1], __float_as_uint(R[2].x) * 129u, make_float2(R[3].x, R[3].y), cell);
+                    if (act && q == 1u) {
+                        splat_write(S, cell, R[0].z, i);
+                        ++writes;
+                    }
+                } else if (MC == 1) {
+                    q = pbvr_fast(f, rs, R);
+                    points += (act && q != 2u) ? q : 0u;
+                } else {
+                    const SoCell c = so_cell(f, k, rs, R);
+                    q = so_fast(f, R, c.r2, gx::next_u(&rs));
+                    if (act && q == 1u) {
+                        splat_write(S, c.cell, R[0].z, i);
+                        ++writes;
+                        ++points;
+                    }
+                }
+                // undecided particles wait in the warp's ring and run the exact path 32 at a time
+                const bool need = act && q == 2u;
                 const uint32_t bal = __ballot_sync(0xffffffffu, need);
                 if (bal == 0u) continue;
                 const uint32_t n = (uint32_t)__popc(bal);
-                if (need) ring[(head + count + (uint32_t)__popc(bal & below)) & (kRing - 1u)] = make_uint2(i, k);
+                if (need) ring[(head + count + (uint32_t)__popc(bal & upto) - 1u) & (kRing - 1u)] = make_uint2(i, k);
                 count += n;
-                exact_runs += need;
+                exact_runs += need ? 1u : 0u;
                 if (n > kFastGiveUp) fast = false;
                 if (count >= 32u) {
                     __syncwarp();
-                    const uint2 e = ring[(head + (uint32_t)lane) & (kRing - 1u)];
+                    const uint2 en = ring[(head + (uint32_t)lane) & (kRing - 1u)];
                     __syncwarp();
                     head += 32u;
                     count -= 32u;
-                    run_exact(e.x, e.y);
+                    run_exact(en.x, en.y);
                 }
-            }
-            // the rest of the tile on the exact path (after the warp gave the fast test up)
-            for (; it < kPIPT; ++it) {
-                if (pp < pend) {
-                    if (pp >= nxt) {
-                        while (pp >= s_off[jj + 1]) ++jj;
-                        ci = s_id[jj];
-                        ck = pp - s_off[jj];
-                        nxt = s_off[jj + 1];
+            } else if (act) {
+                if (FM == 2) {  // validation: the fast answer against the exact path, which alone writes
+                    if (i != cur) load_rec(i);
+                    uint32_t rs = gx::particle_seed(i, k + 1u, seed), rx = rs;
+                    uint32_t q, x;
+                    if (MC == 0) {
+                        uint32_t cell;
+                        q = gps_fast(f, s_lut, rs, R[0], R[1], __float_as_uint(R[2].x) * 129u, gps_limits(f, R[0].x, R[0].y, R[1].x, R[1].y, R[1].z), cell);
+                        const uint32_t xc = subpixel_of(f, gps_position<false>(f, T, s_lut, rx, R[0], R[1], R[2]));
+                        x = xc == kNoCell ? 0u : 1u;
+                        if (q == 1u && xc != cell) x = 3u;
+                    } else if (MC == 1) {
+                        q = pbvr_fast(f, rs, R);
+                        x = emit_pbvr(f, T, i, rx, R, S);
+                        points += x & 1u;
+                        writes += x >> 1;
+                    } else {
+                        const SoCell c = so_cell(f, k, rs, R);
+                        const float u = gx::next_u(&rs);
+                        q = so_fast(f, R, c.r2, u);
+                        x = so_hit(f, T, R, c.r2, u) ? 1u : 0u;
                     }
-                    run_exact(ci, ck++);
-                    ++pp;
+                    mismatch += (q != 2u && q != x) ? 1u : 0u;
+                    exact_runs += q == 2u ? 1u : 0u;
+                    if (MC != 1) run_exact(i, k);
+                } else {
+                    run_exact(i, k);
                 }
             }
+        }
+        if (FM == 1) {
             __syncwarp();
             if ((uint32_t)lane < count) {
                 const uint2 q = ring[(head + (uint32_t)lane) & (kRing - 1u)];
                 run_exact(q.x, q.y);
             }
-        } else if (p < p1) {
-            uint32_t pp = (uint32_t)p;
-            // entry of particle pp in the window
-            uint32_t a = 0, b = w;
-            while (b - a > 1u) {
-                uint32_t m = (a + b) >> 1;
-                if (s_off[m] <= pp) a = m; else b = m;
-            }
-            uint32_t jj = a;
-            uint32_t cur = 0xFFFFFFFFu;
-            float4 R[kRecF4];
-            const uint32_t pend = (uint32_t)(p + kPIPT < p1 ? p + kPIPT : p1);
-            for (; pp < pend; ++pp) {
-                while (pp >= s_off[jj + 1]) ++jj;
-                const uint32_t i = s_id[jj];
-                const uint32_t k = pp - s_off[jj];
-                if (i != cur) {
-                    cur = i;
-                    const float4* Rg = rec + (size_t)i * kRecF4;
-                    R[0] = __ldg(&Rg[0]);
-                    R[1] = __ldg(&Rg[1]);
-                    if (MC != 1) R[2] = __ldg(&Rg[2]);
-                    if (MC == 1) {
-                        R[2] = __ldg(&Rg[2]);
-                        R[3] = __ldg(&Rg[3]);
-                        R[4] = __ldg(&Rg[4]);
-                        R[5] = __ldg(&Rg[5]);
-                    }
-                    if (MC == 2) R[3] = __ldg(&Rg[3]);
-                }
-                uint32_t rs = gx::particle_seed(i, k + 1u, seed);
-                if (MC == 0) {
-                    writes += emit_gps(f, T, s_lut, i, rs, R[0], R[1], R[2], S);
-                } else if (MC == 1) {
-                    uint32_t r;
-                    if (FM == 0) {
-                        r = emit_pbvr(f, T, i, rs, R, S);
-                    } else {
-                        const uint32_t q = pbvr_fast(f, rs, R);
-                        if (FM == 2) {  // validation: always exact, count disagreements
-                            r = emit_pbvr(f, T, i, rs, R, S);
-                            mismatch += (q != 2u && q != r) ? 1u : 0u;
-                        } else {
-                            r = q == 2u ? emit_pbvr(f, T, i, rs, R, S) : q;
-                        }
-                        exact_runs += q == 2u ? 1u : 0u;
-                    }
-                    points += r & 1u;
-                    writes += r >> 1;
-                } else {
-                    uint32_t r = emit_so(f, T, i, k, rs, R, S);
-                    points += r;
-                    writes += r;
-                }
-            }
+            __syncwarp();  // the ring is free again
         }
-        // the first warp done with this tile finds the next one while the others still work
-        uint32_t claim = 0u;
-        if (lane == 0) claim = atomicExch(&s_claim, 1u);
-        if (__shfl_sync(0xffffffffu, claim, 0) == 0u) find_unit();
-        __syncthreads();
     }
     ull v = points, wv = writes, xv = exact_runs, mv = mismatch;
     for (int o = 16; o; o >>= 1) {
@@ -1049,39 +1200,23 @@ __global__ void __launch_bounds__(kPT, FM == 1 ? GPSB_FAST_MIN_BLOCKS : GPSB_PAR
     if (lane == 0 && mv) atomicAdd(&stats[ST_FAST_MISMATCH], mv);
 }
 
-template <int MC, int IPT, int FM>
+template <int MC, int FM>
 static void launch_particles_t(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
                                const EnsTotal* etot, uint32_t first_seed, uint32_t E, unsigned long long* sub,
-                               uint32_t* unit_counter, unsigned long long* stats, int grid, cudaStream_t st) {
-    size_t smem = (kTabFloats + 2 * ((size_t)E + 1) + 2 * (kPT * IPT + 2)) * sizeof(uint32_t);
+                               uint32_t* unit_counter, unsigned long long* stats, int grid, int steps, cudaStream_t st) {
+    size_t smem = ((kStageTabs<MC, FM> ? kTabFloats : 0) + 2 * ((size_t)E + 1)) * sizeof(uint32_t);
+    if (FM == 1) smem += (size_t)(kPT / 32) * kRing * sizeof(uint2);
     if (MC == 0 && !fc.exact_radius) smem += kLutN * sizeof(float);
-    if (MC == 1 && FM == 1) smem += (size_t)(kPT / 32) * kRing * sizeof(uint2);
     // the attribute belongs to each device's context: remember the size set per device ordinal
     static size_t attr[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     const bool known = dev >= 0 && dev < 64;
     if (smem > 48 * 1024 && (!known || smem > attr[dev])) {
-        cudaFuncSetAttribute(k_particles<MC, IPT, FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_particles<MC, FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (known) attr[dev] = smem;
     }
-    k_particles<MC, IPT, FM><<<grid, kPT, smem, st>>>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats);
-}
-
-template <int IPT>
-static void launch_particles_m(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
-                               const EnsTotal* etot, uint32_t first_seed, uint32_t E, unsigned long long* sub,
-                               uint32_t* unit_counter, unsigned long long* stats, int grid, cudaStream_t st) {
-    if (fc.method == 0u)
-        launch_particles_t<0, IPT, 0>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
-    else if (fc.method == 4u)
-        launch_particles_t<2, IPT, 0>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
-    else if (fc.fast_mode == 1u)
-        launch_particles_t<1, IPT, 1>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
-    else if (fc.fast_mode == 2u)
-        launch_particles_t<1, IPT, 2>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
-    else
-        launch_particles_t<1, IPT, 0>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
+    k_particles<MC, FM><<<grid, kPT, smem, st>>>(fc, rec, lut, clist, etot, first_seed, E, (uint32_t)steps, sub, unit_counter, stats);
 }
 
 void launch_particles(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
@@ -1089,12 +1224,22 @@ void launch_particles(const FrameConst& fc, const float4* rec, const float* lut,
                       uint32_t* unit_counter, unsigned long long* stats, int grid, int items, cudaStream_t st) {
     cudaMemsetAsync(unit_counter, 0, sizeof(uint32_t), st);
     if (fc.N == 0 || E == 0) return;
-    if (items >= 24)
-        launch_particles_m<24>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
-    else if (items >= 16)
-        launch_particles_m<16>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
-    else
-        launch_particles_m<8>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, st);
+    // the fast GPS decisions cover single subpixels and the radius table; footprint blocks and the
+    // iterated radius run the exact path
+    uint32_t fm = fc.fast_mode;
+    if (fc.method == 0u && (fc.exact_radius || fc.fp_fixed > 1u || fc.fp_kappa > 0.0f)) fm = 0u;
+    auto go = [&](auto mc, auto mode) {
+        launch_particles_t<decltype(mc)::value, decltype(mode)::value>(fc, rec, lut, clist, etot, first_seed, E, sub,
+                                                                       unit_counter, stats, grid, items, st);
+    };
+    auto method = [&](auto mc) {
+        if (fm == 1u) go(mc, std::integral_constant<int, 1>());
+        else if (fm == 2u) go(mc, std::integral_constant<int, 2>());
+        else go(mc, std::integral_constant<int, 0>());
+    };
+    if (fc.method == 0u) method(std::integral_constant<int, 0>());
+    else if (fc.method == 4u) method(std::integral_constant<int, 2>());
+    else method(std::integral_constant<int, 1>());
 }
 
 // ============================================================================ primitive path

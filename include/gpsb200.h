@@ -181,9 +181,10 @@ gpsb_status gpsb_set_stream(gpsb_renderer* r, void* cuda_stream);
  * blur. footprint_subpixels <= 1 with adaptive_kappa = 0 is the normal GPS renderer. */
 gpsb_status gpsb_set_footprint(gpsb_renderer* r, uint32_t footprint_subpixels, float adaptive_kappa,
                               uint32_t footprint_max, uint32_t compensate_blur);
-/* PBVR fast decisions (no counterpart in the reference, whose shader runs every particle through
- * the full path): 0 off; 1 on, where particles that bounded approximate maths proves are not
- * points or are points off screen skip the exact path, which leaves every output bit-identical;
+/* Fast decisions (no counterpart in the reference, whose shader runs every particle through the
+ * full path): 0 off; 1 on, where particles that bounded approximate maths settles (PBVR: not a
+ * point, or a point off screen; GPS and ScreenOccupancy: the subpixel written, or none) skip the
+ * exact path, which leaves every output bit-identical;
  * 2 validate, where every particle runs the exact path and the fast answer is checked against it
  * (gpsb_debug_fast_counts). Default 1. */
 gpsb_status gpsb_set_fast_decisions(gpsb_renderer* r, uint32_t mode);
