@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "fmath.h"
+#include "pbvr_fast.h"
 
 namespace gpsb {
 
@@ -29,6 +30,7 @@ struct FrameConst {
     uint32_t fp_fixed, fp_max, fp_comp;
     float fp_kappa;
     uint32_t fast_mode;  // PBVR fast decisions: 0 off, 1 on, 2 validate (exact always, count disagreements)
+    gxf::Frame ff;       // their frame constants
 };
 
 enum : uint32_t { FLAG_RADIAL = 1u, FLAG_CENTRE = 2u, FLAG_JITTER = 4u };
@@ -40,13 +42,16 @@ enum : uint32_t { FLAG_RADIAL = 1u, FLAG_CENTRE = 2u, FLAG_JITTER = 4u };
 //   (ScreenOccupancy sparse). Bit 2 = under-covered (ViewConditioned).
 enum : uint32_t { CD_NONE = 0u, CD_POISSON_CAP = 1u, CD_FIXED = 2u, CD_POISSON = 3u, CD_UNDERCOVERED = 4u };
 
-// Particle record: 6 float4 per splat (the reference's proj layout, gps_splat.wgsl:627-628,
-// 566-577, 605-610), plus hoisted per-splat constants in otherwise unused lanes:
-//   GPS : r0 (mean.xy, depth, o)  r1 (l00, l10, l11, lut_a)  r2.x = bits(lut row i0), r2.y = Li2(o)
+// Particle record: 12 float4 per splat. r0..r5 are the reference's proj layout (gps_splat.wgsl:627-628,
+// 566-577, 605-610) plus hoisted per-splat constants in otherwise unused lanes; r6..r11 hold the PBVR
+// fast record (pbvr_fast.h), read instead of r0..r5 by most particles:
+//   GPS : r0 (mean.xy, depth, o)  r1 (l00, l10, l11, lut_a)  r2.x = bits(lut row i0), r2.y = Li2(o),
+//         r2.z footprint  r3.xy half a subpixel minus the fast position's bound
 //   PBVR: r0 (mean.xy, depth, o)  r1.x keep, r1.y h(min(o, 1-1e-6))  r2 (pos, inv_xx)
 //         r3 (inv_xy, inv_yy)  r4 (l00, l10, l11)  r5 (l20, l21, l22)
-//   SO  : r0 (mean.xy, depth, o)  r1 (lo.xy, size.xy)  r2 (inv_xx, inv_xy, inv_yy, peak_tau)  r3.w sparse
-constexpr int kRecF4 = 6;
+//   SO  : r0 (mean.xy, depth, o)  r1 (lo.xy, size.xy)  r2 (inv_xx, inv_xy, inv_yy, peak_tau)
+//         r3.x = bits(floor((2^32 - 1) / width))  r3.w sparse
+constexpr int kRecF4 = 12;
 
 // Statistics words (64-bit): gpsb_stats field order.
 enum : int {

@@ -26,33 +26,22 @@ namespace gpsb {
 
 typedef unsigned long long ull;
 
-// ---------------------------------------------------------------- fast decisions (PBVR)
-// Most particles of a close view are never written: in the near orbit of a 560k-splat scene at
-// 1280x720, 98.6 % of them fall off screen, behind the near plane or out of the radial keep test,
-// and all that matters for them is whether they count as points. pbvr_fast answers that with the
-// MUFU approximations (lg2 / rsqrt / sin / cos / ex2 / rcp, flush-to-zero forms) and bounds on
-// |fast value - exact f32 value|; whenever a bound straddles a threshold, or the particle may
-// land on screen, it answers 2 and the caller runs the exact path (emit_pbvr) from the
-// particle's own stream. Its answers are therefore the exact path's:
-//   0 = not a point, 1 = a point off screen (no write), 2 = undecided (run emit_pbvr).
-// Error model: every standard normal the fast path draws is within kEN of the exact path's and
-// at most kRMax in size (pairs with x = -2 log u1 < kXMin are left undecided), so the camera
-// coordinates' bounds are per-splat constants, written by the geometry kernel into unused lanes
-// of the record (fast_bounds_of); from there on, each step adds its propagated error, 2 kU per
-// rounding of either path times the magnitude rounded, and kSafe for the rounding of the bound
-// arithmetic itself. The constants of the approximations are checked against the exact maths
-// over every input they can get (gpsb_debug_fast_bounds); the exact maths' own errors are those
-// of fmath.h (exp 2 ulp, log 4 * 2^-24 relative or 2e-7 absolute).
-constexpr float kU = 6.0e-8f, kSafe = 1.01f;
-constexpr float kLogAbs = 3.5e-7f, kLogRel = 3.5e-7f;  // |mlog(v) - log(v)| <= kLogAbs + kLogRel |mlog(v)|, v in [kUMin, 1)
-constexpr float kSinCos = 1e-6f;                    // |msin/mcos(t) - sincos(t)|, t = RN(2 pi u), u = k 2^-24
-constexpr float kXMin = 1e-3f;                      // smallest x = -2 log u1 the bounds cover
-constexpr float kErMax = 2.5e-6f;                   // |r - r_exact| for x >= kXMin (r = x rsqrt(x))
-constexpr float kRMax = 5.77f;                      // largest r (u1 >= kUMin)
-constexpr float kEN = kErMax * (1.0f + 2.0f * kSinCos) + kRMax * (kSinCos + 2.01f * kU) + 1e-7f;  // one normal
+// ---------------------------------------------------------------- fast decisions
+// Particles whose effect bounded approximate maths settles skip the exact path; the bounds and the
+// decisions of the PBVR methods are in pbvr_fast.h, those of GPS and ScreenOccupancy below. The
+// approximations are the MUFU forms (lg2 / rsqrt / sin / cos / ex2 / rcp, flush-to-zero).
+using gxf::kErMax;
+using gxf::kLn2;
+using gxf::kLogAbs;
+using gxf::kLogRel;
+using gxf::kRMax;
+using gxf::kSinCos;
+using gxf::kU;
+using gxf::kXMin;
+constexpr float kSafe = 1.01f;
 constexpr float kExpA = 6e-7f, kExpB = 1.5e-7f;     // |mexp(a) - exp(a)| <= (kExpA + kExpB |a|) mexp(a) + kExpTiny, a <= 0
 constexpr float kExpTiny = 1.5e-38f;
-constexpr float kLn2 = 0.693147182f, kLog2e = 1.44269502f;
+constexpr float kLog2e = 1.44269502f;
 
 __device__ __forceinline__ float mufu(float x, int op) {
     float y;
@@ -69,33 +58,19 @@ __device__ __forceinline__ float mufu(float x, int op) {
 __device__ __forceinline__ float mlog(float x) { return mufu(x, 0) * kLn2; }
 __device__ __forceinline__ float mexp(float a) { return mufu(a * kLog2e, 1); }
 
-// Per-splat bounds of the fast path's camera coordinates (written by the geometry kernel into
-// r1.z = |fx| ecx, r1.w = |fy| ecy, r3.z = kSafe ecz, r3.w = |a| + 2|b| + |c|, r4.w = 2(|a| + |b|),
-// r5.w = 2(|b| + |c|) for the conic (a, b, c) = (r2.w, r3.x, r3.y)). World w_j = centre_j +
-// sum_k L_jk u_k (2, 4, 6 operations), p = w - camera (one more), c_i = dot3(rot_i, p) (5 more).
-__device__ __forceinline__ void fast_bounds_of(const FrameConst& f, float3 g0, float k00, float k10, float k11,
-                                               float k20, float k21, float k22, float a, float b, float c,
-                                               float4& r1, float4& r3, float4& r4, float4& r5) {
-    const float sx = fabsf(k00), sy = fabsf(k10) + fabsf(k11), sz = fabsf(k20) + fabsf(k21) + fabsf(k22);
-    const float gm = kRMax + kEN;
-    const float Mx = fabsf(g0.x) + fabsf(f.pos[0]) + sx * gm, My = fabsf(g0.y) + fabsf(f.pos[1]) + sy * gm,
-                Mz = fabsf(g0.z) + fabsf(f.pos[2]) + sz * gm;
-    const float ex = sx * kEN + F_(6.0) * kU * Mx, ey = sy * kEN + F_(10.0) * kU * My, ez = sz * kEN + F_(14.0) * kU * Mz;
-    auto row = [&](const float* q) {
-        const float ax = fabsf(q[0]), ay = fabsf(q[1]), az = fabsf(q[2]);
-        return (ax * ex + ay * ey + az * ez + F_(10.0) * kU * (ax * (Mx + ex) + ay * (My + ey) + az * (Mz + ez))) * F_(1.02);
-    };
-    const float ecx = row(f.rot0), ecy = row(f.rot1), ecz = row(f.rot2);
-    r1.z = fabsf(f.fx) * ecx * F_(1.02);
-    r1.w = fabsf(f.fy) * ecy * F_(1.02);
-    r3.z = ecz * kSafe;
-    r3.w = (fabsf(a) + F_(2.0) * fabsf(b) + fabsf(c)) * F_(1.02);
-    r4.w = F_(2.0) * (fabsf(a) + fabsf(b)) * F_(1.02);
-    r5.w = F_(2.0) * (fabsf(b) + fabsf(c)) * F_(1.02);
-    if (!isfinite(ecx) || !isfinite(ecy) || !isfinite(ecz) || !isfinite(r3.w)) {
-        r1.z = r1.w = r3.z = r3.w = r4.w = r5.w = __int_as_float(0x7F800000);  // never decides
+// The approximations of the PBVR decisions on the GPU.
+struct Mufu {
+    // sqrt(x), x = -2 log u1 (one rounding: scaling by a power of two commutes with it)
+    __device__ __forceinline__ float radius(float u1, float& x) const {
+        x = mufu(u1, 0) * (-F_(2.0) * kLn2);
+        return x * mufu(x, 2);
     }
-}
+    __device__ __forceinline__ float cos(float t) const { return mufu(t, 5); }
+    __device__ __forceinline__ float sin(float t) const { return mufu(t, 4); }
+    __device__ __forceinline__ float rcp(float x) const { return mufu(x, 3); }
+    __device__ __forceinline__ float ex2(float x) const { return mufu(x, 1); }
+    __device__ __forceinline__ float lg2(float x) const { return mufu(x, 0); }
+};
 
 // ---------------------------------------------------------------- fast decisions (GPS): position bound
 // gps_fast computes a particle's image position with the MUFU forms. r = sqrt(-2 log(1 - u1)) is
@@ -106,13 +81,14 @@ __device__ __forceinline__ void fast_bounds_of(const FrameConst& f, float3 g0, f
 // radii up to 5.84, within kGpsEw.
 constexpr float kLutSlope = 0.049f;
 constexpr float kGpsEw = kLutSlope * 1.3e-4f + 4e-6f + 5.84f * (kSinCos + 2.0f * kU) + 6e-7f;
-constexpr float kCellBias = 12582912.0f;  // 1.5 * 2^23: adding it rounds to the nearest whole number
+using gxf::kCellBias;
 // Half a subpixel minus the bound of |position - exact position| in subpixels, along x and y; a
 // sample nearer than that to a subpixel edge is undecided. Per unit of the factor's row sum S:
 // kGpsEw and the products' roundings (below 6e-6); the sums' roundings at the magnitude of the
 // mean and of the grid coordinate; 2e-6 for the subpixel arithmetic.
 __device__ __forceinline__ float2 gps_limits(const FrameConst& f, float mx, float my, float l00, float l10, float l11) {
     const float side = (float)f.side, sx = fabsf(l00), sy = fabsf(l10) + fabsf(l11);
+    if (max(f.W, f.H) > (1u << 20)) return make_float2(F_(-1.0), F_(-1.0));  // kCellBias holds grids below 2^22
     const float ex = (sx * (kGpsEw + 6e-6f) + F_(3e-7) * fabsf(mx)) * side * F_(1.02) + F_(2e-6);
     const float ey = (sy * (kGpsEw + 6e-6f) + F_(3e-7) * fabsf(my)) * side * F_(1.02) + F_(2e-6);
     return make_float2(F_(0.5) - ex, F_(0.5) - ey);  // not positive, or NaN: never decides
@@ -267,18 +243,21 @@ __global__ void __launch_bounds__(128) k_geometry(FrameConst f, const float4* __
                 float k11 = sqrt_(fmax_(a11 - k10 * k10, F_(1e-30)));
                 float k21 = div_(a21 - k20 * k10, k11);
                 float k22 = sqrt_(fmax_(a22 - k20 * k20 - k21 * k21, F_(1e-30)));
-                float4 q1 = make_float4(keep, eol(fmin_(o, gxc::kOneMinus1e6)), F_(0.0), F_(0.0));
-                float4 q3 = make_float4(-pr.b * idet, pr.a * idet, F_(0.0), F_(0.0));
-                float4 q4 = make_float4(k00, k10, k11, F_(0.0));
-                float4 q5 = make_float4(k20, k21, k22, F_(0.0));
-                fast_bounds_of(f, make_float3(g0.x, g0.y, g0.z), k00, k10, k11, k20, k21, k22, pr.c * idet, q3.x, q3.y,
-                               q1, q3, q4, q5);
+                const float oo = fmin_(o, gxc::kOneMinus1e6), h = eol(oo);
                 R[0] = r0;
-                R[1] = q1;
+                R[1] = make_float4(keep, h, F_(0.0), F_(0.0));
                 R[2] = make_float4(g0.x, g0.y, g0.z, pr.c * idet);
-                R[3] = q3;
-                R[4] = q4;
-                R[5] = q5;
+                R[3] = make_float4(-pr.b * idet, pr.a * idet, F_(0.0), F_(0.0));
+                R[4] = make_float4(k00, k10, k11, F_(0.0));
+                R[5] = make_float4(k20, k21, k22, F_(0.0));
+                if (f.fast_mode) {
+                    const float g[3] = {g0.x, g0.y, g0.z};
+                    float q[24];
+                    gxf::make_record(f.ff, f.rot0, f.rot1, f.rot2, f.pos, f.fx, f.fy, g, k00, k10, k11, k20, k21, k22,
+                                     pr.c * idet, -pr.b * idet, pr.a * idet, pr.mx, pr.my, oo, h, q);
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) R[6 + c] = make_float4(q[4 * c], q[4 * c + 1], q[4 * c + 2], q[4 * c + 3]);
+                }
             }
         }
     }
@@ -568,9 +547,10 @@ struct Normal {
     }
 };
 
-// emit_particle_pbvr (gps_splat.wgsl:490-532); returns bit 0 = counts as a point, bit 1 = written
-__device__ __forceinline__ uint32_t emit_pbvr(const FrameConst& f, const FTabs& T, uint32_t i, uint32_t& rs, const float4* R,
-                                              ull* sub) {
+// emit_particle_pbvr (gps_splat.wgsl:490-532); returns bit 0 = counts as a point, bit 1 = on screen, at
+// `cell` with depth `depth_z`
+__device__ __forceinline__ uint32_t pbvr_eval(const FrameConst& f, const FTabs& T, uint32_t& rs, const float4* R,
+                                              uint32_t& cell, float& depth_z) {
     Normal nm{&rs, T, false, F_(0.0)};
     float uz = nm.next();
     float uy = nm.next();
@@ -608,119 +588,36 @@ __device__ __forceinline__ uint32_t emit_pbvr(const FrameConst& f, const FTabs& 
         float keep = clamp_(div_(eol(y, T.lg), r1.y), F_(0.0), F_(1.0));
         if (gx::next_u(&rs) >= keep) return 0u;
     }
-    float depth_z = (flags & FLAG_CENTRE) ? r0.z : cz;
+    depth_z = (flags & FLAG_CENTRE) ? r0.z : cz;
     if (pix_x < F_(0.0) || pix_x >= (float)f.W || pix_y < F_(0.0) || pix_y >= (float)f.H) return 1u;
     uint32_t ipx = f2u(pix_x), ipy = f2u(pix_y);
     uint32_t sx = min(f.side - 1u, f2u((pix_x - (float)ipx) * (float)f.side));
     uint32_t sy = min(f.side - 1u, f2u((pix_y - (float)ipy) * (float)f.side));
-    splat_write(sub, (ipy * f.W + ipx) * f.S + sy * f.side + sx, depth_z, i);
+    cell = (ipy * f.W + ipx) * f.S + sy * f.side + sx;
     return 3u;
 }
-
-// One Box-Muller pair from the stream, drawn in the order of Normal::next (cos part, sin part).
-// Returns false when x = -2 log u1 is below kXMin, where the kEN bound does not hold.
-__device__ __forceinline__ bool fast_pair(uint32_t& st, float& c, float& s) {
-    const float u1 = fmax_(gx::next_u(&st), gxc::kUMin);
-    st = gx::pcg(st);  // u2 = (st >> 8) 2^-24, folded into t below
-    // x = -2 mlog(u1) and t = RN(2 pi u2), each with one rounding: scaling by a power of two
-    // commutes with rounding, so both equal the two-step values bit for bit
-    const float x = mufu(u1, 0) * (-F_(2.0) * kLn2);
-    const float r = x * mufu(x, 2);
-    const float t = (float)(st >> 8u) * (gxc::kTwoPi * (F_(1.0) / F_(16777216.0)));
-    c = r * mufu(t, 5);
-    s = r * mufu(t, 4);
-    return x >= kXMin;
+__device__ __forceinline__ uint32_t emit_pbvr(const FrameConst& f, const FTabs& T, uint32_t i, uint32_t& rs, const float4* R,
+                                              ull* sub) {
+    uint32_t cell;
+    float z;
+    const uint32_t r = pbvr_eval(f, T, rs, R, cell, z);
+    if (r & 2u) splat_write(sub, cell, z, i);
+    return r;
 }
 
-// Straight-line form: every lane computes the whole path and the answer is selected at the end
-// (the lanes of a warp rarely agree on an early exit, and divergent exits cost more than they save).
-__device__ __forceinline__ uint32_t pbvr_fast(const FrameConst& f, uint32_t st, const float4* R) {
-    float uz, uy, ux, jy;
-    bool ok = fast_pair(st, uz, uy);
-    ok &= fast_pair(st, ux, jy);  // jy is the pair's spare, used by the jitter
-    const float4 r1 = R[1];
-    if (f.method == 3u) {
-        if (gx::next_u(&st) >= r1.x) return 0u;  // the exact draw and test
+// grid coordinates (cx, cy) of a subpixel -> its index
+__device__ __forceinline__ uint32_t cell_of(const FrameConst& f, uint32_t cx, uint32_t cy) {
+    if (f.side == 1u) return cy * f.W + cx;
+    uint32_t qx, qy;
+    if (f.side == 3u) {
+        qx = __umulhi(cx, 0x55555556u);
+        qy = __umulhi(cy, 0x55555556u);
+    } else {
+        const uint32_t sh = f.side >> 1;  // 2 -> 1, 4 -> 2
+        qx = cx >> sh;
+        qy = cy >> sh;
     }
-    const float4 r2 = R[2], r3 = R[3], r4 = R[4], r5 = R[5];
-    const float px = __fmaf_rn(r4.x, ux, r2.x) - f.pos[0];
-    const float py = __fmaf_rn(r4.z, uy, __fmaf_rn(r4.y, ux, r2.y)) - f.pos[1];
-    const float pz = __fmaf_rn(r5.z, uz, __fmaf_rn(r5.y, uy, __fmaf_rn(r5.x, ux, r2.z))) - f.pos[2];
-    const float cz = __fmaf_rn(f.rot2[2], pz, __fmaf_rn(f.rot2[1], py, f.rot2[0] * px));
-    const float ecz = r3.z;  // already widened by kSafe
-    const bool behind = cz + ecz <= f.near_z;  // surely not a point
-    const float czl = cz - ecz;
-    bool sure = czl > f.near_z && czl > F_(3.0) * ecz && cz < 1e30f && czl > 1e-6f;  // surely in front
-    const float cx = __fmaf_rn(f.rot0[2], pz, __fmaf_rn(f.rot0[1], py, f.rot0[0] * px));
-    const float cy = __fmaf_rn(f.rot1[2], pz, __fmaf_rn(f.rot1[1], py, f.rot1[0] * px));
-    // t = (f c) / cz; |t - t'| <= (|f| ec + |t| ecz) / (cz - ecz) + the reciprocal's and both
-    // paths' roundings (1e-6 |t|), 1 / (cz - ecz) <= (1 + 2 ecz / cz) / cz for ecz <= cz / 4;
-    // then + f.cx with one more rounding in each path
-    const float icz = mufu(cz, 3);
-    const float icl = icz * __fmaf_rn((F_(2.0) * kSafe) * ecz, icz, kSafe);
-    const float kt = __fmaf_rn(ecz, icl, 1e-6f + F_(2.0) * kU);
-    const float tx = (f.fx * cx) * icz, ty = (f.fy * cy) * icz;
-    float pix_x = tx + f.cx, pix_y = ty + f.cy;
-    float epx = __fmaf_rn(fabsf(tx), kt, __fmaf_rn(r1.z, icl, F_(2.0) * kU * fabsf(f.cx)));
-    float epy = __fmaf_rn(fabsf(ty), kt, __fmaf_rn(r1.w, icl, F_(2.0) * kU * fabsf(f.cy)));
-    const uint32_t flags = f.flags;
-    if (flags & FLAG_JITTER) {
-        float jx, js;
-        sure &= fast_pair(st, jx, js);
-        // |sd j - sd j'| <= |sd| kEN, + the product's and the sum's roundings in both paths
-        const float kj = fabsf(f.jitter_sd) * (kEN + F_(4.0) * kU * kRMax);
-        pix_x = pix_x + f.jitter_sd * jx;
-        pix_y = pix_y + f.jitter_sd * jy;
-        epx = __fmaf_rn(F_(4.0) * kU, fabsf(pix_x), epx + kj);
-        epy = __fmaf_rn(F_(4.0) * kU, fabsf(pix_y), epy + kj);
-    }
-    sure &= fabsf(pix_x) < 1e30f && fabsf(pix_y) < 1e30f && epx < 1e30f && epy < 1e30f;
-    const float mx = kSafe * epx, my = kSafe * epy;
-    const bool off = pix_x + mx < F_(0.0) || pix_x - mx >= (float)f.W || pix_y + my < F_(0.0) || pix_y - my >= (float)f.H;
-    uint32_t res = off ? 1u : 2u;
-    if (flags & FLAG_RADIAL) {
-        const float4 r0 = R[0];
-        const float dvx = pix_x - r0.x, dvy = pix_y - r0.y;
-        const float e = fmaxf(__fmaf_rn(F_(2.0) * kU, fabsf(pix_x) + fabsf(r0.x), epx),
-                              __fmaf_rn(F_(2.0) * kU, fabsf(pix_y) + fabsf(r0.y), epy));
-        // r2v = a dx^2 + 2 b dx dy + c dy^2: |grad . d| <= e (G_x |dx| + G_y |dy|), |Q(d)| <= K e^2,
-        // roundings <= 20 kU (|a| + |b|) dx^2 + (|b| + |c|) dy^2
-        const float dx2 = dvx * dvx, dy2 = dvy * dvy;
-        const float r2v = __fmaf_rn(r2.w, dx2, __fmaf_rn(F_(2.0) * r3.x, dvx * dvy, r3.y * dy2));
-        const float m2 = __fmaf_rn(r4.w, dx2, r5.w * dy2);
-        const float er2 = __fmaf_rn(__fmaf_rn(r4.w, fabsf(dvx), r5.w * fabsf(dvy)), e, __fmaf_rn(r3.w * e, e, F_(10.0) * kU * m2));
-        const float a2 = fmaxf(r2v, F_(0.0));  // arg = -a2 / 2
-        const float earg = er2 * (F_(0.5) * kSafe);
-        // y = min(o, 1 - 1e-6) exp(arg): propagated error (e^earg - 1 <= earg (1 + earg)), the
-        // approximation against exp, exp's own 2 ulp at both arguments, the product's roundings;
-        // with earg < 1/8 every relative term grows by at most (1 + 2 earg) <= 1.25
-        const float oo = fmin_(r0.w, gxc::kOneMinus1e6);
-        const float y = oo * mufu(a2 * (-F_(0.5) * kLog2e), 1);  // = mexp(arg) bit for bit
-        const float rel = __fmaf_rn(earg, F_(1.0) + earg, __fmaf_rn(F_(0.5) * kExpB, a2, kExpA + F_(5.4e-7) + F_(2.0) * kU));
-        const float ey = __fmaf_rn(y, rel * (F_(1.25) * kSafe), F_(2.02) * kExpTiny);
-        // eol's log form, eol(y) = -log(1 - y) / y, which both paths take when y - ey >= 1e-4 (the
-        // short form 1 + y / 2 of y < 1e-4, beyond ~4.3 standard deviations, is left to the exact
-        // path), with 1 / (a - e) <= (1 + 2 e / a) / a for e <= a / 2: the approximation against
-        // log at v, log's own error at both arguments, the argument's error
-        const float v = F_(1.0) - fmin_(y, gxc::kOneMinus1e6);
-        const float ev = ey + F_(2.0) * kU;
-        const float lg = mlog(v);
-        const float iv = mufu(v, 3), iy = mufu(y, 3);
-        const float elg = __fmaf_rn(kLogRel + F_(5e-7), fabsf(lg), kLogAbs + F_(4e-7)) +
-                          ev * iv * __fmaf_rn(F_(2.0) * ev, iv, F_(1.0)) * kSafe;
-        const float eo = -lg * iy;
-        const float eeo = __fmaf_rn(__fmaf_rn(fabsf(eo), ey, elg) * iy, __fmaf_rn(F_(2.0) * ey, iy, F_(1.0)) * kSafe,
-                                    F_(4e-7) * fabsf(eo));
-        sure &= earg < F_(0.125) && y - ey >= F_(1e-4) && ev <= F_(0.5) * v && ey <= F_(0.5) * y;
-        const float de = eeo * kSafe;
-        // keep = clamp(eo / r1.y, 0, 1) against the exact draw, compared as u r1.y against eo
-        const float ur = gx::next_u(&st) * r1.y;
-        const bool reject = ur >= (eo + de) * (F_(1.0) + F_(6.0) * kU);
-        const bool keep = ur * (F_(1.0) + F_(6.0) * kU) < eo - de;
-        res = reject ? 0u : (keep ? res : 2u);
-    }
-    res = behind ? 0u : (sure ? res : 2u);
-    return ok ? res : 2u;
+    return qy * ((f.W - 1u) * f.S) + cy * f.side + qx * (f.S - f.side) + cx;
 }
 
 // Exhaustive check of the constants of the fast decisions: the largest |approximation - exact| /
@@ -903,13 +800,7 @@ __device__ __forceinline__ uint32_t gps_fast(const FrameConst& f, const float* l
     const bool sure = far && fabsf(hx - (bx - kCellBias)) < lim.x && fabsf(hy - (by - kCellBias)) < lim.y;
     const uint32_t cx = __float_as_uint(bx) - 0x4B400000u, cy = __float_as_uint(by) - 0x4B400000u;
     const bool on = cx < f.W * f.side && cy < f.H * f.side;
-    if (f.side == 1u) {
-        cell = cy * f.W + cx;
-    } else {
-        const uint32_t m = f.side == 2u ? 0x80000000u : f.side == 4u ? 0x40000000u : 0x55555556u;
-        const uint32_t qx = __umulhi(cx, m), qy = __umulhi(cy, m);
-        cell = qy * ((f.W - 1u) * f.S) + cy * f.side + qx * (f.S - f.side) + cx;
-    }
+    cell = cell_of(f, cx, cy);
     return sure ? (on ? 1u : 0u) : 2u;
 }
 
@@ -1053,28 +944,50 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
             nx = ej + 1u < nz ? __ldg(&L[ej + 1u].y) : n_part;
         }
         uint32_t cur = 0xFFFFFFFFu;
-        float4 R[kRecF4];
+        float4 R[6];
+        constexpr int kRec = MC == 1 ? 6 : FM == 1 || MC == 2 ? 4 : 3;
         auto load_rec = [&](uint32_t i) {
             const float4* Rg = rec + (size_t)i * kRecF4;
-            constexpr int n = MC == 1 ? kRecF4 : FM == 1 || MC == 2 ? 4 : 3;
 #pragma unroll
-            for (int c = 0; c < n; ++c) R[c] = __ldg(&Rg[c]);
+            for (int c = 0; c < kRec; ++c) R[c] = __ldg(&Rg[c]);
             cur = i;
         };
-        auto run_exact = [&](uint32_t i, uint32_t k) {
-            if (i != cur) load_rec(i);
+        float q[24];  // PBVR: the fast record of splat curq
+        float keep = F_(0.0);
+        uint32_t curq = 0xFFFFFFFFu;
+        auto load_fast = [&](uint32_t i) {
+            const float4* Rg = rec + (size_t)i * kRecF4 + 6;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                const float4 v = __ldg(&Rg[c]);
+                q[4 * c] = v.x;
+                q[4 * c + 1] = v.y;
+                q[4 * c + 2] = v.z;
+                q[4 * c + 3] = v.w;
+            }
+            if (f.method == 3u) keep = __ldg(&rec[(size_t)i * kRecF4 + 1].x);
+            curq = i;
+        };
+        auto exact = [&](uint32_t i, uint32_t k, const float4* X) {
             uint32_t rs = gx::particle_seed(i, k + 1u, seed);
-            uint32_t r;
             if (MC == 0) {
-                writes += emit_gps<FM == 0>(f, T, s_lut, i, rs, R[0], R[1], R[2], S);
-            } else if (MC == 1) {
-                r = emit_pbvr(f, T, i, rs, R, S);
-                points += r & 1u;
-                writes += r >> 1;
+                writes += emit_gps<FM == 0>(f, T, s_lut, i, rs, X[0], X[1], X[2], S);
             } else {
-                r = emit_so(f, T, i, k, rs, R, S);
-                points += r;
-                writes += r;
+                const uint32_t r = MC == 1 ? emit_pbvr(f, T, i, rs, X, S) : emit_so(f, T, i, k, rs, X, S);
+                points += r & 1u;
+                writes += MC == 1 ? r >> 1 : r;
+            }
+        };
+        auto run_exact = [&](uint32_t i, uint32_t k) {
+            if (FM == 1) {  // the lanes' splats differ; the registers of the fast record stay
+                const float4* Rg = rec + (size_t)i * kRecF4;
+                float4 X[kRec];
+#pragma unroll
+                for (int c = 0; c < kRec; ++c) X[c] = __ldg(&Rg[c]);
+                exact(i, k, X);
+            } else {
+                if (i != cur) load_rec(i);
+                exact(i, k, R);
             }
         };
         uint32_t head = 0u, count = 0u;
@@ -1109,30 +1022,58 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
             if (FM == 1 && (MC != 1 || fast)) {
                 // converged fast step: every lane evaluates a particle (a lane past the unit one it does
                 // not own, whose answer is ignored); where any lane's splat changed all lanes reload
-                if (__any_sync(0xffffffffu, i != cur)) load_rec(i);
+                if (MC == 1) {
+                    if (__any_sync(0xffffffffu, i != curq)) load_fast(i);
+                } else if (__any_sync(0xffffffffu, i != cur)) {
+                    load_rec(i);
+                }
                 uint32_t rs = gx::particle_seed(i, k + 1u, seed);
-                uint32_t q;
+                uint32_t a;  // the answer
                 if (MC == 0) {
                     uint32_t cell;
-                    q = gps_fast(f, s_lut, rs, R[0], R[1], __float_as_uint(R[2].x) * 129u, make_float2(R[3].x, R[3].y), cell);
-                    if (act && q == 1u) {
+                    a = gps_fast(f, s_lut, rs, R[0], R[1], __float_as_uint(R[2].x) * 129u, make_float2(R[3].x, R[3].y), cell);
+                    if (act && a == 1u) {
                         splat_write(S, cell, R[0].z, i);
                         ++writes;
                     }
                 } else if (MC == 1) {
-                    q = pbvr_fast(f, rs, R);
-                    points += (act && q != 2u) ? q : 0u;
+                    Mufu ap;
+                    gxf::Point P;
+                    a = gxf::decide(ap, f.ff, f.flags, f.method == 3u, keep, rs, q, P);
+                    if (act && a == 3u) {
+                        // on screen: with the subpixel settled and the depth surely behind the subpixel's
+                        // word (which only ever decreases) the write has no effect but its count
+                        uint32_t cx, cy;
+                        bool on;
+                        a = 2u;
+                        if (gxf::settle(f.ff, f.side, f.W, f.H, P, cx, cy, on)) {
+                            a = 1u;
+                            if (on) {
+                                const uint32_t cell = cell_of(f, cx, cy);
+                                if (f.flags & FLAG_CENTRE) {
+                                    splat_write(S, cell, __ldg(&rec[(size_t)i * kRecF4].z), i);
+                                    ++writes;
+                                } else {
+                                    const uint32_t front = f2b(P.z - q[21]) | 0x80000000u;
+                                    const bool behind = front > __ldcg(reinterpret_cast<const uint32_t*>(S + cell) + 1);
+                                    a = behind ? 1u : 2u;
+                                    writes += behind ? 1u : 0u;
+                                }
+                            }
+                        }
+                    }
+                    points += act ? a & 1u : 0u;
                 } else {
                     const SoCell c = so_cell(f, k, rs, R);
-                    q = so_fast(f, R, c.r2, gx::next_u(&rs));
-                    if (act && q == 1u) {
+                    a = so_fast(f, R, c.r2, gx::next_u(&rs));
+                    if (act && a == 1u) {
                         splat_write(S, c.cell, R[0].z, i);
                         ++writes;
                         ++points;
                     }
                 }
                 // undecided particles wait in the warp's ring and run the exact path 32 at a time
-                const bool need = act && q == 2u;
+                const bool need = act && a == 2u;
                 const uint32_t bal = __ballot_sync(0xffffffffu, need);
                 if (bal == 0u) continue;
                 const uint32_t n = (uint32_t)__popc(bal);
@@ -1152,27 +1093,41 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                 if (FM == 2) {  // validation: the fast answer against the exact path, which alone writes
                     if (i != cur) load_rec(i);
                     uint32_t rs = gx::particle_seed(i, k + 1u, seed), rx = rs;
-                    uint32_t q, x;
+                    uint32_t a, x;
                     if (MC == 0) {
                         uint32_t cell;
-                        q = gps_fast(f, s_lut, rs, R[0], R[1], __float_as_uint(R[2].x) * 129u, gps_limits(f, R[0].x, R[0].y, R[1].x, R[1].y, R[1].z), cell);
+                        a = gps_fast(f, s_lut, rs, R[0], R[1], __float_as_uint(R[2].x) * 129u, gps_limits(f, R[0].x, R[0].y, R[1].x, R[1].y, R[1].z), cell);
                         const uint32_t xc = subpixel_of(f, gps_position<false>(f, T, s_lut, rx, R[0], R[1], R[2]));
                         x = xc == kNoCell ? 0u : 1u;
-                        if (q == 1u && xc != cell) x = 3u;
+                        if (a == 1u && xc != cell) x = 3u;
                     } else if (MC == 1) {
-                        q = pbvr_fast(f, rs, R);
-                        x = emit_pbvr(f, T, i, rx, R, S);
-                        points += x & 1u;
-                        writes += x >> 1;
+                        if (i != curq) load_fast(i);
+                        Mufu ap;
+                        gxf::Point P;
+                        a = gxf::decide(ap, f.ff, f.flags, f.method == 3u, keep, rs, q, P);
+                        uint32_t xc;
+                        float z;
+                        x = pbvr_eval(f, T, rx, R, xc, z);
+                        if (a == 3u) {
+                            uint32_t cx, cy;
+                            bool on, ok = (x & 1u) != 0u;
+                            if (gxf::settle(f.ff, f.side, f.W, f.H, P, cx, cy, on)) {
+                                ok = x == (on ? 3u : 1u);
+                                if (ok && on)
+                                    ok = xc == cell_of(f, cx, cy) && ((f.flags & FLAG_CENTRE) || fabsf(P.z - z) <= q[21]);
+                            }
+                            mismatch += ok ? 0u : 1u;
+                            a = 2u;
+                        }
                     } else {
                         const SoCell c = so_cell(f, k, rs, R);
                         const float u = gx::next_u(&rs);
-                        q = so_fast(f, R, c.r2, u);
+                        a = so_fast(f, R, c.r2, u);
                         x = so_hit(f, T, R, c.r2, u) ? 1u : 0u;
                     }
-                    mismatch += (q != 2u && q != x) ? 1u : 0u;
-                    exact_runs += q == 2u ? 1u : 0u;
-                    if (MC != 1) run_exact(i, k);
+                    mismatch += (a != 2u && a != x) ? 1u : 0u;
+                    exact_runs += a == 2u ? 1u : 0u;
+                    run_exact(i, k);
                 } else {
                     run_exact(i, k);
                 }

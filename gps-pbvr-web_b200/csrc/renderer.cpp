@@ -223,6 +223,7 @@ static FrameConst make_frame(const gpsb_renderer* r, const gpsb_camera& cam, con
     f.fp_comp = r->fp_comp;
     f.fp_kappa = r->fp_kappa;
     f.fast_mode = r->fast_mode;
+    f.ff = gxf::make_frame(f.W, f.H, f.cx, f.cy, f.near_z, f.jitter_sd, f.flags);
     return f;
 }
 

@@ -14,7 +14,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libgpsoracle.so")
 SOURCES = ["o1_core.cpp", "o2_mirror.cpp"]
 HEADERS = [os.path.join(HERE, "..", "include", "gpsb200.h"),
-           os.path.join(HERE, "..", "gps-pbvr-web_b200", "csrc", "fmath.h")]
+           os.path.join(HERE, "..", "gps-pbvr-web_b200", "csrc", "fmath.h"),
+           os.path.join(HERE, "..", "gps-pbvr-web_b200", "csrc", "pbvr_fast.h")]
 
 
 def _stale() -> bool:
