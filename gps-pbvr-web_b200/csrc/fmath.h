@@ -96,9 +96,13 @@ GX_HD float clamp_(float x, float lo, float hi) { return fmin_(fmax_(x, lo), hi)
 
 // WGSL u32(f32): truncation toward zero, saturated to [0, 2^32 - 1]; NaN gives 0.
 GX_HD uint32_t f2u(float x) {
+#if defined(__CUDA_ARCH__)
+    return __float2uint_rz(x);  // saturates the same way (checked over every float)
+#else
     if (!(x > 0.0f)) return 0u;
     if (x >= 4294967296.0f) return 0xFFFFFFFFu;
     return (uint32_t)x;
+#endif
 }
 
 constexpr float kLn2Hi = 0.693147182f;          // nearest f32 to ln 2
@@ -262,7 +266,7 @@ GX_HD uint32_t pcg(uint32_t v) {
 GX_HD uint32_t particle_seed(uint32_t splat_id, uint32_t particle_index, uint32_t frame_index) {
     uint32_t s = pcg(splat_id * 747796405u + particle_index + 1u);
     s = pcg(s ^ (frame_index * 2654435761u + 1u));
-    return s == 0u ? 1u : s;
+    return s > 1u ? s : 1u;
 }
 // U[0,1) from the top 24 bits of the advanced state (gps_splat.wgsl:73-76): exact in f32.
 GX_HD float next_u(uint32_t* st) {

@@ -49,8 +49,8 @@ enum : uint32_t { CD_NONE = 0u, CD_POISSON_CAP = 1u, CD_FIXED = 2u, CD_POISSON =
 //         r2.z footprint  r3.xy half a subpixel minus the fast position's bound
 //   PBVR: r0 (mean.xy, depth, o)  r1.x keep, r1.y h(min(o, 1-1e-6))  r2 (pos, inv_xx)
 //         r3 (inv_xy, inv_yy)  r4 (l00, l10, l11)  r5 (l20, l21, l22)
-//   SO  : r0 (mean.xy, depth, o)  r1 (lo.xy, size.xy)  r2 (inv_xx, inv_xy, inv_yy, peak_tau)
-//         r3.x = bits(floor((2^32 - 1) / width))  r3.w sparse
+//   SO  : r0 (mean.xy, depth, o)  r1 (bits(lo.xy), size.xy)  r2 (inv_xx, 2 inv_xy, inv_yy, peak_tau)
+//         r3 = bits(floor((2^32 - 1) / width), width, samples - 1), sparse
 constexpr int kRecF4 = 12;
 
 // Statistics words (64-bit): gpsb_stats field order.

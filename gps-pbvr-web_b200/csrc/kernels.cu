@@ -198,9 +198,10 @@ __global__ void __launch_bounds__(128) k_geometry(FrameConst f, const float4* __
                     if (sparse) cd = make_uint2(f2b((float)count * density * peak_tau), CD_POISSON);
                     else cd = make_uint2(count, CD_FIXED);
                     R[0] = r0;
-                    R[1] = make_float4(lo_x, lo_y, sz_x, sz_y);
-                    R[2] = make_float4(pr.c * invdet, -pr.b * invdet, pr.a * invdet, peak_tau);
-                    R[3] = make_float4(__uint_as_float(0xFFFFFFFFu / f2u(sz_x)), F_(0.0), F_(0.0), sparse ? F_(1.0) : F_(0.0));
+                    R[1] = make_float4(__uint_as_float(f2u(lo_x)), __uint_as_float(f2u(lo_y)), sz_x, sz_y);
+                    R[2] = make_float4(pr.c * invdet, F_(2.0) * (-pr.b * invdet), pr.a * invdet, peak_tau);
+                    R[3] = make_float4(__uint_as_float(0xFFFFFFFFu / f2u(sz_x)), __uint_as_float(f2u(sz_x)), __uint_as_float(count - 1u),
+                                       sparse ? F_(1.0) : F_(0.0));
                 }
             }
         } else {
@@ -674,7 +675,8 @@ void launch_fast_bounds(uint32_t* out, cudaStream_t st) {
 // draw's squared distance (particle_pass, gps_splat.wgsl:686-703): integer arithmetic and single
 // roundings in the shader's order, shared by the exact and the fast decision. Divisions by the
 // rectangle's width and by the subpixel count are multiplications by their reciprocals: R[3].x
-// holds floor((2^32 - 1) / width), whose quotient is at most one too small.
+// holds floor((2^32 - 1) / width), whose quotient is at most one too small; R[1].xy, R[3].y and R[3].z hold the
+// rectangle's corner, its width and its last sample as integers.
 struct SoCell {
     uint32_t cell;  // subpixel index
     float r2;       // squared Mahalanobis distance of the jittered sample
@@ -682,10 +684,9 @@ struct SoCell {
 __device__ __forceinline__ SoCell so_cell(const FrameConst& f, uint32_t k, uint32_t& rs, const float4* R) {
     const float4 r0 = R[0], b = R[1], inv = R[2], r3 = R[3];
     const uint32_t side = f.side, samples = f.S;
-    const uint32_t bz = f2u(b.z);
+    const uint32_t bz = __float_as_uint(r3.y);
     uint32_t cell = k;
-    if (r3.w > F_(0.0))
-        cell = min(f2u(gx::next_u(&rs) * b.z * b.w * (float)samples), bz * f2u(b.w) * samples - 1u);
+    if (r3.w > F_(0.0)) cell = min(f2u(gx::next_u(&rs) * b.z * b.w * (float)samples), __float_as_uint(r3.z));
     uint32_t pixel = cell, sub_i = 0u;
     if (side > 1u) {
         pixel = side == 2u ? cell >> 2 : side == 4u ? cell >> 4 : cell / 9u;
@@ -696,7 +697,7 @@ __device__ __forceinline__ SoCell so_cell(const FrameConst& f, uint32_t k, uint3
         col -= bz;
         ++row;
     }
-    const uint32_t xx = f2u(b.x) + col, yy = f2u(b.y) + row;
+    const uint32_t xx = __float_as_uint(b.x) + col, yy = __float_as_uint(b.y) + row;
     const float n1 = gx::next_u(&rs);
     const float n2 = gx::next_u(&rs);
     float uvx = n1, uvy = n2;
@@ -715,7 +716,7 @@ __device__ __forceinline__ SoCell so_cell(const FrameConst& f, uint32_t k, uint3
     }
     const float dx = (float)xx + uvx - r0.x, dy = (float)yy + uvy - r0.y;
     SoCell c;
-    c.r2 = fmax_(inv.x * dx * dx + F_(2.0) * inv.y * dx * dy + inv.z * dy * dy, F_(0.0));
+    c.r2 = fmax_(inv.x * dx * dx + inv.y * dx * dy + inv.z * dy * dy, F_(0.0));  // inv.y is doubled (exact)
     c.cell = (yy * f.W + xx) * samples + sub_i;
     return c;
 }
@@ -806,12 +807,6 @@ __device__ __forceinline__ uint32_t gps_fast(const FrameConst& f, const float* l
 
 constexpr int kPT = 256;               // threads per particle block
 constexpr uint32_t kRing = 64;         // per-warp ring of undecided particles (uint2 entries)
-#ifndef GPSB_FAST_GIVE_UP
-#define GPSB_FAST_GIVE_UP 10
-#endif
-// undecided lanes of one step above which a warp stops the PBVR fast test for the rest of its unit
-// (measured on the bench views: 10 beats 4, 7, 16, 24 and never giving up)
-constexpr uint32_t kFastGiveUp = GPSB_FAST_GIVE_UP;
 static_assert(kTabFloats % 2 == 0, "the unit table after the maths tables needs 8-byte alignment");
 
 // Largest j in [lo, hi) with off(j) <= v, by a 32-ary warp search (off(lo) <= v must hold).
@@ -839,7 +834,8 @@ constexpr bool kStageTabs = MC == 1 || FM != 1;
 // Persistent particle kernel. A unit of work is up to steps * 32 consecutive particles of one
 // ensemble; every warp by itself takes the next unit from a device counter, finds its first list
 // entry with a 32-ary search and steps through it 32 particles at a time, lane l on particle
-// p + l. Each particle is mapped to (splat i, k) through the compact list, regenerated from its own
+// p + l. Units are long (128 steps by default: near view 45.8 ms for 4 ensembles, 52.0 with 16)
+// because each one pays for its search and for its last, partly filled run of undecided particles. Each particle is mapped to (splat i, k) through the compact list, regenerated from its own
 // stream particle_seed(i, k + 1, seed) and written with one 64-bit atomicMin of (depth key << 32 | i),
 // which equals the reference's depth pass followed by the colour pass (gps_splat.wgsl:276-281).
 // Ensembles flagged skipped get no work.
@@ -850,13 +846,14 @@ constexpr bool kStageTabs = MC == 1 || FM != 1;
 // records they load: the list entries of the step are one coalesced 256-byte read, the boundaries
 // within it a __reduce_or_sync of one bit each. No list staging in shared memory, no block barrier.
 // Measured against tiles of 4096 particles per block, 16 consecutive ones per thread, staged lists
-// and the exact path for GPS and ScreenOccupancy (B200): GPS, 560k splats, 1280x720, 2x2 subpixels, 4
-// ensembles (773M particles) 9.14 -> 4.9 ms, 252 -> 190 instructions per particle; ScreenOccupancy,
-// 2M splats, 1920x1080, 2 ensembles (4.9G particles) 56.4 -> 34 ms, 379 -> 220 instructions.
+// and the exact path for GPS and ScreenOccupancy (B200): a whole GPS frame, 560k splats, 1280x720, 2x2
+// subpixels, 4 ensembles (773M particles) 10.9 -> 5.8 ms; ScreenOccupancy, 2M splats, 1920x1080, two
+// cameras of 2 ensembles (9.8G particles) 114.6 -> 57.4 ms.
 //
 // MC: 0 GPS, 1 PBVR, 2 ScreenOccupancy; FM: fast decisions (0 off, 1 on, 2 validate: exact always,
 // disagreements counted), template parameters so each variant gets its own register allocation.
-template <int MC, int FM>
+// FL: the PBVR flags known at compile time (never ViewConditioned), or -1: read from f.
+template <int MC, int FM, int FL = -1>
 __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS : GPSB_PARTICLE_MIN_BLOCKS)
     k_particles(FrameConst f, const float4* __restrict__ rec, const float* __restrict__ lut, const uint2* __restrict__ clist,
                 const EnsTotal* __restrict__ etot, uint32_t first_seed, uint32_t E, uint32_t max_steps, ull* sub,
@@ -870,7 +867,8 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     float* s_lut = reinterpret_cast<float*>(s_ring + (FM == 1 ? (kPT / 32) * kRing : 0));
     __shared__ uint32_t s_steps;
     const int tid = threadIdx.x, lane = tid & 31;
-    // particles per unit: max_steps * 32, fewer when the call is so small that warps would get none
+    // particles per unit: max_steps * 32, fewer when warps would get less than four units each
+    // (560k splats, far view, 4 ensembles: 0.775 ms; with one unit each 0.847)
     if (tid < 32) {
         uint64_t total = 0;
         for (uint32_t e = lane; e < E; e += 32) {
@@ -878,7 +876,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
             total += t.flags == 0u ? t.particles : 0ull;
         }
         for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-        const uint64_t want = total / ((uint64_t)gridDim.x * kPT);
+        const uint64_t want = total / ((uint64_t)gridDim.x * kPT * 4u);
         const uint32_t steps = want >= max_steps ? max_steps : want < 1u ? 1u : (uint32_t)want;
         uint64_t acc = 0;
         for (uint32_t e0 = 0; e0 < E; e0 += 32) {
@@ -914,6 +912,8 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     const uint64_t PS = (uint64_t)f.W * f.H * f.S;
     const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);  // lanes up to this one
     uint2* ring = s_ring + (size_t)(tid >> 5) * kRing;
+    const uint32_t flags = FL >= 0 ? (uint32_t)FL : f.flags;
+    const bool vc = FL >= 0 ? false : f.method == 3u;
     uint32_t points = 0, writes = 0, exact_runs = 0, mismatch = 0;
     uint32_t next = 0u;
     if (lane == 0) next = atomicAdd(unit_counter, 1u);
@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                 q[4 * c + 2] = v.z;
                 q[4 * c + 3] = v.w;
             }
-            if (f.method == 3u) keep = __ldg(&rec[(size_t)i * kRecF4 + 1].x);
+            if (vc) keep = __ldg(&rec[(size_t)i * kRecF4 + 1].x);
             curq = i;
         };
         auto exact = [&](uint32_t i, uint32_t k, const float4* X) {
@@ -991,7 +991,6 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
             }
         };
         uint32_t head = 0u, count = 0u;
-        bool fast = true;  // warp-uniform
         for (uint32_t d0 = 0; d0 < left; d0 += 32u) {
             const uint32_t pp0 = p0 + d0;  // first particle of the step
             const bool act = d0 + (uint32_t)lane < left;
@@ -1019,7 +1018,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                     nx = ej + 1u < nz ? (adv < 32u ? __shfl_sync(0xffffffffu, en.y, adv & 31u) : __ldg(&L[ej + 1u].y)) : n_part;
                 }
             }
-            if (FM == 1 && (MC != 1 || fast)) {
+            if (FM == 1) {
                 // converged fast step: every lane evaluates a particle (a lane past the unit one it does
                 // not own, whose answer is ignored); where any lane's splat changed all lanes reload
                 if (MC == 1) {
@@ -1039,7 +1038,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                 } else if (MC == 1) {
                     Mufu ap;
                     gxf::Point P;
-                    a = gxf::decide(ap, f.ff, f.flags, f.method == 3u, keep, rs, q, P);
+                    a = gxf::decide(ap, f.ff, flags, vc, keep, rs, q, P);
                     if (act && a == 3u) {
                         // on screen: with the subpixel settled and the depth surely behind the subpixel's
                         // word (which only ever decreases) the write has no effect but its count
@@ -1050,7 +1049,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                             a = 1u;
                             if (on) {
                                 const uint32_t cell = cell_of(f, cx, cy);
-                                if (f.flags & FLAG_CENTRE) {
+                                if (flags & FLAG_CENTRE) {
                                     splat_write(S, cell, __ldg(&rec[(size_t)i * kRecF4].z), i);
                                     ++writes;
                                 } else {
@@ -1080,7 +1079,6 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                 if (need) ring[(head + count + (uint32_t)__popc(bal & upto) - 1u) & (kRing - 1u)] = make_uint2(i, k);
                 count += n;
                 exact_runs += need ? 1u : 0u;
-                if (n > kFastGiveUp) fast = false;
                 if (count >= 32u) {
                     __syncwarp();
                     const uint2 en = ring[(head + (uint32_t)lane) & (kRing - 1u)];
@@ -1155,7 +1153,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     if (lane == 0 && mv) atomicAdd(&stats[ST_FAST_MISMATCH], mv);
 }
 
-template <int MC, int FM>
+template <int MC, int FM, int FL = -1>
 static void launch_particles_t(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
                                const EnsTotal* etot, uint32_t first_seed, uint32_t E, unsigned long long* sub,
                                uint32_t* unit_counter, unsigned long long* stats, int grid, int steps, cudaStream_t st) {
@@ -1168,10 +1166,10 @@ static void launch_particles_t(const FrameConst& fc, const float4* rec, const fl
     cudaGetDevice(&dev);
     const bool known = dev >= 0 && dev < 64;
     if (smem > 48 * 1024 && (!known || smem > attr[dev])) {
-        cudaFuncSetAttribute(k_particles<MC, FM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_particles<MC, FM, FL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (known) attr[dev] = smem;
     }
-    k_particles<MC, FM><<<grid, kPT, smem, st>>>(fc, rec, lut, clist, etot, first_seed, E, (uint32_t)steps, sub, unit_counter, stats);
+    k_particles<MC, FM, FL><<<grid, kPT, smem, st>>>(fc, rec, lut, clist, etot, first_seed, E, (uint32_t)steps, sub, unit_counter, stats);
 }
 
 void launch_particles(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
@@ -1192,7 +1190,14 @@ void launch_particles(const FrameConst& fc, const float4* rec, const float* lut,
         else if (fm == 2u) go(mc, std::integral_constant<int, 2>());
         else go(mc, std::integral_constant<int, 0>());
     };
-    if (fc.method == 0u) method(std::integral_constant<int, 0>());
+    // the two common flag sets of the fast PBVR decisions, compiled with the flags known
+    constexpr int kJR = (int)(FLAG_JITTER | FLAG_RADIAL), kJ = (int)FLAG_JITTER;
+    const bool pbvr = fc.method == 1u || fc.method == 2u;
+    if (pbvr && fm == 1u && fc.flags == (uint32_t)kJR)
+        launch_particles_t<1, 1, kJR>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, items, st);
+    else if (pbvr && fm == 1u && fc.flags == (uint32_t)kJ)
+        launch_particles_t<1, 1, kJ>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, items, st);
+    else if (fc.method == 0u) method(std::integral_constant<int, 0>());
     else if (fc.method == 4u) method(std::integral_constant<int, 2>());
     else method(std::integral_constant<int, 1>());
 }

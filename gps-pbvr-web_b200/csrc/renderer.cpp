@@ -308,7 +308,7 @@ static gpsb_status render_batch(gpsb_renderer* r, const FrameConst& f, bool part
             sc.kernels(1);
             launch_particles(f, r->rec.as<float4>(), r->lut.as<float>(), r->clist.as<uint2>(), r->etot.as<EnsTotal>(),
                              first_seed, E, r->sub.as<ull_t>(), cnt + 1, stats,
-                             r->sm_count * (int)r->particle_blocks_per_sm, (int)r->particle_items, r->stream);
+                             r->sm_count * (int)r->particle_blocks_per_sm, (int)r->particle_items * 8, r->stream);
             CK(r, cudaGetLastError(), "particle kernel");
         }
     } else {
