@@ -105,20 +105,40 @@ __device__ inline Proj project(const FrameConst& f, float4 g0, float4 g1, float4
     return pr;
 }
 
-// dilog (gps_splat.wgsl:79-94)
+// dilog (gps_splat.wgsl:79-94). The series' terms fall (x <= 1/2), and so do their quotients, so once
+// adding one leaves the sum unchanged every later one does too and the loop ends there with the
+// same bits as all 30 terms (at most 19 are needed). The division by k^2 is the correctly
+// rounded quotient from the rounded reciprocal, one exact remainder and one correction (Markstein, IBM
+// J. Res. Dev. 34 (1990)); the terms it changes the sum by are far above the subnormals.
+struct SquareRcp {
+    float sq[32], rc[32];
+    constexpr SquareRcp() : sq(), rc() {
+        for (int k = 1; k < 32; ++k) {
+            sq[k] = (float)(k * k);
+            rc[k] = (float)(1.0 / (double)(k * k));
+        }
+    }
+};
+static __constant__ SquareRcp kSquares = SquareRcp();
 __device__ inline float dilog_series(float x) {
     float term = x, sum = x;
+#pragma unroll 1
     for (uint32_t k = 2; k < 32; ++k) {
         term = term * x;
-        sum = sum + div_(term, (float)(k * k));
+        const float sq = kSquares.sq[k], rc = kSquares.rc[k];
+        const float q = term * rc;
+        const float next = sum + __fmaf_rn(__fmaf_rn(-q, sq, term), rc, q);
+        if (next == sum) break;
+        sum = next;
     }
     return sum;
 }
 __device__ inline float dilog(float x) {
     if (x >= F_(1.0)) return gxc::kDilogOne;
     if (x <= F_(0.0)) return F_(0.0);
-    if (x <= F_(0.5)) return dilog_series(x);
-    return gxc::kDilogOne - gx::log(x) * gx::log(F_(1.0) - x) - dilog_series(F_(1.0) - x);
+    const float s = dilog_series(x <= F_(0.5) ? x : F_(1.0) - x);  // one loop for the lanes of both halves
+    if (x <= F_(0.5)) return s;
+    return gxc::kDilogOne - gx::log(x) * gx::log(F_(1.0) - x) - s;
 }
 // inv_dilog / corrected_radius (gps_splat.wgsl:97-140), Li2(o) precomputed per splat
 __device__ inline float inv_dilog(float tgt, float hi_in) {

@@ -184,6 +184,20 @@ GX_HD float exp_t(float x, const float* T) {
     return (v * pow2i(n + 64)) * pow2i(-64);
 }
 GX_HD float exp(float x) { return exp_t(x, tab_exp()); }
+// exp_t for arguments known to lie in [-80, 0]: the same arithmetic without the range tests, so the
+// same result bit for bit.
+GX_HD float exp_mid(float x, const float* T) {
+    const float kf = rint_(x * kExpK);
+    float r = fma_(kf, -kExpLHi, x);
+    r = fma_(kf, -kExpLLo, r);
+    const int k = (int)kf;
+    float th, tl;
+    ld2(T, k & 63, &th, &tl);
+    float q = fma_(r, 4.16666679e-2f, 1.66666672e-1f);
+    q = fma_(r, q, 0.5f);
+    const float p = fma_(r * r, q, r);
+    return (th + fma_(th, p, tl)) * pow2i(k >> 6);
+}
 
 GX_HD float log_t(float x, const float* T) {
     uint32_t b = f2b(x);

@@ -7,9 +7,9 @@
 //                   peer groups (each lane ORs its bit into its digit's word of a per-warp row in
 //                   shared memory and reads the word back), resolves tile offsets by a decoupled
 //                   lookback per digit and scatters. Digit width 4, 6 or 8 bits.
-//   tile binning    (tile id, sorted rank) entries, stably sorted by tile, give every screen tile its
-//                   splats in depth order.
-//   k_blend         one block per tile, front-to-back f32 blending with early termination
+//   binning         (bin, splat id) entries in depth order, stably sorted by bin, give every screen bin
+//                   its splats in depth order.
+//   k_blend         one block per bin, front-to-back f32 blending with early termination
 //                   (replaces the rgba16f back-to-front raster of gps_sorted_draw.wgsl:15-38 and the
 //                   blend state of sorted.rs:125-138), written to accum = (rgb, 1) like sp_resolve.
 //   k_composite     gps_composite.wgsl:41-55 into a headless RGBA8 buffer.
@@ -94,18 +94,25 @@ __global__ void __launch_bounds__(256) k_radix_hist(const uint32_t* __restrict__
         if (s[k]) atomicAdd(&hist[k], s[k]);
 }
 
-// exclusive scan of every pass's histogram, in place (one block)
+// exclusive scan of every pass's histogram, in place: one block of BINS threads per pass (a single
+// thread per pass took 8 us for 256 bins, a chain of dependent loads and stores; this takes 2 us)
 template <int BITS>
-__global__ void k_radix_hist_scan(uint32_t* hist, int passes) {
-    constexpr int BINS = 1 << BITS;
-    int p = threadIdx.x;
-    if (p >= passes) return;
-    uint32_t acc = 0;
-    for (int d = 0; d < BINS; ++d) {
-        uint32_t c = hist[p * BINS + d];
-        hist[p * BINS + d] = acc;
-        acc += c;
+__global__ void k_radix_hist_scan(uint32_t* hist) {
+    constexpr int BINS = 1 << BITS, WARPS = (BINS + 31) / 32;
+    __shared__ uint32_t s_sum[WARPS];
+    const int tid = threadIdx.x, lane = tid & 31;
+    uint32_t* h = hist + blockIdx.x * BINS;
+    const uint32_t c = tid < BINS ? h[tid] : 0u;
+    uint32_t incl = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
+    if (lane == 31) s_sum[tid >> 5] = incl;
+    __syncthreads();
+    uint32_t base = 0;
+    for (int w = 0; w < tid >> 5; ++w) base += s_sum[w];
+    if (tid < BINS) h[tid] = base + incl - c;
 }
 
 template <int BITS>
@@ -335,9 +342,7 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS>::min_blocks) k_onesw
 }
 
 void radix_release(RadixScratch& s) {
-    if (s.hist) cudaFree(s.hist);
-    if (s.lookback) cudaFree(s.lookback);
-    if (s.counters) cudaFree(s.counters);
+    if (s.mem) cudaFree(s.mem);
     s = RadixScratch();
 }
 
@@ -354,44 +359,41 @@ static void onesweep_launch(uint32_t tiles, const uint32_t* ik, const uint32_t* 
 
 template <int BITS>
 static cudaError_t radix_impl(RadixScratch& s, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t n,
-                              int key_bits, uint32_t* err, cudaStream_t st) {
+                              int key_bits, uint32_t* err, bool placed, cudaStream_t st) {
     constexpr int BINS = 1 << BITS;
     int passes = std::max(1, (key_bits + BITS - 1) / BITS);
     if (passes > kMaxPasses) return cudaErrorInvalidValue;
     const uint32_t tiles = (n + RsShape<BITS>::tile - 1) / RsShape<BITS>::tile;
-    size_t hb = (size_t)passes * BINS * 4, lbb = (size_t)passes * std::max(tiles, 1u) * BINS * 4;
+    // [digit histograms][tile counters][lookback words], cleared together
+    constexpr size_t kCounterWords = 32;  // the lookback rows start on a 128-byte line
+    const size_t hw = ((size_t)passes * BINS + 31) / 32 * 32,
+                 words = hw + kCounterWords + (size_t)passes * std::max(tiles, 1u) * BINS;
     cudaError_t e;
-    if (hb > s.hist_bytes) {
-        if (s.hist) cudaFree(s.hist);
-        s.hist = nullptr;
-        if ((e = cudaMalloc(&s.hist, hb)) != cudaSuccess) return e;
-        s.hist_bytes = hb;
+    if (words * 4 > s.bytes) {
+        if (s.mem) cudaFree(s.mem);
+        s.mem = nullptr;
+        s.bytes = 0;
+        if ((e = cudaMalloc(&s.mem, words * 4)) != cudaSuccess) return e;
+        s.bytes = words * 4;
     }
-    if (lbb > s.lookback_bytes) {
-        if (s.lookback) cudaFree(s.lookback);
-        s.lookback = nullptr;
-        if ((e = cudaMalloc(&s.lookback, lbb)) != cudaSuccess) return e;
-        s.lookback_bytes = lbb;
-    }
-    if (!s.counters && (e = cudaMalloc(&s.counters, kMaxPasses * 4)) != cudaSuccess) return e;
-    uint32_t* hist = (uint32_t*)s.hist;
-    cudaMemsetAsync(hist, 0, hb, st);
-    cudaMemsetAsync(s.lookback, 0, lbb, st);
-    cudaMemsetAsync(s.counters, 0, kMaxPasses * 4, st);
+    uint32_t* hist = (uint32_t*)s.mem;
+    uint32_t* counters = hist + hw;
+    uint32_t* lookback = counters + kCounterWords;
+    cudaMemsetAsync(hist, 0, words * 4, st);
     if (n == 0) return cudaGetLastError();
-    k_radix_hist<BITS><<<std::min<uint32_t>((n + 4095) / 4096, 1184u), 256, 0, st>>>(ka, n, passes, hist);
-    k_radix_hist_scan<BITS><<<1, 32, 0, st>>>(hist, passes);
     // ping-pong so that the last pass writes (kb, vb)
     uint32_t *ik = ka, *iv = va, *ok = kb, *ov = vb;
     if (passes % 2 == 0) { ok = ka; ov = va; ik = kb; iv = vb; }
-    if (passes % 2 == 0) {
+    k_radix_hist<BITS><<<std::min<uint32_t>((n + 4095) / 4096, 1184u), 256, 0, st>>>(placed ? ik : ka, n, passes, hist);
+    k_radix_hist_scan<BITS><<<passes, BINS < 32 ? 32 : BINS, 0, st>>>(hist);
+    if (passes % 2 == 0 && !placed) {
         // first pass reads the input from (ka, va): copy it to (kb, vb) so the parity works out
         cudaMemcpyAsync(kb, ka, (size_t)n * 4, cudaMemcpyDeviceToDevice, st);
         cudaMemcpyAsync(vb, va, (size_t)n * 4, cudaMemcpyDeviceToDevice, st);
     }
     for (int p = 0; p < passes; ++p) {
         onesweep_launch<BITS>(tiles, ik, iv, ok, ov, n, p * BITS, hist + p * BINS,
-                              (uint32_t*)s.lookback + (size_t)p * tiles * BINS, (uint32_t*)s.counters + p, err, st);
+                              lookback + (size_t)p * tiles * BINS, counters + p, err, st);
         std::swap(ik, ok);
         std::swap(iv, ov);
     }
@@ -414,10 +416,10 @@ constexpr size_t kNoAllocWords = kNoAllocHistWords + kNoAllocCounterWords + (siz
 static __device__ __align__(256) uint32_t g_noalloc_sort_scratch[kNoAllocWords];
 
 cudaError_t radix_sort_pairs(RadixScratch& s, uint32_t* ka, uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t n,
-                             int key_bits, int digit_bits, uint32_t* err, cudaStream_t st) {
-    if (digit_bits == 4) return radix_impl<4>(s, ka, va, kb, vb, n, key_bits, err, st);
-    if (digit_bits == 6) return radix_impl<6>(s, ka, va, kb, vb, n, key_bits, err, st);
-    return radix_impl<8>(s, ka, va, kb, vb, n, key_bits, err, st);
+                             int key_bits, int digit_bits, uint32_t* err, cudaStream_t st, bool placed) {
+    if (digit_bits == 4) return radix_impl<4>(s, ka, va, kb, vb, n, key_bits, err, placed, st);
+    if (digit_bits == 6) return radix_impl<6>(s, ka, va, kb, vb, n, key_bits, err, placed, st);
+    return radix_impl<8>(s, ka, va, kb, vb, n, key_bits, err, placed, st);
 }
 
 // Device address of g_noalloc_sort_scratch on the current device. In host code the array's name is
@@ -451,87 +453,26 @@ static void* noalloc_scratch_address(cudaStream_t st, cudaError_t* err, bool* ca
     return addr[dev];
 }
 
-// ============================================================================ u32 exclusive scan
-constexpr int kScT = 256, kScI = 8, kScTile = kScT * kScI;
-
-__global__ void __launch_bounds__(kScT) k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint32_t* sums) {
-    __shared__ uint32_t s[kScT / 32];
-    uint32_t base = blockIdx.x * kScTile, v = 0;
-    for (int q = 0; q < kScI; ++q) {
-        uint32_t i = base + q * kScT + threadIdx.x;
-        if (i < n) v += in[i];
-    }
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < kScT / 32; ++w) t += s[w];
-        sums[blockIdx.x] = t;
-    }
-}
-// single block: exclusive scan of the block sums (nb <= 1024 * 16), total into *total
-__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* sums, uint32_t nb, uint32_t* total) {
-    __shared__ uint32_t s[1024];
-    const int per = (nb + 1023) / 1024;
-    uint32_t loc = 0;
-    for (int q = 0; q < per; ++q) {
-        uint32_t i = threadIdx.x * per + q;
-        if (i < nb) loc += sums[i];
-    }
-    s[threadIdx.x] = loc;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        uint32_t v = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
-        __syncthreads();
-        s[threadIdx.x] += v;
-        __syncthreads();
-    }
-    uint32_t run = s[threadIdx.x] - loc;
-    for (int q = 0; q < per; ++q) {
-        uint32_t i = threadIdx.x * per + q;
-        if (i < nb) {
-            uint32_t c = sums[i];
-            sums[i] = run;
-            run += c;
-        }
-    }
-    if (threadIdx.x == 1023) *total = s[1023];
-}
-__global__ void __launch_bounds__(kScT) k_scan_apply(uint32_t* data, uint32_t n, const uint32_t* sums) {
-    __shared__ uint32_t s[kScT];
-    uint32_t base = blockIdx.x * kScTile + threadIdx.x * kScI;
-    uint32_t v[kScI], t = 0;
-    for (int q = 0; q < kScI; ++q) {
-        v[q] = base + q < n ? data[base + q] : 0u;
-        t += v[q];
-    }
-    s[threadIdx.x] = t;
-    __syncthreads();
-    for (int o = 1; o < kScT; o <<= 1) {
-        uint32_t a = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
-        __syncthreads();
-        s[threadIdx.x] += a;
-        __syncthreads();
-    }
-    uint32_t run = sums[blockIdx.x] + s[threadIdx.x] - t;
-    for (int q = 0; q < kScI; ++q) {
-        if (base + q < n) data[base + q] = run;
-        run += v[q];
-    }
-}
-
 // ============================================================================ sorted path
+constexpr uint64_t kBin64Pixels = 4ull << 20;  // frames from this size on use 64 x 64 bins
+// Screen bins of the blend (tw x th pixels).
 struct TileGeom {
     uint32_t tw, th, tiles_x, tiles_y;
 };
 
+__device__ __forceinline__ uint32_t rect_tiles(uint2 r) {
+    if (r.x == 0xFFFFFFFFu) return 0u;
+    uint32_t w = (r.y & 0xFFFFu) - (r.x & 0xFFFFu) + 1u, h = (r.y >> 16) - (r.x >> 16) + 1u;
+    return w * h;
+}
+
 // sp_project (gps_splat.wgsl:737-777) + tile rectangle
 __global__ void __launch_bounds__(128) k_sp_project(FrameConst f, TileGeom tg, const float4* __restrict__ splats,
                                                      const float* __restrict__ sh, uint32_t* keys, uint32_t* vals,
-                                                     float4* rec, uint2* rect, ull* stats, int full) {
+                                                     float4* rec, uint2* rect, ull* stats, ull* entries, int full) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     ull demand = 0;
+    uint32_t bins = 0;  // bins of the splat's rectangle; their sum sizes the entry lists
     if (i < f.N) {
         if (full) {
             keys[i] = 0xFFFFFFu;
@@ -584,136 +525,341 @@ __global__ void __launch_bounds__(128) k_sp_project(FrameConst f, TileGeom tg, c
                 if (x1f >= 0.0f && y1f >= 0.0f && x0f <= (float)(f.W - 1) && y0f <= (float)(f.H - 1)) {
                     uint32_t x0 = (uint32_t)fmaxf(x0f, 0.0f), y0 = (uint32_t)fmaxf(y0f, 0.0f);
                     uint32_t x1 = (uint32_t)fminf(x1f, (float)(f.W - 1)), y1 = (uint32_t)fminf(y1f, (float)(f.H - 1));
-                    rect[i] = make_uint2((x0 / tg.tw) | ((y0 / tg.th) << 16), (x1 / tg.tw) | ((y1 / tg.th) << 16));
+                    const uint2 r = make_uint2((x0 / tg.tw) | ((y0 / tg.th) << 16), (x1 / tg.tw) | ((y1 / tg.th) << 16));
+                    rect[i] = r;
+                    bins = rect_tiles(r);
                 }
             }
         }
     }
     for (int o = 16; o; o >>= 1) demand += __shfl_xor_sync(0xffffffffu, demand, o);
     if ((threadIdx.x & 31) == 0 && demand) atomicAdd(&stats[ST_PROBE], demand);
+    if (full) {
+        ull b = bins;
+        for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+        if ((threadIdx.x & 31) == 0 && b) atomicAdd(entries, b);
+    }
 }
 
-__device__ __forceinline__ uint32_t rect_tiles(uint2 r) {
-    if (r.x == 0xFFFFFFFFu) return 0u;
-    uint32_t w = (r.y & 0xFFFFu) - (r.x & 0xFFFFu) + 1u, h = (r.y >> 16) - (r.x >> 16) + 1u;
-    return w * h;
+// ---- bin entries: for every splat in depth order, one (bin, splat id) pair per bin of its rectangle.
+// A block takes kEbSplats sorted splats, a warp kEbSplats / 8 of them in groups of 32 (one per lane).
+constexpr int kEbT = 256, kEbGroups = 8, kEbSplats = kEbT * kEbGroups;
+
+// sorted position of group g of this thread
+__device__ __forceinline__ uint32_t entry_splat(int g) {
+    return blockIdx.x * kEbSplats + (threadIdx.x >> 5) * (32 * kEbGroups) + g * 32 + (threadIdx.x & 31);
+}
+__device__ __forceinline__ uint2 sorted_rect(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect, uint32_t j,
+                                             uint32_t n) {
+    return j < n ? rect[__ldg(&vals_sorted[j])] : make_uint2(0xFFFFFFFFu, 0u);  // unbinned splats have no rectangle
 }
 
-__global__ void k_gather_counts(const uint32_t* __restrict__ keys_sorted, const uint32_t* __restrict__ vals_sorted,
-                                const uint2* __restrict__ rect, uint32_t n, uint32_t* cnt) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    cnt[j] = keys_sorted[j] == 0xFFFFFFu ? 0u : rect_tiles(rect[vals_sorted[j]]);
+// entries of every block's splats
+__global__ void __launch_bounds__(kEbT) k_entry_sums(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect,
+                                                     uint32_t n, uint32_t* sums) {
+    __shared__ uint32_t s[kEbT / 32];
+    uint32_t v = 0;
+#pragma unroll
+    for (int g = 0; g < kEbGroups; ++g) v += rect_tiles(sorted_rect(vals_sorted, rect, entry_splat(g), n));
+    v = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (int w = 0; w < kEbT / 32; ++w) t += s[w];
+        sums[blockIdx.x] = t;
+    }
 }
-
-__global__ void k_emit_entries(const uint32_t* __restrict__ keys_sorted, const uint32_t* __restrict__ vals_sorted,
-                               const uint2* __restrict__ rect, const uint32_t* __restrict__ offs, uint32_t n,
-                               uint32_t tiles_x, uint32_t* ekey, uint32_t* eval) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n || keys_sorted[j] == 0xFFFFFFu) return;
-    uint2 r = rect[vals_sorted[j]];
-    if (r.x == 0xFFFFFFFFu) return;
-    uint32_t o = offs[j];
-    for (uint32_t ty = r.x >> 16; ty <= (r.y >> 16); ++ty)
-        for (uint32_t tx = r.x & 0xFFFFu; tx <= (r.y & 0xFFFFu); ++tx) {
-            ekey[o] = ty * tiles_x + tx;
-            eval[o] = j;
-            ++o;
+// single block: exclusive scan of the block sums, in place
+__global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* sums, uint32_t nb) {
+    __shared__ uint32_t s[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t base = 0;
+    for (uint32_t b0 = 0; b0 < nb; b0 += 1024) {
+        const uint32_t i = b0 + threadIdx.x, c = i < nb ? sums[i] : 0u;
+        uint32_t incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
         }
-}
-
-__global__ void k_tile_ranges(const uint32_t* __restrict__ ekey, uint32_t m, uint2* ranges) {
-    uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= m) return;
-    uint32_t t = ekey[o];
-    if (o == 0 || ekey[o - 1] != t) ranges[t].x = o;
-    if (o == m - 1 || ekey[o + 1] != t) ranges[t].y = o + 1;
-}
-
-// One block per screen tile: pixels blend their tile's splats nearest first.
-template <int TW, int TH>
-__global__ void __launch_bounds__(TW* TH) k_blend(uint32_t W, uint32_t H, uint32_t tiles_x, const uint2* __restrict__ ranges,
-                                                 const uint32_t* __restrict__ erank, const uint32_t* __restrict__ vals_sorted,
-                                                 const float4* __restrict__ rec, float bg0, float bg1, float bg2,
-                                                 float4* accum) {
-    constexpr int NT = TW * TH;
-    __shared__ float4 s_a[NT], s_b[NT], s_c[NT];
-    const uint32_t tile = blockIdx.x;
-    const uint32_t px = (tile % tiles_x) * TW + threadIdx.x % TW, py = (tile / tiles_x) * TH + threadIdx.x / TW;
-    const bool inside = px < W && py < H;
-    const float pcx = (float)px + F_(0.5), pcy = (float)py + F_(0.5);
-    const uint2 range = ranges[tile];
-    float T = F_(1.0), cr = F_(0.0), cg = F_(0.0), cb = F_(0.0);
-    bool done = !inside;
-    for (int end = (int)range.y; end > (int)range.x; end -= NT) {
-        int cnt = min(NT, end - (int)range.x);
+        if (lane == 31) s[warp] = incl;
         __syncthreads();
-        if ((int)threadIdx.x < cnt) {
-            uint32_t id = __ldg(&vals_sorted[__ldg(&erank[end - 1 - threadIdx.x])]);
-            s_a[threadIdx.x] = __ldg(&rec[3 * (size_t)id]);
-            s_b[threadIdx.x] = __ldg(&rec[3 * (size_t)id + 1]);
-            s_c[threadIdx.x] = __ldg(&rec[3 * (size_t)id + 2]);
+        if (warp == 0) {
+            uint32_t w = s[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += v;
+            }
+            s[lane] = w;  // inclusive over the warps
         }
         __syncthreads();
-        if (!done) {
-            for (int q = 0; q < cnt; ++q) {
-                float4 a = s_a[q], b = s_b[q];
-                float dx = pcx - a.x, dy = pcy - a.y;
-                float u = dx * b.x + dy * b.y;
-                float v = dx * b.z + dy * b.w;
-                float r2 = u * u + v * v;
-                if (r2 > a.w * a.w) continue;
-                float alpha = fmin_(a.z * gx::exp(-F_(0.5) * r2), F_(0.99));
-                if (alpha < gxc::kSpMinAlpha) continue;
-                float4 c = s_c[q];
-                float wgt = T * alpha;
-                cr = cr + wgt * c.x;
-                cg = cg + wgt * c.y;
-                cb = cb + wgt * c.z;
-                T = T * (F_(1.0) - alpha);
-                if (T < F_(1e-4)) {
-                    done = true;
-                    break;
-                }
+        if (i < nb) sums[i] = base + (warp ? s[warp - 1] : 0u) + incl - c;
+        base += s[31];
+        __syncthreads();
+    }
+}
+// first entry of every sorted splat
+__global__ void __launch_bounds__(kEbT) k_entry_offsets(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect,
+                                                        const uint32_t* __restrict__ sums, uint32_t n, uint32_t* __restrict__ offs) {
+    __shared__ uint32_t s[kEbT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t c[kEbGroups], v = 0;
+#pragma unroll
+    for (int g = 0; g < kEbGroups; ++g) {
+        c[g] = rect_tiles(sorted_rect(vals_sorted, rect, entry_splat(g), n));
+        v += c[g];
+    }
+    v = __reduce_add_sync(0xffffffffu, v);
+    if (lane == 0) s[warp] = v;
+    __syncthreads();
+    uint32_t base = sums[blockIdx.x];
+    for (int w = 0; w < warp; ++w) base += s[w];
+#pragma unroll
+    for (int g = 0; g < kEbGroups; ++g) {
+        uint32_t incl = c[g];
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t a = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += a;
+        }
+        const uint32_t j = entry_splat(g);
+        if (j < n) offs[j] = base + incl - c[g];
+        base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+}
+// The entries. A warp writes kEwEntries consecutive ones, whatever the splats' sizes: it finds the
+// first one's splat by a binary search in the offsets and steps on 32 entries at a time, the splats
+// that begin within a step found by one bit per lane. (One thread per splat writing its entries one by
+// one took 4.4 ms at 6M splats, 3840x2160, where some splats cover the whole frame; one warp per 32
+// splats 0.85 ms, as the nearest splats, neighbours in depth order, are the largest.)
+constexpr uint32_t kEwEntries = 512;
+__global__ void __launch_bounds__(256) k_entries(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect,
+                                                 const uint32_t* __restrict__ offs, uint32_t n, uint32_t tiles_x, uint32_t m,
+                                                 uint32_t* __restrict__ ekey, uint32_t* __restrict__ eval) {
+    const uint32_t lane = threadIdx.x & 31u, upto = 0xFFFFFFFFu >> (31u - lane);
+    const uint32_t first = ((blockIdx.x * 256u + threadIdx.x) >> 5) * kEwEntries;
+    if (first >= m) return;
+    const uint32_t last = m - first < kEwEntries ? m : first + kEwEntries;
+    // splat of entry `first`: the last j with offs[j] <= first (it has entries: the next offset is larger)
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 1u) {
+        const uint32_t step = (hi - lo + 31u) / 32u, idx = lo + (lane + 1u) * step;
+        const uint32_t c = __popc(__ballot_sync(0xffffffffu, idx < hi && __ldg(&offs[idx]) <= first));
+        const uint32_t nh = lo + (c + 1u) * step;
+        lo += c * step;
+        hi = nh < hi ? nh : hi;
+    }
+    uint32_t j = lo;
+    uint32_t co = __ldg(&offs[j]), nx = j + 1u < n ? __ldg(&offs[j + 1u]) : m;
+    uint32_t id = __ldg(&vals_sorted[j]);
+    uint2 r = rect[id];
+    for (uint32_t p = first; p < last; p += 32u) {
+        uint32_t myid = id, o = co;
+        uint2 mr = r;
+        while (nx - p < 32u && nx < m) {  // splats that begin within the step, 32 candidates at a time
+            const uint32_t jj = j + 1u + lane;
+            const uint32_t of = jj < n ? __ldg(&offs[jj]) : m;
+            const uint32_t d = of - p;
+            // a splat without entries shares its offset with the next one: the last of equals counts
+            const uint32_t nxt = __shfl_down_sync(0xffffffffu, of, 1);
+            const uint32_t after = lane < 31u ? nxt : (jj + 1u < n ? __ldg(&offs[jj + 1u]) : m);
+            const bool starts = jj < n && d < 32u && after > of;
+            const uint32_t mask = __ballot_sync(0xffffffffu, starts);
+            const uint32_t bits = __reduce_or_sync(0xffffffffu, starts ? 1u << d : 0u);
+            uint32_t sid = 0;
+            uint2 sr = make_uint2(0u, 0u);
+            if (starts) {
+                sid = __ldg(&vals_sorted[jj]);
+                sr = rect[sid];
+            }
+            // the c-th starting splat of the mask serves this lane's entry
+            const uint32_t c = __popc(bits & upto);
+            uint32_t src = c - 1u;
+            if (mask & (mask + 1u)) src = c ? __fns(mask, 0u, (int)c) : 0u;  // empty splats among them
+            const uint32_t a = __shfl_sync(0xffffffffu, sid, src & 31u), b = __shfl_sync(0xffffffffu, of, src & 31u);
+            const uint32_t rx = __shfl_sync(0xffffffffu, sr.x, src & 31u), ry = __shfl_sync(0xffffffffu, sr.y, src & 31u);
+            if (c) {
+                myid = a;
+                o = b;
+                mr = make_uint2(rx, ry);
+            }
+            // step on to the last splat that began here, or past 32 empty ones
+            const uint32_t seen = __popc(__ballot_sync(0xffffffffu, jj < n && d < 32u));
+            if (mask) {
+                const uint32_t l = 31u - __clz(mask);
+                id = __shfl_sync(0xffffffffu, sid, l);
+                co = __shfl_sync(0xffffffffu, of, l);
+                r = make_uint2(__shfl_sync(0xffffffffu, sr.x, l), __shfl_sync(0xffffffffu, sr.y, l));
+            }
+            j += seen;
+            nx = j + 1u < n ? __ldg(&offs[j + 1u]) : m;
+            if (seen < 32u) break;
+        }
+        const uint32_t pos = p + lane;
+        if (pos < last) {
+            const uint32_t t = pos - o, w = (mr.y & 0xFFFFu) - (mr.x & 0xFFFFu) + 1u, ty = t / w;
+            ekey[pos] = ((mr.x >> 16) + ty) * tiles_x + (mr.x & 0xFFFFu) + (t - ty * w);
+            eval[pos] = myid;
+        }
+        // p + 32 may fall on the next splat's first entry
+        while (nx == p + 32u && nx < m) {
+            ++j;
+            co = nx;
+            nx = j + 1u < n ? __ldg(&offs[j + 1u]) : m;
+            if (nx > co) {
+                id = __ldg(&vals_sorted[j]);
+                r = rect[id];
             }
         }
-        if (__syncthreads_count(!done) == 0) break;
     }
-    if (inside) accum[(size_t)py * W + px] = make_float4(cr + T * bg0, cg + T * bg1, cb + T * bg2, F_(1.0));
 }
 
-static cudaError_t grow(void** p, size_t& cap_bytes, size_t want) {
-    if (*p && cap_bytes >= want) return cudaSuccess;
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    cap_bytes = 0;
-    cudaError_t e = cudaMalloc(p, std::max<size_t>(want, 256));
-    if (e == cudaSuccess) cap_bytes = std::max<size_t>(want, 256);
-    return e;
+// first entry of every bin (bin b: [ranges[b], ranges[b + 1])): one warp each, a 32-ary search in the
+// sorted keys
+__global__ void __launch_bounds__(128) k_bin_ranges(const uint32_t* __restrict__ ekey, uint32_t m, uint32_t bins, uint32_t* ranges) {
+    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (b > bins) return;
+    uint32_t lo = 0, n = m;  // the first position with key >= b lies in [lo, lo + n]
+    while (n) {
+        const uint32_t step = (n + 31u) / 32u, idx = lane * step;
+        const uint32_t c = __popc(__ballot_sync(0xffffffffu, idx < n && __ldg(&ekey[lo + idx]) < b));
+        if (c == 0u) break;
+        // key[lo + (c - 1) step] < b, and key[lo + c step] >= b where that is within the range
+        const uint32_t next = (c - 1u) * step + 1u, stop = c * step < n ? c * step : n;
+        lo += next;
+        n = stop - next;
+    }
+    if (lane == 0) ranges[b] = lo;
+}
+
+// Blending, nearest splats first, per pixel the arithmetic of one thread per pixel. One warp, a block of
+// its own, per region of RW x RH pixels (8 x 8, two pixels a lane) of a screen bin: it reads the bin's
+// entries 32 at a time, each lane tests one record against the region, and the warp steps only through
+// those that can touch it. Bound: instruction issue and, at the end, the longest regions; warps
+// of their own end by themselves and leave their place to the next.
+// Measured (B200), 560k splats at 1280x720 with 32 x 32 bins: 8 x 8 regions 203 us, 16 x 8 279, 8 x 4 218;
+// bins of 16 / 64 pixels 201 / 308 us, but more entries to sort, or longer lists to test; 6M splats at
+// 3840x2160 with 64 x 64 bins: 1.19 ms, 1.22, 1.42. (A block per 16 x 16 tile with every record tested by
+// every pixel: 340 us and 1.87 ms; blocks of 8 warps per 32 x 32 bin 430 us, waiting for their
+// slowest warp.)
+template <int RW, int RH>
+__global__ void __launch_bounds__(32) k_blend(uint32_t W, uint32_t H, uint32_t tiles_x, uint32_t bw, uint32_t bh,
+                                              uint32_t regions_x, const uint32_t* __restrict__ ranges,
+                                              const uint32_t* __restrict__ eid, const float4* __restrict__ rec, float bg0,
+                                              float bg1, float bg2, float4* accum) {
+    constexpr int PX = RW * RH / 32, LH = 32 / RW;  // a lane's pixels are LH rows apart
+    __shared__ float4 s_a[32], s_b[32], s_c[32];
+    __shared__ __align__(8) float s_exp[gx::kExpNodes * 2];
+    const int lane = threadIdx.x;
+    for (int k = lane; k < gx::kExpNodes * 2; k += 32) s_exp[k] = gx::kExpTabD[k];
+    const uint32_t rx = (blockIdx.x % regions_x) * RW, ry = (blockIdx.x / regions_x) * RH;
+    const uint32_t tile = (ry / bh) * tiles_x + rx / bw;
+    const uint32_t px = rx + (lane % RW), py = ry + (lane / RW);  // pixels (px, py + LH j)
+    const float pcx = (float)px + F_(0.5);
+    const float mcx = (float)rx + 0.5f * RW, mcy = (float)ry + 0.5f * RH;
+    constexpr float hx = 0.5f * (RW - 1), hy = 0.5f * (RH - 1);
+    float T[PX], cr[PX], cg[PX], cb[PX];
+    bool live = false;
+#pragma unroll
+    for (int j = 0; j < PX; ++j) {
+        T[j] = px < W && py + LH * j < H ? F_(1.0) : F_(0.0);  // a pixel is done below 1e-4
+        cr[j] = cg[j] = cb[j] = F_(0.0);
+        live |= T[j] > F_(0.0);
+    }
+    const int begin = (int)ranges[tile];
+    int end = (int)ranges[tile + 1];
+    // the records of the next 32 entries and the ids of the 32 after them are on their way meanwhile
+    float4 na, nb, nc;
+    uint32_t nid = 0;
+    auto fetch_id = [&](int e) { if (e - 1 - lane >= begin) nid = __ldg(&eid[e - 1 - lane]); };
+    auto fetch = [&](int e) {
+        if (e - 1 - lane >= begin) {
+            na = __ldg(&rec[3 * (size_t)nid]);
+            nb = __ldg(&rec[3 * (size_t)nid + 1]);
+            nc = __ldg(&rec[3 * (size_t)nid + 2]);
+        }
+    };
+    fetch_id(end);
+    fetch(end);
+    fetch_id(end - 32);
+    for (; end > begin; end -= 32) {
+        // can the record touch the region? |(u, v)| at its middle less the largest change of u and v over it
+        // (and of their roundings) against K
+        bool hit = false;
+        if (end - 1 - lane >= begin) {
+            const float dx = mcx - na.x, dy = mcy - na.y;
+            const float ux = dx * nb.x, uy = dy * nb.y, vx = dx * nb.z, vy = dy * nb.w;
+            const float eu = hx * fabsf(nb.x) + hy * fabsf(nb.y) + 1e-6f * (fabsf(ux) + fabsf(uy)) + 0.01f;
+            const float ev = hx * fabsf(nb.z) + hy * fabsf(nb.w) + 1e-6f * (fabsf(vx) + fabsf(vy)) + 0.01f;
+            const float u = fmaxf(fabsf(ux + uy) - eu, 0.0f), v = fmaxf(fabsf(vx + vy) - ev, 0.0f);
+            hit = !(u * u + v * v > na.w * na.w * 1.001f);
+        }
+        uint32_t todo = __ballot_sync(0xffffffffu, hit);
+        __syncwarp();
+        if (hit) {
+            s_a[lane] = na;
+            s_b[lane] = nb;
+            s_c[lane] = nc;
+        }
+        __syncwarp();
+        fetch(end - 32);
+        fetch_id(end - 64);
+        while (todo) {
+            const int q = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            const float4 a = s_a[q], b = s_b[q];
+            const float dx = pcx - a.x, ub = dx * b.x, vb = dx * b.z, kk = a.w * a.w;
+            bool in[PX], any = false;
+            float r2[PX];
+#pragma unroll
+            for (int j = 0; j < PX; ++j) {
+                const float dy = ((float)(py + LH * j) + F_(0.5)) - a.y;
+                const float u = ub + dy * b.y, v = vb + dy * b.w;
+                r2[j] = u * u + v * v;
+                in[j] = !(r2[j] > kk) && !(T[j] < F_(1e-4));
+                any |= in[j];
+            }
+            if (!any) continue;
+            const float4 c = s_c[q];
+#pragma unroll
+            for (int j = 0; j < PX; ++j) {
+                if (!in[j]) continue;
+                const float alpha = fmin_(a.z * gx::exp_mid(-F_(0.5) * r2[j], s_exp), F_(0.99));
+                if (alpha < gxc::kSpMinAlpha) continue;
+                const float wgt = T[j] * alpha;
+                cr[j] = cr[j] + wgt * c.x;
+                cg[j] = cg[j] + wgt * c.y;
+                cb[j] = cb[j] + wgt * c.z;
+                T[j] = T[j] * (F_(1.0) - alpha);
+            }
+        }
+        live = false;
+#pragma unroll
+        for (int j = 0; j < PX; ++j) live |= !(T[j] < F_(1e-4));
+        if (!__any_sync(0xffffffffu, live)) break;
+    }
+#pragma unroll
+    for (int j = 0; j < PX; ++j)
+        if (px < W && py + LH * j < H)
+            accum[(size_t)(py + LH * j) * W + px] = make_float4(cr[j] + T[j] * bg0, cg[j] + T[j] * bg1, cb[j] + T[j] * bg2, F_(1.0));
 }
 
 void sorted_release(SortedState& s) {
-    void* ptrs[] = {s.keys_a, s.vals_a, s.keys_b, s.vals_b, s.rec, s.tiles, s.cnt, s.scan_scratch,
+    void* ptrs[] = {s.keys_a, s.vals_a, s.keys_b, s.vals_b, s.rec, s.tiles, s.sums, s.offs, s.total,
                     s.ent_key_a, s.ent_val_a, s.ent_key_b, s.ent_val_b, s.ranges};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (s.host_total) cudaFreeHost(s.host_total);
+    if (s.counted) cudaEventDestroy(s.counted);
     radix_release(s.rs_keys);
     radix_release(s.rs_tiles);
     s = SortedState();
 }
 
-static cudaError_t exclusive_scan(SortedState& s, uint32_t* data, uint32_t n, uint32_t* total_dev, cudaStream_t st) {
-    uint32_t nb = (n + kScTile - 1) / kScTile;
-    if (nb > 1024u * 16u) return cudaErrorInvalidValue;
-    cudaError_t e = grow(&s.scan_scratch, s.scan_scratch_bytes, ((size_t)nb + 64) * 4);
-    if (e != cudaSuccess) return e;
-    uint32_t* sums = (uint32_t*)s.scan_scratch;
-    if (n == 0) return cudaMemsetAsync(total_dev, 0, 4, st);
-    k_scan_reduce<<<nb, kScT, 0, st>>>(data, n, sums);
-    k_scan_sums<<<1, 1024, 0, st>>>(sums, nb, total_dev);
-    k_scan_apply<<<nb, kScT, 0, st>>>(data, n, sums);
-    return cudaGetLastError();
+template <int RW, int RH>
+static void blend_launch(const SortedState& s, const FrameConst& f, const TileGeom& tg, float4* accum, cudaStream_t st) {
+    const uint32_t rx = (f.W + RW - 1) / RW, ry = (f.H + RH - 1) / RH;
+    k_blend<RW, RH><<<rx * ry, 32, 0, st>>>(f.W, f.H, tg.tiles_x, tg.tw, tg.th, rx, (uint32_t*)s.ranges, (uint32_t*)s.ent_val_b,
+                                            (float4*)s.rec, f.bg[0], f.bg[1], f.bg[2], accum);
 }
 
 cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* splats, const float* sh, float4* accum,
@@ -723,50 +869,60 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
     const uint32_t n = f.N;
     cudaError_t e;
     if (n > s.cap_n || !s.keys_a) {
-        void** bufs[] = {&s.keys_a, &s.vals_a, &s.keys_b, &s.vals_b, &s.cnt};
+        void** bufs[] = {&s.keys_a, &s.vals_a, &s.keys_b, &s.vals_b, &s.offs};
         for (void** b : bufs) {
             if (*b) cudaFree(*b);
             *b = nullptr;
             if ((e = cudaMalloc(b, (size_t)std::max(n, 1u) * 4 + 64)) != cudaSuccess) { *what = "sorted buffers"; return e; }
         }
-        if (s.rec) cudaFree(s.rec);
-        if (s.tiles) cudaFree(s.tiles);
-        s.rec = s.tiles = nullptr;
+        for (void** b : {&s.rec, &s.tiles, &s.sums}) {
+            if (*b) cudaFree(*b);
+            *b = nullptr;
+        }
         if ((e = cudaMalloc(&s.rec, (size_t)std::max(n, 1u) * 48)) != cudaSuccess) { *what = "sorted records"; return e; }
         if ((e = cudaMalloc(&s.tiles, (size_t)std::max(n, 1u) * 8)) != cudaSuccess) { *what = "sorted rectangles"; return e; }
+        if ((e = cudaMalloc(&s.sums, ((size_t)n / kEbSplats + 1) * 4)) != cudaSuccess) { *what = "entry sums"; return e; }
+        if (!s.total && (e = cudaMalloc(&s.total, 64)) != cudaSuccess) { *what = "entry total"; return e; }
         if (!s.host_total && (e = cudaMallocHost(&s.host_total, 64)) != cudaSuccess) { *what = "pinned total"; return e; }
+        if (!s.counted && (e = cudaEventCreateWithFlags(&s.counted, cudaEventDisableTiming)) != cudaSuccess) { *what = "event"; return e; }
         s.cap_n = n;
     }
+    // Bins of the blend: the tuned shape, and by default (16 x 16) the size with the lower time of the whole
+    // frame: large frames hold larger splats, where larger bins save more in entries than they cost in
+    // records tested (560k splats, 1280x720: 32 x 32 0.44 ms, 64 x 64 0.51, 16 x 16 0.47; 6M splats,
+    // 3840x2160: 64 x 64 2.3 ms, 32 x 32 2.9, 16 x 16 4.8). All are multiples of the blend's 8 x 8 regions.
     TileGeom tg;
     tg.tw = s.tw;
     tg.th = s.th;
+    if (s.tw == 16) tg.tw = tg.th = (uint64_t)f.W * f.H >= kBin64Pixels ? 64u : 32u;
+    else if (s.th == 8) tg.th = 16u;
     tg.tiles_x = (f.W + tg.tw - 1) / tg.tw;
     tg.tiles_y = (f.H + tg.th - 1) / tg.th;
     cudaMemsetAsync(stats + ST_PROBE, 0, 8, st);  // the probe reports the last view (sorted.rs:316-322)
+    if (full) cudaMemsetAsync(s.total, 0, 8, st);
     k_sp_project<<<(n + 127) / 128, 128, 0, st>>>(f, tg, splats, sh, (uint32_t*)s.keys_a, (uint32_t*)s.vals_a,
-                                                  (float4*)s.rec, (uint2*)s.tiles, stats, full ? 1 : 0);
+                                                  (float4*)s.rec, (uint2*)s.tiles, stats, (ull*)s.total, full ? 1 : 0);
     if ((e = cudaGetLastError()) != cudaSuccess) { *what = "sp_project kernel"; return e; }
     if (!full) return cudaSuccess;
+    // the number of bin entries sizes their buffers: it comes back while the depth sort runs
+    cudaMemcpyAsync(s.host_total, s.total, 8, cudaMemcpyDeviceToHost, st);
+    if ((e = cudaEventRecord(s.counted, st)) != cudaSuccess) { *what = "sorted path"; return e; }
     e = radix_sort_pairs(s.rs_keys, (uint32_t*)s.keys_a, (uint32_t*)s.vals_a, (uint32_t*)s.keys_b, (uint32_t*)s.vals_b, n, 24,
                          s.digit_bits, err, st);
     if (e != cudaSuccess) { *what = "depth sort"; return e; }
-    k_gather_counts<<<(n + 255) / 256, 256, 0, st>>>((uint32_t*)s.keys_b, (uint32_t*)s.vals_b, (uint2*)s.tiles, n,
-                                                     (uint32_t*)s.cnt);
-    // total of tile entries: scan, then read it back to size the entry buffers
-    e = grow(&s.scan_scratch, s.scan_scratch_bytes, ((size_t)((n + kScTile - 1) / kScTile) + 64) * 4);
-    if (e != cudaSuccess) { *what = "scan scratch"; return e; }
-    uint32_t nb = (n + kScTile - 1) / kScTile;
-    uint32_t* total_dev = (uint32_t*)s.scan_scratch + nb + 16;
-    if ((e = exclusive_scan(s, (uint32_t*)s.cnt, n, total_dev, st)) != cudaSuccess) { *what = "tile-count scan"; return e; }
-    total_dev = (uint32_t*)s.scan_scratch + nb + 16;
-    cudaMemcpyAsync(s.host_total, total_dev, 4, cudaMemcpyDeviceToHost, st);
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) { *what = "sorted path"; return e; }
-    uint32_t m = *(uint32_t*)s.host_total;
-    uint32_t n_tiles = tg.tiles_x * tg.tiles_y;
-    if (m > (1u << 30)) { *what = "more than 2^30 tile entries"; return cudaErrorInvalidValue; }
+    const uint32_t nb = (n + kEbSplats - 1) / kEbSplats;
+    k_entry_sums<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, n, (uint32_t*)s.sums);
+    k_scan_sums<<<1, 1024, 0, st>>>((uint32_t*)s.sums, nb);
+    k_entry_offsets<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, (uint32_t*)s.sums, n, (uint32_t*)s.offs);
+    if ((e = cudaEventSynchronize(s.counted)) != cudaSuccess) { *what = "sorted path"; return e; }
+    const ull total = *(ull*)s.host_total;
+    const uint32_t n_tiles = tg.tiles_x * tg.tiles_y;
+    if (total > (1ull << 30)) { *what = "more than 2^30 tile entries"; return cudaErrorInvalidValue; }
+    const uint32_t m = (uint32_t)total;
     if (m > s.cap_entries) {
         void** bufs[] = {&s.ent_key_a, &s.ent_val_a, &s.ent_key_b, &s.ent_val_b};
         size_t want = (size_t)m + m / 4 + 1024;
+        s.cap_entries = 0;
         for (void** b : bufs) {
             if (*b) cudaFree(*b);
             *b = nullptr;
@@ -777,30 +933,23 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
     if (n_tiles > s.n_tiles || !s.ranges) {
         if (s.ranges) cudaFree(s.ranges);
         s.ranges = nullptr;
-        if ((e = cudaMalloc(&s.ranges, (size_t)n_tiles * 8)) != cudaSuccess) { *what = "tile ranges"; return e; }
+        if ((e = cudaMalloc(&s.ranges, ((size_t)n_tiles + 1) * 4)) != cudaSuccess) { *what = "tile ranges"; return e; }
         s.n_tiles = n_tiles;
     }
-    cudaMemsetAsync(s.ranges, 0, (size_t)n_tiles * 8, st);
     if (m) {
-        k_emit_entries<<<(n + 255) / 256, 256, 0, st>>>((uint32_t*)s.keys_b, (uint32_t*)s.vals_b, (uint2*)s.tiles,
-                                                        (uint32_t*)s.cnt, n, tg.tiles_x, (uint32_t*)s.ent_key_a,
-                                                        (uint32_t*)s.ent_val_a);
         int tbits = 1;
         while ((1u << tbits) < n_tiles) ++tbits;
+        // the entries start in the buffer from which the sort's passes end in (ent_key_b, ent_val_b)
+        const bool even = ((tbits + 7) / 8) % 2 == 0;
+        k_entries<<<(m + 8 * kEwEntries - 1) / (8 * kEwEntries), 256, 0, st>>>(
+            (uint32_t*)s.vals_b, (uint2*)s.tiles, (uint32_t*)s.offs, n, tg.tiles_x, m,
+            (uint32_t*)(even ? s.ent_key_b : s.ent_key_a), (uint32_t*)(even ? s.ent_val_b : s.ent_val_a));
         e = radix_sort_pairs(s.rs_tiles, (uint32_t*)s.ent_key_a, (uint32_t*)s.ent_val_a, (uint32_t*)s.ent_key_b,
-                             (uint32_t*)s.ent_val_b, m, tbits, 8, err, st);
+                             (uint32_t*)s.ent_val_b, m, tbits, 8, err, st, true);
         if (e != cudaSuccess) { *what = "tile sort"; return e; }
-        k_tile_ranges<<<(m + 255) / 256, 256, 0, st>>>((uint32_t*)s.ent_key_b, m, (uint2*)s.ranges);
     }
-    if (s.tw == 16 && s.th == 16)
-        k_blend<16, 16><<<n_tiles, 256, 0, st>>>(f.W, f.H, tg.tiles_x, (uint2*)s.ranges, (uint32_t*)s.ent_val_b,
-                                                 (uint32_t*)s.vals_b, (float4*)s.rec, f.bg[0], f.bg[1], f.bg[2], accum);
-    else if (s.tw == 32 && s.th == 8)
-        k_blend<32, 8><<<n_tiles, 256, 0, st>>>(f.W, f.H, tg.tiles_x, (uint2*)s.ranges, (uint32_t*)s.ent_val_b,
-                                                (uint32_t*)s.vals_b, (float4*)s.rec, f.bg[0], f.bg[1], f.bg[2], accum);
-    else
-        k_blend<32, 32><<<n_tiles, 1024, 0, st>>>(f.W, f.H, tg.tiles_x, (uint2*)s.ranges, (uint32_t*)s.ent_val_b,
-                                                  (uint32_t*)s.vals_b, (float4*)s.rec, f.bg[0], f.bg[1], f.bg[2], accum);
+    k_bin_ranges<<<n_tiles / 4 + 1, 128, 0, st>>>((uint32_t*)s.ent_key_b, m, n_tiles, (uint32_t*)s.ranges);
+    blend_launch<8, 8>(s, f, tg, accum, st);
     if ((e = cudaGetLastError()) != cudaSuccess) { *what = "blend kernel"; return e; }
     return cudaSuccess;
 }
@@ -909,8 +1058,7 @@ extern "C" gpsb_status gpsb_sort_pairs_noalloc(uint32_t* keys_in, uint32_t* vals
     uint32_t* err = err_dev;
     uint32_t* lookback = base + kNoAllocHistWords + kNoAllocCounterWords;
     // the array keeps the previous call's contents: clear what this call needs at zero
-    e = cudaMemsetAsync(base, 0, (kNoAllocHistWords + kNoAllocCounterWords) * 4, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(lookback, 0, (size_t)passes * tiles * 256 * 4, st);
+    e = cudaMemsetAsync(base, 0, (kNoAllocHistWords + kNoAllocCounterWords + (size_t)passes * tiles * 256) * 4, st);
     uint32_t *ik = keys_in, *iv = vals_in, *ok = keys_out, *ov = vals_out;
     if (e == cudaSuccess && passes % 2 == 0) {
         // an even number of passes ends in the first buffer: start from a copy in the output
@@ -920,7 +1068,7 @@ extern "C" gpsb_status gpsb_sort_pairs_noalloc(uint32_t* keys_in, uint32_t* vals
     }
     if (e == cudaSuccess) {
         k_radix_hist<8><<<std::min<uint32_t>((n + 4095) / 4096, 1184u), 256, 0, st>>>(ik, n, passes, hist);
-        k_radix_hist_scan<8><<<1, 32, 0, st>>>(hist, passes);
+        k_radix_hist_scan<8><<<passes, 256, 0, st>>>(hist);
         for (int p = 0; p < passes; ++p) {
             onesweep_launch<8>(tiles, ik, iv, ok, ov, n, p * 8, hist + p * 256, lookback + (size_t)p * tiles * 256,
                                counters + p, err, st);

@@ -14,19 +14,17 @@ namespace gpsb {
 
 // Device scratch of one radix sort of n (key, value) pairs.
 struct RadixScratch {
-    void* hist = nullptr;      // passes x bins u32 global digit histograms (exclusive after the scan)
-    void* lookback = nullptr;  // passes x tiles x bins u32 chained-scan words
-    void* counters = nullptr;  // passes u32 tile counters
-    size_t hist_bytes = 0, lookback_bytes = 0;
-    uint32_t cap_n = 0, cap_bins = 0, cap_passes = 0;
+    void* mem = nullptr;  // passes x bins u32 digit histograms (exclusive after the scan), the passes' tile
+    size_t bytes = 0;     // counters, passes x tiles x bins u32 chained-scan words
 };
 void radix_release(RadixScratch& s);
 // Stable ascending LSD sort of `n` pairs on the low `key_bits` bits with `digit_bits` (4, 6 or 8)
 // per pass. Sorted pairs end in (keys_out, vals_out); keys_in/vals_in are used as ping-pong
-// buffers and are clobbered.
+// buffers and are clobbered. An even number of passes starts from a copy of the input in (keys_out,
+// vals_out); with `placed` the caller has put the input there.
 cudaError_t radix_sort_pairs(RadixScratch& s, uint32_t* keys_in, uint32_t* vals_in, uint32_t* keys_out,
                              uint32_t* vals_out, uint32_t n, int key_bits, int digit_bits, uint32_t* err,
-                             cudaStream_t st);
+                             cudaStream_t st, bool placed = false);
 
 struct SortedState {
     uint32_t cap_n = 0, cap_entries = 0, W = 0, H = 0, tw = 16, th = 16;
@@ -35,14 +33,15 @@ struct SortedState {
     void* keys_b = nullptr;   // sorted keys (the test hook)
     void* vals_b = nullptr;   // sorted splat ids
     void* rec = nullptr;      // n x 3 float4: (mean, o, K), (w1, w2), (rgb, -)
-    void* tiles = nullptr;    // n x uint2: tile rectangle of the splat (packed), 0 when invalid
-    void* cnt = nullptr;      // n u32 tiles touched, in sorted order, then exclusive offsets
-    void* scan_scratch = nullptr;
-    size_t scan_scratch_bytes = 0;
-    void* ent_key_a = nullptr; void* ent_val_a = nullptr;   // tile entries (tile id, sorted rank)
+    void* tiles = nullptr;    // n x uint2: bin rectangle of the splat (packed), x all ones when it has none
+    void* sums = nullptr;     // entries of each block of sorted splats, then their exclusive sums
+    void* offs = nullptr;     // n u32 first entry of every splat, in sorted order
+    void* total = nullptr;    // u64 number of bin entries, and its copy on the host with the copy's event
+    void* host_total = nullptr;
+    cudaEvent_t counted = nullptr;
+    void* ent_key_a = nullptr; void* ent_val_a = nullptr;   // bin entries (bin, splat id)
     void* ent_key_b = nullptr; void* ent_val_b = nullptr;
-    void* ranges = nullptr;   // n_tiles x uint2 [start, end)
-    void* host_total = nullptr;  // pinned u32
+    void* ranges = nullptr;   // first entry of every bin (n_tiles + 1 u32)
     uint32_t n_tiles = 0;
     int digit_bits = 8;
     RadixScratch rs_keys, rs_tiles;

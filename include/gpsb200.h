@@ -306,7 +306,8 @@ gpsb_status gpsb_debug_fmath(uint32_t which, const float* in_dev, float* out_dev
 
 /* Launch-shape tuning (no reference counterpart). Zero fields keep the current value.
  *   sort_digit_bits        radix digit width of the depth sort: 4, 6 or 8 (default 8)
- *   blend_tile_w/h         screen tiles of the sorted blend: 16x16 (default), 32x8 or 32x32
+ *   blend_tile_w/h         screen bins of the sorted blend: 16x16 (default: bins chosen by the frame's
+ *                          size), 32x8 (32x16 bins) or 32x32
  *   particle_items         work units of the particle kernel: 8, 16 (default) or 24 times 256 particles
  *   particle_blocks_per_sm persistent grid of the particle kernel (default 5 per SM)
  *   ensemble_batch         most ensembles per device batch (default 64, at most 1024) */
