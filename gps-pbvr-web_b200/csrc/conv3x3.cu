@@ -618,6 +618,278 @@ static cudaError_t launch(const bf16* x, int ldx, int xoff, int cin, const Param
     return launch_pdl(k_conv3<N, CHS>, dim3(grid), dim3(kThreads), smem, st, map, q);
 }
 
+// ============================================================================ weight gradient
+// dW[co][3 dy + dx][ci] = sum over pixels of dY[p][co] X[p + (dy - 1, dx - 1)][ci], a contraction over
+// pixels, which is the dimension the chunk-planar layout keeps contiguous: eight consecutive pixels
+// of one 8-channel plane, 16 bytes each, are a core matrix of the MMA's M- or N-major ("transposed")
+// operand layout without swizzle, channels along M or N and pixels along K. Both operands are therefore the
+// staged planes themselves: A = dY's planes (M = 128 output channels, those past cout reading other
+// bytes of shared memory into accumulator rows nobody stores), B = X's planes of a group of 8 CHX input
+// channels, shifted by one 16-byte pixel slot per dx. X is staged [row][plane][pixel], so the planes of rows
+// r, r + 1, r + 2 lie at one constant stride and one MMA of N = 3 x 8 CHX covers the three vertical taps;
+// the three dx are three accumulators of tensor memory, 9 x 8 CHX fp32 columns in all.
+// A CTA takes one input group and every splits-th unit (R rows x one segment of up to 112 pixels of an
+// image, K-steps of 16 pixels). Every kFlush steps at most the accumulators are read back and added to sums
+// in the registers of eight warps: the tensor core drops the low bits of what it adds to a growing
+// accumulator, about half a unit in the last place a step, so a chain per CTA (hundreds of steps) would
+// lose 1e-5 of the result. The sums are added to dw once.
+// Pixels and rows outside the image are TMA's zero fill in both operands.
+// Roles: lane 0 of warp 0 issues the TMA boxes (one per operand and stage), lane 0 of warp 1 the MMAs,
+// warps 2-9 (two per tensor-memory lane quarter, each half of the columns) keep the sums. Waits are
+// bounded as in k_conv3.
+// Bound: the MMAs' shared-memory reads (56 clocks per K-step and dx for 96 columns), half of the M rows
+// or more idle below 128 output channels. Measured, training step on eight 256x256 crops, eleven
+// layers: 4.40 -> 0.46 ms (threads gathering and transposing 8x8 blocks into K-major tiles, one 64-pixel
+// K-step at a time).
+constexpr int kDwSeg = 112;               // most pixels of a unit's row segment
+constexpr int kDwThreads = 320;
+constexpr int kDwSumWarps = 8;
+
+template <int CHX, int CHY>
+struct DwCfg {
+    static constexpr int R = CHY == 16 ? 2 : (CHX == 1 && CHY == 4) ? 8 : 4;
+    static constexpr int FLUSH = 24 / R;                      // units between read-backs: 168 K-steps at most
+    static constexpr int N = CHX == 1 ? 32 : 24 * CHX;        // one MMA's columns (24 used of 32 for one plane)
+    static constexpr int XB = (R + 2) * CHX * kRow, YB = R * CHY * kDwSeg * 16;  // room for the operands of a stage
+    static constexpr int STAGE = YB + XB;
+    static constexpr int S = 2;
+    // rows past cout read up to (16 - CHY) planes past the last dY row, the 25th..32nd column one X row
+    // past the last: both stay within the stage behind them or this slack
+    static constexpr size_t SLACK = 4096;
+    static_assert((16 - CHY) * kDwSeg * 16 <= XB + 4096, "reads past the last dY plane");
+    static constexpr size_t SMEM = (size_t)S * STAGE + SLACK + 1024;
+    static_assert(STAGE % 128 == 0 && SMEM <= 227 * 1024, "shared memory of one CTA");
+    static_assert(3 * N <= 512 && 3 * N % 32 == 0, "tensor-memory columns, halved in units of 16");
+};
+
+struct DwParams {
+    float* dw;  // [cout][kp], k = tap * cin + ci
+    int cout, kp, cin, groups, splits, units, segs, rowblocks, W;
+    int seg, xpx;  // pixels of a segment and of the staged X row (seg + 16), multiples of 16
+    uint32_t* err;
+};
+
+template <int CHX, int CHY>
+__global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant__ CUtensorMap ymap,
+                                                          const __grid_constant__ CUtensorMap xmap, const DwParams p) {
+    using C = DwCfg<CHX, CHY>;
+    extern __shared__ __align__(1024) uint8_t s_raw[];
+    __shared__ __align__(8) uint64_t s_full[C::S], s_empty[C::S], s_acc_full, s_acc_empty, s_drain;
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_abort;
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s_tmem)), "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 32) {
+        for (int s = 0; s < C::S; ++s) {
+            bar_init(&s_full[s], 1);
+            bar_init(&s_empty[s], 1);
+        }
+        bar_init(&s_acc_full, 1);
+        bar_init(&s_acc_empty, kDwSumWarps);
+        bar_init(&s_drain, 1);
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    const int g = blockIdx.x % p.groups, split = blockIdx.x / p.groups;
+    const int mine = (p.units - split + p.splits - 1) / p.splits;  // units of this CTA (at least one)
+    auto fail = [&]() {
+        s_abort = 1;
+        if (p.err) atomicOr(p.err, CONV3_ERR_TIMEOUT);
+    };
+    if (warp == 0) {
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0, armed = 0;
+            bool ok = true;
+            for (int i = 0; i < mine; ++i) {
+                const int u = split + i * p.splits, seg = u % p.segs, rb = (u / p.segs) % p.rowblocks,
+                          b = u / (p.segs * p.rowblocks);
+                ok = !s_abort && bar_wait(&s_empty[stage], phase ^ 1u, &s_abort);
+                if (!ok) {
+                    fail();
+                    break;
+                }
+                bar_expect(&s_full[stage], (uint32_t)(C::R * CHY * p.seg * 16 + (C::R + 2) * CHX * p.xpx * 16));
+                const uint32_t st = saddr(base + (size_t)stage * C::STAGE);
+                tma_load4(st, &ymap, 2 * p.seg * seg, 0, rb * C::R, b, &s_full[stage]);
+                tma_load4(st + C::YB, &xmap, 2 * (p.seg * seg - 1), g * CHX, rb * C::R - 1, b, &s_full[stage]);
+                armed |= 1u << stage;
+                if (++stage == C::S) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+            if (!ok) {  // this CTA's copies land before it can exit
+                for (int k = 0; k < C::S; ++k) {
+                    if (--stage < 0) {
+                        stage = C::S - 1;
+                        phase ^= 1u;
+                    }
+                    if (armed & (1u << stage))
+                        for (uint32_t i = 0; i < kSpin && !bar_test(&s_full[stage], phase); ++i) {
+                        }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t id = umma::idesc_bf16(C::N) | (1u << 15) | (1u << 16);  // A and B M/N-major
+            const uint32_t sy = (uint32_t)p.seg * 16, sx = (uint32_t)p.xpx * 16;  // bytes of a staged plane's row
+            int stage = 0;
+            uint32_t phase = 0, aphase = 0;
+            bool fresh = true;
+            for (int i = 0; i < mine; ++i) {
+                if (i > 0 && i % C::FLUSH == 0) {  // the sums have taken the accumulators
+                    if (!bar_wait(&s_acc_empty, aphase, &s_abort)) {
+                        fail();
+                        break;
+                    }
+                    aphase ^= 1u;
+                    fresh = true;
+                }
+                if (!bar_wait(&s_full[stage], phase, &s_abort)) {
+                    fail();
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int left = p.W - ((split + i * p.splits) % p.segs) * p.seg;
+                const int steps = ((left < p.seg ? left : p.seg) + 15) / 16;
+                const uint32_t st = saddr(base + (size_t)stage * C::STAGE);
+                // leading byte offset: the next 8 pixels; stride byte offset: the next 8 channels
+                const uint64_t a0 = desc(st, 128, sy), b0 = desc(st + C::YB, 128, sx);
+#pragma unroll 1
+                for (int r = 0; r < C::R; ++r) {
+#pragma unroll 1
+                    for (int k = 0; k < steps; ++k) {
+                        const uint64_t ad = a0 + (uint64_t)(r * CHY * (int)(sy / 16) + k * 16);
+                        const uint64_t bd = b0 + (uint64_t)(r * CHX * (int)(sx / 16) + k * 16);
+#pragma unroll
+                        for (int dx = 0; dx < 3; ++dx)
+                            umma::mma_bf16(tmem + (uint32_t)(dx * C::N), ad, bd + (uint64_t)dx, id, !fresh);
+                        fresh = false;
+                    }
+                }
+                umma::mma_commit(&s_empty[stage]);
+                if (i + 1 == mine || (i + 1) % C::FLUSH == 0) umma::mma_commit(&s_acc_full);
+                if (++stage == C::S) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+            // every MMA this CTA issued has completed before its tensor memory can be freed
+            umma::mma_commit(&s_drain);
+            for (uint32_t i = 0; i < kSpin && !bar_test(&s_drain, 0); ++i) {
+            }
+        }
+        __syncwarp();
+    } else {
+        constexpr int kCols = 3 * C::N / 2, kLoads = kCols / 16;
+        const int quad = warp & 3, part = (warp - 2) >> 2, co = quad * 32 + lane;
+        const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * kCols);
+        float sum[kCols];
+#pragma unroll
+        for (int c = 0; c < kCols; ++c) sum[c] = 0.0f;
+        uint32_t aphase = 0;
+        bool ok = true;
+        for (int done = 0; done < mine; done += C::FLUSH) {
+            if (!bar_wait(&s_acc_full, aphase, &s_abort)) {
+                fail();
+                ok = false;
+                break;
+            }
+            aphase ^= 1u;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (quad * 32 < p.cout) {
+#pragma unroll
+                for (int q = 0; q < kLoads; ++q) {
+                    float v[16];
+                    umma::tmem_ld16_issue(at + (uint32_t)(q * 16), v);
+                    umma::tmem_ld_wait(v);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[q * 16 + e] += v[e];
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&s_acc_empty);
+        }
+        if (ok && co < p.cout) {
+            float* row = p.dw + (size_t)co * p.kp;
+            const bool vec = p.kp % 4 == 0 && (reinterpret_cast<uintptr_t>(p.dw) & 15u) == 0;
+#pragma unroll
+            for (int h = 0; h < kCols / 4; ++h) {
+                const int col = part * kCols + 4 * h, dx = col / C::N, n = col - dx * C::N;
+                const int dy = n / (8 * CHX), ci = g * 8 * CHX + n - dy * (8 * CHX);
+                if (dy >= 3 || ci >= p.cin) continue;
+                float* o = row + (3 * dy + dx) * p.cin + ci;
+                if (vec) {
+                    atomicAdd(reinterpret_cast<float4*>(o),
+                              make_float4(sum[4 * h], sum[4 * h + 1], sum[4 * h + 2], sum[4 * h + 3]));
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) atomicAdd(o + e, sum[4 * h + e]);
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+}
+
+// (2 W, plane, H, B) view of channels [off, off + c) of a chunk-planar tensor of ld channels, as 8-byte
+// elements; boxes of px pixels x planes x rows
+static CUresult planes_map(CUtensorMap* map, const bf16* x, int ld, int off, int c, int B, int H, int W, int px, int planes,
+                           int rows) {
+    const cuuint64_t plane = (cuuint64_t)W * H * 16;
+    const cuuint64_t dims[4] = {(cuuint64_t)W * 2, (cuuint64_t)((c + 7) / 8), (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t strides[3] = {plane, (cuuint64_t)W * 16, plane * (cuuint64_t)(ld / 8)};
+    const cuuint32_t box[4] = {(cuuint32_t)(2 * px), (cuuint32_t)planes, (cuuint32_t)rows, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return encoder()(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, (void*)(x + (size_t)(off / 8) * W * H * 8), dims, strides, box,
+                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+
+template <int CHX, int CHY>
+static cudaError_t launch_dw(const bf16* dy, int ldy, const bf16* x, int ldx, int xoff, int B, int H, DwParams q, cudaStream_t st) {
+    using Cf = DwCfg<CHX, CHY>;
+    if (!encoder()) return cudaErrorNotSupported;
+    // segments of equal width, a multiple of the 16-pixel K-step
+    q.segs = (q.W + kDwSeg - 1) / kDwSeg;
+    q.seg = ((q.W + q.segs - 1) / q.segs + 15) / 16 * 16;
+    q.segs = (q.W + q.seg - 1) / q.seg;
+    q.xpx = q.seg + 16;
+    CUtensorMap ymap, xmap;
+    if (planes_map(&ymap, dy, ldy, 0, q.cout, B, H, q.W, q.seg, CHY, Cf::R) != CUDA_SUCCESS ||
+        planes_map(&xmap, x, ldx, xoff, q.cin, B, H, q.W, q.xpx, CHX, Cf::R + 2) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    q.rowblocks = (H + Cf::R - 1) / Cf::R;
+    q.units = q.segs * q.rowblocks * B;
+    q.groups = (q.cin + 8 * CHX - 1) / (8 * CHX);
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    q.splits = sms / q.groups > 1 ? sms / q.groups : 1;
+    if (q.splits > q.units) q.splits = q.units;
+    if (q.splits <= 0) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(k_conv_dw<CHX, CHY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cf::SMEM);
+    if (e != cudaSuccess) return e;
+    k_conv_dw<CHX, CHY><<<q.groups * q.splits, kDwThreads, Cf::SMEM, st>>>(ymap, xmap, q);
+    return cudaGetLastError();
+}
+
 }  // namespace c3
 }  // namespace gpsb
 
@@ -679,6 +951,34 @@ int gpsb_dn_conv3(const void* x, int ldx, int xoff, int cin, int B, int H, int W
         case 128: return (int)(narrow ? launch<128, 2>(xb, ldx, xoff, cin, prm, st) : launch<128, 4>(xb, ldx, xoff, cin, prm, st));
         default: return (int)launch<192, 2>(xb, ldx, xoff, cin, prm, st);
     }
+}
+
+// Weight gradient dw[co][k] += sum_p dy[p][co] * xcol[p][k] (fp32, added to dw); dy (channels [0, cout)
+// of ldy) and x (channels [xoff, xoff + cin) of ldx) chunk-planar, 16-byte aligned; cout <= 128.
+int gpsb_dn_conv_dw(const void* dy, int ldy, const void* x, int ldx, int xoff, int cin, int B, int H, int W, int cout,
+                    int kp, float* dw, void* stream, uint32_t* err) {
+    if (cin % 8 || ldx % 8 || xoff % 8 || ldy % 8 || kp < 9 * cin || cout < 1 || cout > 128) return (int)cudaErrorInvalidValue;
+    if (cin < 1 || B < 1 || H < 1 || W < 1) return (int)cudaSuccess;
+    if (!dy || !x || !dw || cout > ldy || xoff < 0 || xoff + cin > ldx ||
+        ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 15u))
+        return (int)cudaErrorInvalidValue;
+    DwParams q{};
+    q.dw = dw;
+    q.cout = cout;
+    q.kp = kp;
+    q.cin = cin;
+    q.W = W;
+    q.err = err;
+    cudaStream_t st = (cudaStream_t)stream;
+    const bf16 *yb = (const bf16*)dy, *xb = (const bf16*)x;
+    if (cin <= 8) {
+        if (cout <= 32) return (int)launch_dw<1, 4>(yb, ldy, xb, ldx, xoff, B, H, q, st);
+        if (cout <= 64) return (int)launch_dw<1, 8>(yb, ldy, xb, ldx, xoff, B, H, q, st);
+        return (int)launch_dw<1, 16>(yb, ldy, xb, ldx, xoff, B, H, q, st);
+    }
+    if (cout <= 32) return (int)launch_dw<4, 4>(yb, ldy, xb, ldx, xoff, B, H, q, st);
+    if (cout <= 64) return (int)launch_dw<4, 8>(yb, ldy, xb, ldx, xoff, B, H, q, st);
+    return (int)launch_dw<4, 16>(yb, ldy, xb, ldx, xoff, B, H, q, st);
 }
 
 }  // extern "C"

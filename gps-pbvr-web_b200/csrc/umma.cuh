@@ -2,11 +2,11 @@
 // the denoiser's convolutions. One CTA of 128 threads computes a 128 x BN tile of
 //     C[m][n] = sum_k A[m][k] * B[n][k]        (A, B bf16, accumulation in fp32 in tensor memory)
 // over the K range [k_begin, k_end), in steps of 64. Operand tiles are staged in shared memory by
-// all threads through problem-specific loaders (implicit im2col, transposing gathers), in the
+// all threads through a problem-specific loader (implicit im2col), in the
 // canonical K-major layout without swizzle: core matrices of 8 rows x 16 bytes, row group rg and
 // 8-element K chunk kc at byte (rg * 8 + kc) * 128, so the K-adjacent core matrices of one MMA
 // are 128 bytes apart (leading byte offset) and the next 8 rows 1024 bytes (stride byte offset).
-// Two stages: while the tensor core multiplies one stage, the threads fill the other. Thread 0
+// While the tensor core multiplies one stage, copies fill the others. Thread 0
 // issues the MMAs (M = 128, N = BN, K = 16 each) and commits them to an mbarrier per stage; the
 // accumulator (128 lanes x BN fp32 columns of tensor memory) is read back by the four warps with
 // tcgen05.ld (warp w owns lanes 32w..32w+31 = tile rows) and handed to the problem's epilogue.
@@ -116,95 +116,6 @@ template <int BN>
 __host__ __device__ constexpr uint32_t tmem_cols() {
     return BN <= 32 ? 32u : BN <= 64 ? 64u : BN <= 128 ? 128u : 256u;
 }
-template <int BN>
-__host__ __device__ constexpr size_t smem_bytes() {
-    return 2 * ((size_t)kBM * kBK * 2 + (size_t)BN * kBK * 2) + 128;
-}
-
-// The GEMM mainloop. P provides:
-//   __device__ void load_a(uint8_t* tile, int m0, int k0) const   // 128 x 64 bf16 K-major tile
-//   __device__ void load_b(uint8_t* tile, int n0, int k0) const   // BN x 64
-//   __device__ void epilogue(int m0, int n0, int row, int col0, const float* v16) const
-//   int k_begin, k_end (multiples of 64), m0/n0 from the grid via tile(), err (uint32_t*)
-template <int BN, class P>
-__device__ __forceinline__ void gemm_tile(const P& pb, int m0, int n0, int k_begin, int k_end) {
-    static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "N of one MMA");
-    extern __shared__ __align__(128) uint8_t s_raw[];
-    __shared__ __align__(8) uint64_t s_bar[2];
-    __shared__ uint32_t s_tmem;
-    __shared__ int s_fail;
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 127) & ~(uintptr_t)127);
-    constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = BN * kBK * 2;
-    auto sa = [&](int b) { return base + b * kABytes; };
-    auto sb = [&](int b) { return base + 2 * kABytes + b * kBBytes; };
-    const int tid = threadIdx.x, warp = tid >> 5;
-    constexpr uint32_t kCols = tmem_cols<BN>();
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s_tmem)),
-                     "r"(kCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        mbar_init(&s_bar[0]);
-        mbar_init(&s_bar[1]);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_fail = 0;
-    }
-    const int steps = (k_end - k_begin) / kBK;
-    if (steps > 0) {
-        pb.load_a(sa(0), m0, k_begin);
-        pb.load_b(sb(0), n0, k_begin);
-    }
-    fence_async_smem();
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const uint32_t tmem = s_tmem;
-    constexpr uint32_t idesc = idesc_bf16(BN);
-    for (int s = 0; s < steps; ++s) {
-        const int buf = s & 1;
-        if (tid == 0) {
-            const uint32_t a0 = saddr(sa(buf)), b0 = saddr(sb(buf));
-#pragma unroll
-            for (int j = 0; j < kBK / 16; ++j)  // K = 16 = two core matrices = 256 bytes per MMA
-                mma_bf16(tmem, smem_desc(a0 + j * 256), smem_desc(b0 + j * 256), idesc, s > 0 || j > 0);
-            mma_commit(&s_bar[buf]);
-        }
-        if (s + 1 < steps) {
-            if (s >= 1 && !mbar_wait(&s_bar[buf ^ 1], ((s - 1) >> 1) & 1)) s_fail = 1;
-            pb.load_a(sa(buf ^ 1), m0, k_begin + (s + 1) * kBK);
-            pb.load_b(sb(buf ^ 1), n0, k_begin + (s + 1) * kBK);
-            fence_async_smem();
-        }
-        fence_before();
-        __syncthreads();
-        fence_after();
-        if (s_fail) break;
-    }
-    bool ok = !s_fail;
-    if (steps > 0 && ok) ok = mbar_wait(&s_bar[(steps - 1) & 1], ((steps - 1) >> 1) & 1);
-    if (!ok) {
-        if (tid == 0) atomicOr(pb.err, GEMM_ERR_TIMEOUT);
-        // let every MMA this CTA issued finish before its tensor memory is freed
-        if (steps > 0) mbar_wait(&s_bar[(steps - 1) & 1], ((steps - 1) >> 1) & 1);
-    }
-    fence_after();
-    if (ok && steps > 0) {
-        const int row = warp * 32 + (tid & 31);
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 16) {
-            float v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-            pb.epilogue(m0, n0, row, c, v);
-        }
-    }
-    fence_before();
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
-}
-
 // Issue one asynchronous 16-byte global -> shared copy; bytes < 16 zero-fills the rest (0: all zero).
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr(dst)), "l"(src), "r"(bytes) : "memory");
@@ -221,7 +132,8 @@ __host__ __device__ constexpr size_t smem_bytes_async() {
 // The mainloop with S stages filled by asynchronous copies: P provides
 //   __device__ void prepare(int m0, int n0)                   // per-tile loader state (registers)
 //   __device__ void issue(uint8_t* a_tile, uint8_t* b_tile, int k0)   // cp.async of one K step
-//   __device__ void epilogue(...), err    (as gemm_tile)
+//   __device__ void epilogue(int m0, int n0, int row, int col0, const float* v16) const
+//   uint32_t* err
 // Stage s is copied S-1 steps ahead; a stage is refilled only after the MMAs that read it have
 // completed (their mbarrier), and the tensor core reads a stage only after every thread's copies
 // into it have landed (cp.async.wait_group + proxy fence + barrier).
