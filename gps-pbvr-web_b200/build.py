@@ -20,7 +20,7 @@ NVCC = os.path.join(CUDA, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_FLAGS = ARCH + ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off",
                    "-I" + CSRC, "-I" + os.path.join(ROOT, "include")]
-CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fno-fast-math", "-I" + os.path.join(CUDA, "include"),
+CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-pthread", "-ffp-contract=off", "-fno-fast-math", "-I" + os.path.join(CUDA, "include"),
              "-I" + CSRC, "-I" + os.path.join(ROOT, "include")]
 # extra nvcc flags for tuning builds (e.g. GPSB_NVCC_EXTRA="-DGPSB_SORT_LOOKAHEAD=16"; rebuild with --force)
 CU_FLAGS += os.environ.get("GPSB_NVCC_EXTRA", "").split()
@@ -59,7 +59,7 @@ def build(force=False, verbose=False):
             else:
                 _run(["g++"] + CXX_FLAGS + ["-c", path, "-o", obj], verbose)
     if force or _newer(LIB, objs):
-        _run([NVCC] + ARCH + ["-shared", "-o", LIB + ".tmp"] + objs + ["-lcudart"], verbose)
+        _run([NVCC] + ARCH + ["-shared", "-o", LIB + ".tmp"] + objs + ["-lcudart", "-Xcompiler", "-pthread"], verbose)
         os.replace(LIB + ".tmp", LIB)
     cli_src = os.path.join(CSRC, "gpsb_verify.cpp")
     if os.path.exists(cli_src) and (force or _newer(CLI, [cli_src, LIB] + hdrs)):
