@@ -79,16 +79,25 @@ struct EnsTotal {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr int kPartThreads = 256;
-constexpr int kPartItems = 8;
-constexpr int kPartTile = kPartThreads * kPartItems;
+constexpr uint32_t kScanSmallTiles = 2 * 148;  // below this many tiles a batch is scanned with one splat a thread
+
+// Scratch of a batch's count scan and particle kernels, cleared by one memset per batch: [64 bytes of counters:
+// scan tiles, particle units][EnsTotal of each ensemble][lookback words].
+struct ScanScratch {
+    void* mem;
+    uint32_t* counters() const { return (uint32_t*)mem; }
+    EnsTotal* totals() const { return (EnsTotal*)((char*)mem + 64); }
+    uint64_t* lookback(uint32_t E) const { return (uint64_t*)(totals() + E); }
+};
+inline size_t scan_scratch_bytes(uint32_t E, uint64_t lookback_words) {
+    return 64 + (size_t)E * sizeof(EnsTotal) + (size_t)lookback_words * 8;
+}
 
 // ------------------------------------------------------------------ launchers (kernels.cu)
 void launch_geometry(const FrameConst& fc, const float4* splats, const float* sh, const float* lut, float4* rec,
                      uint2* cdesc, float4* colour, cudaStream_t st);
-void launch_count_scan(const FrameConst& fc, const uint2* cdesc, uint32_t first_seed, uint32_t E, uint64_t* lookback,
-                       uint32_t* tile_counter, uint2* clist, EnsTotal* etot, unsigned long long* stats,
-                       uint32_t* err, cudaStream_t st);
+void launch_count_scan(const FrameConst& fc, const uint2* cdesc, uint32_t first_seed, uint32_t E, const ScanScratch& sc,
+                       uint2* clist, unsigned long long* stats, uint32_t* err, cudaStream_t st);
 void launch_fast_bounds(uint32_t* out, cudaStream_t st);
 void launch_particles(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
                       const EnsTotal* etot, uint32_t first_seed, uint32_t E, unsigned long long* sub,

@@ -290,12 +290,16 @@ __device__ __forceinline__ uint64_t lb_pack(uint64_t status, uint64_t sum, uint3
     return status | ((sum > kLbSumSat ? kLbSumSat : sum) << 24) | (uint64_t)nz;
 }
 
-// Per ensemble e and tile t of kScanTile splats: Poisson count of every splat with the stream
+// Per ensemble e and tile t of 256 x ITEMS splats: Poisson count of every splat with the stream
 // particle_seed(i, 0, first_seed + e) (gps_splat.wgsl:539-548, 593-602, 573-574), the per-splat cap,
 // the statistics of prepare, then a block scan and a decoupled lookback over the tiles of the
 // ensemble. Splats with a non-zero count are written, in splat order, to the compact list
 // clist[e * N + j] = (splat id, exclusive particle offset). The last tile writes the ensemble
 // total; a total above 2^32 - 1 marks the ensemble skipped (gps_splat.wgsl:635-639, 648-654).
+// Bound: the draws of small means, one uniform per event (poisson): a thread draws for all its splats in
+// one loop, going on to its next splat when one is done, so a warp runs as long as its largest sum of counts
+// instead of the sum of each round's largest count (560k splats, far view, 64 ensembles: 1.06 -> 1.03 ms; mid view, 8: 0.156 -> 0.130).
+template <int ITEMS>
 __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const uint2* __restrict__ cdesc,
                                                              uint32_t first_seed, uint32_t tiles_per_e,
                                                              uint64_t* lookback, uint32_t* tile_counter,
@@ -316,35 +320,71 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
     const uint32_t seed = first_seed + e;
     const uint32_t N = f.N, cap = f.cap;
     const bool gps = f.method == 0u;
-    const uint32_t base = t * kScanTile + tid * kScanItems;
+    const uint32_t base = (t * kScanThreads + tid) * ITEMS;
 
-    uint32_t cnt[kScanItems];
+    uint32_t cnt[ITEMS];
     ull st_pts = 0, st_trunc = 0, st_drop = 0, st_vis = 0, st_cand = 0, st_under = 0;
     uint64_t tsum = 0;
     uint32_t tnz = 0;
+    // raw counts: fixed ones, and the normal approximation of large means; small means are left to the loop below
+    __shared__ float s_l[ITEMS][kScanThreads];        // exp(-lambda)
+    __shared__ uint32_t s_rs[ITEMS][kScanThreads];    // stream state, then the count
+    uint32_t todo = 0u, modes = 0u;
 #pragma unroll
-    for (int q = 0; q < kScanItems; ++q) {
-        uint32_t i = base + q;
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t i = base + q;
+        const uint2 cd = i < N ? __ldg(&cdesc[i]) : make_uint2(0u, CD_NONE);
+        const uint32_t mode = cd.y & 3u;
         uint32_t n = 0;
-        if (i < N) {
-            uint2 cd = __ldg(&cdesc[i]);
-            uint32_t mode = cd.y & 3u;
-            if (mode == CD_FIXED) {
-                n = cd.x;
-                st_cand += n;
-                st_vis += 1;
-            } else if (mode != CD_NONE) {
-                uint32_t rs = gx::particle_seed(i, 0u, seed);
-                n = poisson(__uint_as_float(cd.x), &rs);
-                if (gps) st_pts += n; else st_cand += n;
-                st_vis += 1;
-                if (mode == CD_POISSON_CAP && n > cap) {
-                    st_trunc += 1;
-                    st_drop += n - cap;
-                    n = cap;
-                }
+        if (mode == CD_FIXED) {
+            n = cd.x;
+        } else if (mode != CD_NONE) {
+            uint32_t rs = gx::particle_seed(i, 0u, seed);
+            const float lambda = __uint_as_float(cd.x);
+            if (lambda > F_(0.0) && lambda < F_(30.0)) {
+                s_l[q][tid] = gx::exp(-lambda);
+                n = rs;
+                todo |= 1u << q;
+            } else {
+                n = poisson(lambda, &rs);
             }
-            if (cd.y & CD_UNDERCOVERED) st_under += 1;
+        }
+        s_rs[q][tid] = n;
+        modes |= mode << (2 * q);
+        if (cd.y & CD_UNDERCOVERED) st_under += 1;
+    }
+    // gps_splat.wgsl:142-150 (poisson): uniforms until their product is at most exp(-lambda)
+    {
+        int q = todo ? __ffs(todo) - 1 : 0;
+        float l = todo ? s_l[q][tid] : F_(0.0), p = F_(1.0);
+        uint32_t rs = s_rs[q][tid], k = 0u;
+        while (todo) {
+            p = p * gx::next_u(&rs);
+            if (p <= l) {
+                s_rs[q][tid] = k;
+                todo &= todo - 1u;
+                q = todo ? __ffs(todo) - 1 : q;
+                l = s_l[q][tid];
+                rs = s_rs[q][tid];
+                p = F_(1.0);
+                k = 0u;
+            } else {
+                k += 1u;
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < ITEMS; ++q) {
+        const uint32_t mode = (modes >> (2 * q)) & 3u;
+        uint32_t n = s_rs[q][tid];
+        if (mode != CD_NONE) {
+            st_vis += 1;
+            if (gps && mode != CD_FIXED) st_pts += n; else st_cand += n;
+            if (mode == CD_POISSON_CAP && n > cap) {
+                st_trunc += 1;
+                st_drop += n - cap;
+                n = cap;
+            }
         }
         cnt[q] = n;
         tsum += n;
@@ -433,7 +473,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
     uint32_t j = s_excl_nz + wpre_nz + (inz - tnz);
     uint2* out = clist + (size_t)e * N;
 #pragma unroll
-    for (int q = 0; q < kScanItems; ++q) {
+    for (int q = 0; q < ITEMS; ++q) {
         if (cnt[q]) {
             out[j] = make_uint2(base + q, (uint32_t)off);
             off += cnt[q];
@@ -449,6 +489,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
         etot[e].particles = total;
         etot[e].nonzero = s_excl_nz + agg_nz;
         atomicAdd(&stats[ST_ENTRIES], (ull)(s_excl_nz + agg_nz));
+        atomicAdd(&stats[ST_ENSEMBLES], 1ull);
         if (total > 0xFFFFFFFFull) {
             atomicOr(&etot[e].flags, 1u);
             atomicAdd(&stats[ST_SKIPPED], 1ull);
@@ -458,16 +499,21 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
     }
 }
 
-void launch_count_scan(const FrameConst& fc, const uint2* cdesc, uint32_t first_seed, uint32_t E, uint64_t* lookback,
-                       uint32_t* tile_counter, uint2* clist, EnsTotal* etot, unsigned long long* stats, uint32_t* err,
-                       cudaStream_t st) {
-    uint32_t tiles = (fc.N + kScanTile - 1) / kScanTile;
-    cudaMemsetAsync(lookback, 0, (size_t)E * tiles * sizeof(uint64_t), st);
-    cudaMemsetAsync(tile_counter, 0, sizeof(uint32_t), st);
-    cudaMemsetAsync(etot, 0, (size_t)E * sizeof(EnsTotal), st);
+void launch_count_scan(const FrameConst& fc, const uint2* cdesc, uint32_t first_seed, uint32_t E, const ScanScratch& sc,
+                       uint2* clist, unsigned long long* stats, uint32_t* err, cudaStream_t st) {
+    const uint32_t large = (fc.N + kScanTile - 1) / kScanTile;
+    // few tiles of eight splats a thread leave most SMs idle: one splat a thread (10k splats, one ensemble,
+    // 5 blocks: 22 us; 40 blocks: 9 us)
+    const bool small = (uint64_t)large * E < kScanSmallTiles;
+    const uint32_t tiles = small ? (fc.N + kScanThreads - 1) / kScanThreads : large;
+    cudaMemsetAsync(sc.mem, 0, scan_scratch_bytes(E, (uint64_t)E * tiles), st);
     if (fc.N == 0 || E == 0) return;
-    k_count_scan<<<tiles * E, kScanThreads, 0, st>>>(fc, cdesc, first_seed, tiles, lookback, tile_counter, clist, etot,
-                                                      stats, err);
+    if (small)
+        k_count_scan<1><<<tiles * E, kScanThreads, 0, st>>>(fc, cdesc, first_seed, tiles, sc.lookback(E), sc.counters(), clist,
+                                                            sc.totals(), stats, err);
+    else
+        k_count_scan<kScanItems><<<tiles * E, kScanThreads, 0, st>>>(fc, cdesc, first_seed, tiles, sc.lookback(E), sc.counters(),
+                                                                     clist, sc.totals(), stats, err);
 }
 
 // ============================================================================ particles
@@ -868,7 +914,8 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     __shared__ uint32_t s_steps;
     const int tid = threadIdx.x, lane = tid & 31;
     // particles per unit: max_steps * 32, fewer when warps would get less than four units each
-    // (560k splats, far view, 4 ensembles: 0.775 ms; with one unit each 0.847)
+    // (560k splats, far view, 4 ensembles: 0.775 ms; with one unit each 0.847), but at least two steps, as every
+    // block that has a unit stages its tables (10k splats: 10.2 us; one step 12.9, four 11.6)
     if (tid < 32) {
         uint64_t total = 0;
         for (uint32_t e = lane; e < E; e += 32) {
@@ -877,7 +924,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
         }
         for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
         const uint64_t want = total / ((uint64_t)gridDim.x * kPT * 4u);
-        const uint32_t steps = want >= max_steps ? max_steps : want < 1u ? 1u : (uint32_t)want;
+        const uint32_t steps = want >= max_steps ? max_steps : want < 2u ? 2u : (uint32_t)want;
         uint64_t acc = 0;
         for (uint32_t e0 = 0; e0 < E; e0 += 32) {
             const uint32_t e = e0 + lane;
@@ -915,12 +962,15 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     const uint32_t flags = FL >= 0 ? (uint32_t)FL : f.flags;
     const bool vc = FL >= 0 ? false : f.method == 3u;
     uint32_t points = 0, writes = 0, exact_runs = 0, mismatch = 0;
-    uint32_t next = 0u;
-    if (lane == 0) next = atomicAdd(unit_counter, 1u);
+    // the first unit is the warp's own number, the next ones come from the counter (a call with no more units
+    // than warps asks it nothing: thousands of warps queue up on one word)
+    const uint32_t warps = gridDim.x * (kPT / 32);
+    uint32_t next = blockIdx.x * (kPT / 32) + (tid >> 5);
     for (;;) {
         const uint32_t un = __shfl_sync(0xffffffffu, next, 0);
         if ((uint64_t)un >= total_units) break;
-        if (lane == 0) next = atomicAdd(unit_counter, 1u);  // the next unit; its latency is covered by this one
+        next = 0xFFFFFFFFu;
+        if (total_units > warps && lane == 0) next = warps + atomicAdd(unit_counter, 1u);  // its latency is covered by this unit
         // ensemble of the unit: largest e with s_ubase[e] <= un
         uint32_t e = 0, eh = E;
         while (eh - e > 1u) {
@@ -1175,7 +1225,6 @@ static void launch_particles_t(const FrameConst& fc, const float4* rec, const fl
 void launch_particles(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
                       const EnsTotal* etot, uint32_t first_seed, uint32_t E, unsigned long long* sub,
                       uint32_t* unit_counter, unsigned long long* stats, int grid, int items, cudaStream_t st) {
-    cudaMemsetAsync(unit_counter, 0, sizeof(uint32_t), st);
     if (fc.N == 0 || E == 0) return;
     // the fast GPS decisions cover single subpixels and the radius table; footprint blocks and the
     // iterated radius run the exact path

@@ -112,7 +112,7 @@ struct gpsb_renderer {
     // per frame
     DevBuf accum, stats, err;
     // per ensemble batch
-    DevBuf sub, clist, lookback, etot, counters;
+    DevBuf sub, clist, scan;  // scan: ScanScratch
     uint32_t batch_cap = 0;
     uint32_t last_batch = 0;     // ensembles in the last batch rendered
     uint32_t last_seed = 0;      // seed of its first ensemble
@@ -293,9 +293,8 @@ static gpsb_status ensure_batch(gpsb_renderer* r, uint32_t E) {
     uint32_t tiles = (r->n + kScanTile - 1) / kScanTile;
     CK(r, r->sub.ensure((size_t)E * PS * 8), "subpixel buffers");
     CK(r, r->clist.ensure((size_t)E * std::max(r->n, 1u) * 8), "particle list");
-    CK(r, r->lookback.ensure((size_t)E * std::max(tiles, 1u) * 8), "scan lookback");
-    CK(r, r->etot.ensure((size_t)E * sizeof(EnsTotal)), "ensemble totals");
-    CK(r, r->counters.ensure(64), "counters");
+    // a small batch's lookback has up to kScanItems words per large tile
+    CK(r, r->scan.ensure(scan_scratch_bytes(E, (uint64_t)E * tiles + (uint64_t)kScanSmallTiles * kScanItems)), "scan scratch");
     r->batch_cap = E;
     return GPSB_OK;
 }
@@ -331,24 +330,24 @@ static gpsb_status render_batch(gpsb_renderer* r, const FrameConst& f, bool part
     ull_t* stats = r->stats.as<ull_t>();
     {
         StageScope sc(r, GPSB_STAGE_CLEAR);
-        sc.kernels(1);
+        sc.kernels(particles ? 0 : 1);
         CK(r, cudaMemsetAsync(r->sub.p, 0xFF, (size_t)E * PS * 8, r->stream), "clear subpixels");
-        launch_add_stat(stats, ST_ENSEMBLES, E, r->stream);
+        if (!particles) launch_add_stat(stats, ST_ENSEMBLES, E, r->stream);  // the count scan counts its own
     }
-    uint32_t* cnt = r->counters.as<uint32_t>();
+    const ScanScratch scan{r->scan.p};
     if (particles) {
         {
             StageScope sc(r, GPSB_STAGE_COUNT_SCAN);
             sc.kernels(1);
-            launch_count_scan(f, r->cdesc.as<uint2>(), first_seed, E, r->lookback.as<uint64_t>(), cnt,
-                              r->clist.as<uint2>(), r->etot.as<EnsTotal>(), stats, r->err.as<uint32_t>(), r->stream);
+            launch_count_scan(f, r->cdesc.as<uint2>(), first_seed, E, scan, r->clist.as<uint2>(), stats,
+                              r->err.as<uint32_t>(), r->stream);
             CK(r, cudaGetLastError(), "count/scan kernel");
         }
         {
             StageScope sc(r, GPSB_STAGE_PARTICLES);
             sc.kernels(1);
-            launch_particles(f, r->rec.as<float4>(), r->lut.as<float>(), r->clist.as<uint2>(), r->etot.as<EnsTotal>(),
-                             first_seed, E, r->sub.as<ull_t>(), cnt + 1, stats,
+            launch_particles(f, r->rec.as<float4>(), r->lut.as<float>(), r->clist.as<uint2>(), scan.totals(),
+                             first_seed, E, r->sub.as<ull_t>(), scan.counters() + 1, stats,
                              r->sm_count * (int)r->particle_blocks_per_sm, (int)r->particle_items * 8, r->stream);
             CK(r, cudaGetLastError(), "particle kernel");
         }
@@ -356,18 +355,18 @@ static gpsb_status render_batch(gpsb_renderer* r, const FrameConst& f, bool part
         StageScope sc(r, GPSB_STAGE_PRIMITIVE);
         sc.kernels(1);
         launch_primitive(f, r->rec.as<float4>(), r->cdesc.as<uint2>(), r->lut.as<float>(), first_seed, E,
-                         r->sub.as<ull_t>(), r->etot.as<EnsTotal>(), stats, r->stream);
+                         r->sub.as<ull_t>(), scan.totals(), stats, r->stream);
         CK(r, cudaGetLastError(), "primitive kernel");
     }
     {
         StageScope sc(r, GPSB_STAGE_RESOLVE);
         sc.kernels(1);
-        launch_resolve(f, r->sub.as<ull_t>(), r->etot.as<EnsTotal>(), r->colour.as<float4>(), E, accum, stats,
+        launch_resolve(f, r->sub.as<ull_t>(), scan.totals(), r->colour.as<float4>(), E, accum, stats,
                        r->stream);
         CK(r, cudaGetLastError(), "resolve kernel");
         if (r->feat) {
             sc.kernels(1);
-            launch_features(f, r->sub.as<ull_t>(), r->etot.as<EnsTotal>(), r->colour.as<float4>(), E, r->feat,
+            launch_features(f, r->sub.as<ull_t>(), scan.totals(), r->colour.as<float4>(), E, r->feat,
                             r->stream);
             CK(r, cudaGetLastError(), "feature kernel");
         }
@@ -568,7 +567,7 @@ void gpsb_destroy(gpsb_renderer* r) {
     cudaSetDevice(r->device);
     if (r->stream) cudaStreamSynchronize(r->stream);
     DevBuf* bufs[] = {&r->splats, &r->sh, &r->lut, &r->rec, &r->cdesc, &r->colour, &r->accum, &r->stats, &r->err,
-                      &r->sub, &r->clist, &r->lookback, &r->etot, &r->counters, &r->rgba8};
+                      &r->sub, &r->clist, &r->scan, &r->rgba8};
     for (DevBuf* b : bufs) b->release();
     for (DevBuf& b : r->spare) b.release();
     r->upload.release();
@@ -840,7 +839,7 @@ gpsb_status gpsb_render_trajectory_graph(gpsb_renderer* r, const gpsb_camera* ca
     // the device buffers baked into the graph: a reallocation (bigger batch, new scene or frame
     // size) must re-capture, never replay stale pointers
     const void* bufs[] = {r->splats.p, r->sh.p, r->lut.p, r->rec.p, r->cdesc.p, r->colour.p, r->stats.p, r->err.p,
-                          r->sub.p, r->clist.p, r->lookback.p, r->etot.p, r->counters.p};
+                          r->sub.p, r->clist.p, r->scan.p};
     put(bufs, sizeof bufs);
     if (!r->traj_exec || key != r->traj_key) {
         if (r->traj_exec) {
@@ -851,10 +850,9 @@ gpsb_status gpsb_render_trajectory_graph(gpsb_renderer* r, const gpsb_camera* ca
         uint32_t B = pick_batch(r, E);
         gpsb_status s = ensure_batch(r, B);
         if (s != GPSB_OK) return s;
-        CK(r, r->counters.ensure(64), "counters");
         // the buffers may have just been (re)allocated: key them as they are now
         const void* now[] = {r->splats.p, r->sh.p, r->lut.p, r->rec.p, r->cdesc.p, r->colour.p, r->stats.p, r->err.p,
-                             r->sub.p, r->clist.p, r->lookback.p, r->etot.p, r->counters.p};
+                             r->sub.p, r->clist.p, r->scan.p};
         key.resize(key.size() - sizeof now);
         put(now, sizeof now);
         cudaGraph_t g = nullptr;
@@ -1031,7 +1029,7 @@ gpsb_status gpsb_debug_read_counts(gpsb_renderer* r, uint32_t slot, uint32_t* co
     if (!r->last_particle || slot >= r->last_batch) return fail(r, GPSB_ERR_STATE, "slot not in the last particle-path batch");
     cudaSetDevice(r->device);
     EnsTotal t;
-    CK(r, cudaMemcpyAsync(&t, r->etot.as<EnsTotal>() + slot, sizeof t, cudaMemcpyDeviceToHost, r->stream), "read totals");
+    CK(r, cudaMemcpyAsync(&t, ScanScratch{r->scan.p}.totals() + slot, sizeof t, cudaMemcpyDeviceToHost, r->stream), "read totals");
     CK(r, cudaStreamSynchronize(r->stream), "synchronise");
     std::vector<uint2> L(t.nonzero);
     if (t.nonzero)
@@ -1051,7 +1049,7 @@ gpsb_status gpsb_debug_particle_seeds(gpsb_renderer* r, uint32_t slot, uint64_t 
     if (!r->last_particle || slot >= r->last_batch) return fail(r, GPSB_ERR_STATE, "slot not in the last particle-path batch");
     cudaSetDevice(r->device);
     EnsTotal t;
-    CK(r, cudaMemcpyAsync(&t, r->etot.as<EnsTotal>() + slot, sizeof t, cudaMemcpyDeviceToHost, r->stream), "read totals");
+    CK(r, cudaMemcpyAsync(&t, ScanScratch{r->scan.p}.totals() + slot, sizeof t, cudaMemcpyDeviceToHost, r->stream), "read totals");
     CK(r, cudaStreamSynchronize(r->stream), "synchronise");
     if (t.flags != 0u) return fail(r, GPSB_ERR_STATE, "the ensemble was skipped");
     if (first_particle > t.particles || n > t.particles - first_particle)
@@ -1153,8 +1151,7 @@ gpsb_status gpsb_set_tuning(gpsb_renderer* r, const gpsb_tuning* t) {
         r->batch_cap = 0;
         r->sub.release();
         r->clist.release();
-        r->lookback.release();
-        r->etot.release();
+        r->scan.release();
     }
     return GPSB_OK;
 }

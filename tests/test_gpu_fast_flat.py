@@ -6,7 +6,7 @@ of thousands; every subpixel side; sparse and dense ScreenOccupancy."""
 import numpy as np
 import pytest
 
-from _parity import PKG
+from _parity import PKG, assert_bit_exact
 
 pytestmark = pytest.mark.gpu
 M = PKG.Method
@@ -73,3 +73,16 @@ def test_most_particles_are_decided():
         _, st, (undecided, mismatch), _ = render(r, cam, PKG.RenderParams(spp_side=2, method=method), 2, 2)
         assert mismatch == 0 and st.particles > 100_000 and undecided < 0.02 * st.particles, (method, undecided, st.particles)
     r.close()
+
+
+@pytest.mark.parametrize("n,ens", [(1, 1), (255, 1), (256, 3), (257, 2), (2047, 1), (2049, 40), (75_000, 7), (75_000, 8)])
+def test_count_scan_shapes(n, ens):
+    """Both tile sizes of the count scan (one splat a thread below 296 tiles of 2048 splats, eight from there
+    on): the counts of every splat and ensemble, the statistics and the image equal the CPU mirror's, with
+    fixed counts, small and large means and capped splats among them."""
+    s = scene(n, n, -6.0, lambda r, k: r.uniform(0.0, 1.0, k))
+    s[: 1 + n // 5000, 4:7] = -2.0  # large means
+    cam = PKG.OrbitCamera(distance=5.0).to_camera(160, 90)
+    for method in (M.Gps, M.Extinction, M.ScreenOccupancy):
+        assert_bit_exact(s, None, 0, 160, 90, 1, cam, PKG.RenderParams(spp_side=1, method=method, max_points_per_splat=500),
+                         first_seed=5, count=ens)
