@@ -5,7 +5,7 @@
 //   radix_sort_pairs  stable LSD onesweep sort (replaces gps_sort.wgsl): one histogram pass for
 //                   all digits, then one kernel per digit that ranks keys within each warp by
 //                   peer groups (each lane ORs its bit into its digit's word of a per-warp row in
-//                   shared memory and reads the word back), resolves tile offsets by a decoupled
+//                   shared memory and reads the word back, or ballots), resolves tile offsets by a decoupled
 //                   lookback per digit and scatters. Digit width 4, 6 or 8 bits.
 //   binning         (bin, splat id) entries in depth order, stably sorted by bin, give every screen bin
 //                   its splats in depth order.
@@ -45,39 +45,35 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // ============================================================================ radix sort
 constexpr int kRsThreads = 256;
 constexpr int kRsWarps = kRsThreads / 32;
-// Keys per thread and resident blocks per SM of a onesweep pass, per digit width: 8-bit digits
-// take 25 keys per thread (6400 per tile, 62.5 KB of staging, 3 blocks per SM), whose longer
-// digit runs write out in fuller sectors (2^26 pairs: 15 keys 2.24 TB/s, 21 2.31, 23 2.41, 25
-// 2.47); 4- and 6-bit digits 15 (3840, 37.5 KB, 4 blocks per SM), where larger tiles gained nothing.
+// Keys per thread of a onesweep pass, per digit width: 8-bit digits take 27 (6912 keys per tile, 54 KB of
+// staging, 3 blocks per SM), whose longer digit runs write out in fuller sectors (2^24 pairs, three passes: 17
+// keys 359 us, 23 355, 25 347, 27 343); 4- and 6-bit digits 15 (3840, 4 blocks per SM), where larger
+// tiles gained nothing. Sorts of up to kRsSmallMax pairs take 8 (2048): large tiles would leave most SMs
+// idle and make the few blocks' chains long (large / small tiles: 50k pairs 51 / 41 us, 400k 57 / 50,
+// 560k 55 / 53, 800k 55 / 58, 2M 73 / 96).
 #ifndef GPSB_SORT_IPT8
-#define GPSB_SORT_IPT8 25
+#define GPSB_SORT_IPT8 27
 #endif
 #ifndef GPSB_SORT_IPT
 #define GPSB_SORT_IPT 15
 #endif
+constexpr int kRsIptSmall = 8;
+constexpr uint32_t kRsSmallMax = 600u * 1024u;  // pairs; also bounds the tiles of the no-allocation scratch
 template <int BITS>
+constexpr int kRsIptLarge = BITS >= 8 ? GPSB_SORT_IPT8 : GPSB_SORT_IPT;
+template <int BITS, int IPT>
 struct RsShape {
-    static constexpr int ipt = BITS >= 8 ? GPSB_SORT_IPT8 : GPSB_SORT_IPT;
-    static constexpr int tile = kRsThreads * ipt;
-    static constexpr size_t stage = (size_t)tile * 10;  // dynamic shared memory of one block
-    static constexpr int min_blocks = stage + 8 * 1024 > 56 * 1024 ? 3 : 4;
-    static_assert(tile % 4 == 0 && tile <= 65536, "tile staging layout");
+    static constexpr int tile = kRsThreads * IPT;
+    static constexpr size_t rows = (size_t)kRsWarps * (1 << BITS) * 8;
+    static constexpr size_t stage = (size_t)tile * 8 > rows ? (size_t)tile * 8 : rows;  // dynamic shared memory of one block
+    static constexpr int min_blocks = IPT >= 20 ? 3 : 4;
 };
 constexpr int kMaxPasses = 8;
 #ifndef GPSB_SORT_LOOKAHEAD
-#define GPSB_SORT_LOOKAHEAD 8
+#define GPSB_SORT_LOOKAHEAD 4
 #endif
 constexpr int kRsLook = GPSB_SORT_LOOKAHEAD;  // predecessor tiles read per lookback round trip
-#ifndef GPSB_SORT_BALLOT_PEERS
-// 0 match.any, 1 ballots, 2 alternating per key, 3 shared-memory OR (2^26 pairs, 8-bit digits:
-// ballots 1.421 ms, shared OR 1.368, with the bulk value copy 1.330; A/B on one B200)
-#define GPSB_SORT_BALLOT_PEERS 3
-#endif
 constexpr uint32_t kStAgg = 1u << 30, kStPre = 2u << 30, kStMask = (1u << 30) - 1u;
-#ifndef GPSB_SORT_BULK_VALUES
-#define GPSB_SORT_BULK_VALUES 1  // 1: a full tile's values arrive by one cp.async.bulk (mbarrier), 0: 16-byte cp.async
-#endif
-
 template <int BITS>
 __global__ void __launch_bounds__(256) k_radix_hist(const uint32_t* __restrict__ keys, uint32_t n, int passes,
                                                     uint32_t* hist) {
@@ -85,10 +81,19 @@ __global__ void __launch_bounds__(256) k_radix_hist(const uint32_t* __restrict__
     __shared__ uint32_t s[kMaxPasses * BINS];
     for (int k = threadIdx.x; k < passes * BINS; k += blockDim.x) s[k] = 0;
     __syncthreads();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t k = __ldg(&keys[i]);
+    auto count = [&](uint32_t k) {
         for (int p = 0; p < passes; ++p) atomicAdd(&s[p * BINS + ((k >> (p * BITS)) & (BINS - 1))], 1u);
+    };
+    const uint32_t start = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    const uint32_t quads = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0 ? n / 4u : 0u;  // 16-byte loads where aligned
+    for (uint32_t i = start; i < quads; i += step) {
+        const uint4 k = __ldg(reinterpret_cast<const uint4*>(keys) + i);
+        count(k.x);
+        count(k.y);
+        count(k.z);
+        count(k.w);
     }
+    for (uint32_t i = 4u * quads + start; i < n; i += step) count(__ldg(&keys[i]));
     __syncthreads();
     for (int k = threadIdx.x; k < passes * BINS; k += blockDim.x)
         if (s[k]) atomicAdd(&hist[k], s[k]);
@@ -115,119 +120,84 @@ __global__ void k_radix_hist_scan(uint32_t* hist) {
     if (tid < BINS) h[tid] = base + incl - c;
 }
 
-template <int BITS>
-__global__ void __launch_bounds__(kRsThreads, RsShape<BITS>::min_blocks) k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                         uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                         uint32_t n, int shift, const uint32_t* __restrict__ gstart,
-                                                         uint32_t* lookback, uint32_t* tile_counter, uint32_t* err) {
+// One digit pass over a tile: rank, scan, scatter into shared memory in digit order, lookback, write-out.
+// Bound: shared-memory wavefronts (accesses by digit or by rank fall on the banks at random, 3 to 4 wavefronts
+// each), so what counts is how many of them a key takes: the warps' and the tile's digit prefixes are one word,
+// and the values follow the keys straight to their rank (their loads come back in one go, before the
+// lookback). 2^24 pairs, 24-bit keys, three passes, the histogram and the scan: 335 us; with two prefixes,
+// and with the values staged in input order by a bulk copy and fetched through each key's 16-bit
+// input index: 388 us.
+template <int BITS, int IPT>
+__global__ void __launch_bounds__(kRsThreads, RsShape<BITS, IPT>::min_blocks)
+    k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
+               uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* __restrict__ gstart, uint32_t* lookback,
+               uint32_t* tile_counter, uint32_t* err) {
     constexpr int BINS = 1 << BITS;
-    constexpr int kRsIpt = RsShape<BITS>::ipt, kRsTile = RsShape<BITS>::tile;
-    __shared__ uint32_t s_wcnt[kRsWarps][BINS];  // per-warp digit counts, then exclusive prefix over warps
-    __shared__ uint32_t s_dstart[BINS];          // tile-local exclusive prefix over digits
-    __shared__ uint32_t s_gbase[BINS];           // global position of the digit's first key of this tile, minus s_dstart
-    // dynamic shared memory (RsShape::stage bytes): keys in digit order, the tile's values in input order
-    // (16-byte aligned for cp.async), the tile-local input index of each ordered key
+    constexpr int kRsTile = RsShape<BITS, IPT>::tile;
+    __shared__ uint32_t s_wpos[kRsWarps][BINS];  // each warp's digit counts, then the rank in the tile of its first key of a digit
+    __shared__ uint32_t s_gbase[BINS];           // global position of the digit's first key of this tile, minus its rank
+    // dynamic shared memory (RsShape::stage bytes): keys, then values, in digit order. Until the ranking ends
+    // the warps' rows of peer masks lie in it.
     extern __shared__ __align__(16) uint32_t s_stage[];
     uint32_t* s_key = s_stage;
-    uint32_t* s_vin = s_stage + kRsTile;
-    uint16_t* s_src = reinterpret_cast<uint16_t*>(s_stage + 2 * kRsTile);
+    uint32_t* s_val = s_stage + kRsTile;
     __shared__ uint32_t s_wsum[kRsWarps];
     __shared__ uint32_t s_tile;
-    __shared__ __align__(8) uint64_t s_vbar;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) {
-        s_tile = atomicAdd(tile_counter, 1u);
-        if (GPSB_SORT_BULK_VALUES) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&s_vbar))
-                         : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-    }
-    for (int k = tid; k < kRsWarps * BINS; k += kRsThreads) (&s_wcnt[0][0])[k] = 0;
+    if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
+    for (int k = tid; k < kRsWarps * BINS; k += kRsThreads) s_stage[k] = (&s_wpos[0][0])[k] = 0u;
     __syncthreads();
     const uint32_t t = s_tile;
     const uint32_t tile0 = t * kRsTile;
     const uint32_t tile_n = n - tile0 < (uint32_t)kRsTile ? n - tile0 : (uint32_t)kRsTile;
-    const uint32_t base = tile0 + warp * 32 * kRsIpt;
-    // the tile's values travel to shared memory asynchronously while the keys are ranked
-    const bool vasync = (((uintptr_t)vin) & 15u) == 0;
-    const bool vbulk = GPSB_SORT_BULK_VALUES && vasync && tile_n == (uint32_t)kRsTile;
-    if (vbulk) {
-        if (tid == 0) {
-            const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_vbar);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kRsTile * 4u)
-                         : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(s_vin)),
-                         "l"(vin + tile0), "r"(kRsTile * 4u), "r"(bar)
-                         : "memory");
-        }
-    } else if (!vasync) {
-        for (uint32_t e = tid; e < tile_n; e += kRsThreads) s_vin[e] = vin[tile0 + e];
-    } else {
-        for (uint32_t c = tid; c < (uint32_t)kRsTile / 4u; c += kRsThreads) {
-            const uint32_t e = c * 4u;
-            const uint32_t bytes = e < tile_n ? min(tile_n - e, 4u) * 4u : 0u;
-            const uint32_t* src = bytes ? vin + tile0 + e : vin;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(s_vin + e)),
-                         "l"(src), "r"(bytes)
-                         : "memory");
-        }
-    }
-    uint32_t key[kRsIpt], rank[kRsIpt];
+    const bool whole = tile_n == (uint32_t)kRsTile;
+    const uint32_t base = tile0 + warp * 32 * IPT + lane;  // this lane's keys lie 32 apart from here
+    uint32_t key[IPT], rank[IPT];
     const uint32_t lt = lanemask_lt();
-    uint32_t* wc = s_wcnt[warp];
-    // peer masks through shared memory (variant 3): each warp's row of BINS words lives in the key
-    // staging area, which the ranking does not use yet (it is written after the block barrier that
-    // ends the ranking); rows start at zero and every group's lowest lane clears its digit's word
-    uint32_t* wm = s_key + warp * BINS;
-    if (GPSB_SORT_BALLOT_PEERS == 3) {
-        for (int k = lane; k < BINS; k += 32) wm[k] = 0u;
-        __syncwarp();
-    }
-    // rank every key within its warp's sub-tile in input order (stable): the lanes holding one digit
-    // find each other (peers: one ballot per digit bit, or match.any), every lane reads its digit's
-    // running count of the warp, and the lowest lane of each group adds the group's size (the
-    // groups hold distinct digits, so the warp's counter row needs no atomics)
+    uint32_t* msk = s_stage + warp * BINS;
+    uint32_t* cnts = s_wpos[warp];
+    // rank every key within its warp's sub-tile in input order (stable). The lanes that hold one digit find
+    // each other (peers) through shared memory (every lane ORs its bit into the digit's mask and reads the
+    // word back; the lowest lane clears it) or, every third key, by one ballot per digit bit, which leaves the
+    // shared-memory unit free. Then every lane reads its digit's running count of the warp, and the
+    // lowest lane of each group adds the group's size (the groups hold distinct digits: no atomics).
+    // 2^24 pairs: all OR 343 us, every third by ballots 335, every second 341, all 384.
     auto rank_key = [&](int q, uint32_t d, uint32_t live) {
+        const bool mine = (live >> lane) & 1u;
         uint32_t peers;
-        if (GPSB_SORT_BALLOT_PEERS == 3) {
-            if ((live >> lane) & 1u) atomicOr(&wm[d], 1u << lane);
-            __syncwarp();
-            peers = wm[d] & live;
-        } else if (GPSB_SORT_BALLOT_PEERS == 1 || (GPSB_SORT_BALLOT_PEERS == 2 && (q & 1))) {
+        const bool vote = q % 3 == 2;
+        if (vote) {
             peers = live;
 #pragma unroll
-            for (int b = 0; b < BITS; ++b) {
-                const bool bs = (d >> b) & 1u;
-                const uint32_t m = __ballot_sync(0xffffffffu, bs);
-                peers &= bs ? m : ~m;
+            for (int k = 0; k < BITS; ++k) {
+                const bool set = (d >> k) & 1u;
+                const uint32_t m = __ballot_sync(0xffffffffu, set);
+                peers &= set ? m : ~m;
             }
         } else {
-            peers = __match_any_sync(0xffffffffu, d) & live;
+            if (mine) atomicOr(&msk[d], 1u << lane);
+            __syncwarp();
+            peers = msk[d] & live;
         }
-        const uint32_t below = __popc(peers & lt);
-        const uint32_t old = wc[d];
+        const uint32_t below = __popc(peers & lt), old = cnts[d];
         __syncwarp();
-        if (below == 0u && ((live >> lane) & 1u)) {
-            wc[d] = old + (uint32_t)__popc(peers);
-            if (GPSB_SORT_BALLOT_PEERS == 3) wm[d] = 0u;
+        if (below == 0u && mine) {
+            if (!vote) msk[d] = 0u;
+            cnts[d] = old + (uint32_t)__popc(peers);
         }
-        __syncwarp();  // orders this key's count update before the next key's reads
+        __syncwarp();  // orders this key's update before the next key's accesses
         rank[q] = old + below;
     };
-    if (tile_n == (uint32_t)kRsTile) {
-        const uint32_t* kp = kin + base + lane;  // the keys of this lane, 32 apart
+    if (whole) {
 #pragma unroll
-        for (int q = 0; q < kRsIpt; ++q) {
-            key[q] = __ldg(kp + q * 32);
+        for (int q = 0; q < IPT; ++q) {
+            key[q] = __ldg(kin + base + q * 32);
             rank_key(q, (key[q] >> shift) & (BINS - 1), 0xffffffffu);
         }
     } else {
 #pragma unroll
-        for (int q = 0; q < kRsIpt; ++q) {
-            const uint32_t idx = base + q * 32 + lane;
+        for (int q = 0; q < IPT; ++q) {
+            const uint32_t idx = base + q * 32;
             const bool valid = idx < n;
             key[q] = valid ? __ldg(&kin[idx]) : 0u;
             rank_key(q, valid ? ((key[q] >> shift) & (BINS - 1)) : 0u, __ballot_sync(0xffffffffu, valid));
@@ -236,13 +206,13 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS>::min_blocks) k_onesw
     __syncthreads();
     // per digit: exclusive prefix over warps and the tile count; publish the tile's aggregate early
     uint32_t* lb = lookback + (size_t)t * BINS;
-    uint32_t cnt = 0;
+    uint32_t cnt = 0, pre[kRsWarps];
     if (tid < BINS) {
 #pragma unroll
         for (int w = 0; w < kRsWarps; ++w) {
-            uint32_t c = s_wcnt[w][tid];
-            s_wcnt[w][tid] = cnt;
-            cnt += c;
+            pre[w] = cnt;
+            cnt += s_wpos[w][tid];
+
         }
         st_relaxed32(&lb[tid], (t == 0 ? kStPre : kStAgg) | cnt);
     }
@@ -254,37 +224,27 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS>::min_blocks) k_onesw
     }
     if (lane == 31) s_wsum[warp] = incl;
     __syncthreads();
-    uint32_t wbase = 0;
-    for (int w = 0; w < warp; ++w) wbase += s_wsum[w];
-    if (tid < BINS) s_dstart[tid] = wbase + incl - cnt;
-    if (vbulk) {
-        if (tid == 0) {  // the bulk copy has landed (bounded wait); the barrier below shares it
-            const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_vbar);
-            uint32_t ok = 0;
-            for (uint32_t i = 0; i < (1u << 24) && !ok; ++i)
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-                    "selp.u32 %0, 1, 0, p;\n\t}"
-                    : "=r"(ok)
-                    : "r"(bar)
-                    : "memory");
-            if (!ok) atomicOr(err, ERR_SORT_LOOKBACK);
-        }
-    } else if (vasync) {
-        asm volatile("cp.async.wait_all;" ::: "memory");  // own copies done; the barrier shares them
+    uint32_t dstart = incl - cnt;
+    for (int w = 0; w < warp; ++w) dstart += s_wsum[w];
+    if (tid < BINS) {
+#pragma unroll
+        for (int w = 0; w < kRsWarps; ++w) s_wpos[w][tid] = dstart + pre[w];
     }
     __syncthreads();
-    // scatter into shared memory in digit order (stable); values follow through their input index
+    // scatter the keys into shared memory in digit order (stable), then fetch the values, which arrive during
+    // the lookback
 #pragma unroll
-    for (int q = 0; q < kRsIpt; ++q) {
-        uint32_t idx = base + q * 32 + lane;
-        if (idx < n) {
-            uint32_t d = (key[q] >> shift) & (BINS - 1);
-            uint32_t pos = s_dstart[d] + s_wcnt[warp][d] + rank[q];
-            s_key[pos] = key[q];
-            s_src[pos] = (uint16_t)(idx - tile0);
+    for (int q = 0; q < IPT; ++q) {
+        const uint32_t idx = base + q * 32;
+        if (whole || idx < n) {
+            rank[q] += cnts[(key[q] >> shift) & (BINS - 1)];
+            s_key[rank[q]] = key[q];
+            key[q] = __ldg(&vin[idx]);
         }
     }
+#pragma unroll
+    for (int q = 0; q < IPT; ++q)
+        if (whole || base + q * 32 < n) s_val[rank[q]] = key[q];
     // lookback per digit, kRsLook predecessors per round trip; an unpublished word is polled again
     if (tid < BINS) {
         uint32_t excl = 0;
@@ -316,7 +276,7 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS>::min_blocks) k_onesw
             if (failed) atomicOr(err, ERR_SORT_LOOKBACK);
             st_relaxed32(&lb[tid], kStPre | ((excl + cnt) & kStMask));
         }
-        s_gbase[tid] = gstart[tid] + excl - s_dstart[tid];
+        s_gbase[tid] = gstart[tid] + excl - dstart;
     }
     __syncthreads();
     // coalesced write-out: consecutive threads write consecutive keys of each digit run
@@ -329,12 +289,12 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS>::min_blocks) k_onesw
         bad |= !ok;
         if (ok) {
             kout[pos] = k;
-            vout[pos] = s_vin[s_src[i]];
+            vout[pos] = s_val[i];
         }
     };
-    if (tile_n == (uint32_t)kRsTile) {
+    if (whole) {
 #pragma unroll
-        for (int q = 0; q < kRsIpt; ++q) write_one((uint32_t)(q * kRsThreads + tid));
+        for (int q = 0; q < IPT; ++q) write_one((uint32_t)(q * kRsThreads + tid));
     } else {
         for (uint32_t i = tid; i < tile_n; i += kRsThreads) write_one(i);
     }
@@ -346,15 +306,31 @@ void radix_release(RadixScratch& s) {
     s = RadixScratch();
 }
 
-// One onesweep pass; the staging lives in dynamic shared memory (above 48 KB for large tiles).
+// Tiles of a sort of n pairs, and one onesweep pass over them; the staging lives in dynamic shared memory
+// (above 48 KB for large tiles).
+template <int BITS>
+static uint32_t onesweep_tiles(uint32_t n) {
+    const uint32_t tile = n <= kRsSmallMax ? RsShape<BITS, kRsIptSmall>::tile : RsShape<BITS, kRsIptLarge<BITS>>::tile;
+    return (n + tile - 1) / tile;
+}
+template <int BITS, int IPT>
+static void onesweep_launch_t(uint32_t tiles, const uint32_t* ik, const uint32_t* iv, uint32_t* ok, uint32_t* ov, uint32_t n,
+                              int shift, const uint32_t* gstart, uint32_t* lookback, uint32_t* counter, uint32_t* err,
+                              cudaStream_t st) {
+    // set on every launch: the attributes belong to the current device's context
+    constexpr size_t stage = RsShape<BITS, IPT>::stage;
+    cudaFuncSetAttribute(k_onesweep<BITS, IPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage);
+    cudaFuncSetAttribute(k_onesweep<BITS, IPT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    k_onesweep<BITS, IPT><<<tiles, kRsThreads, stage, st>>>(ik, iv, ok, ov, n, shift, gstart, lookback, counter, err);
+}
 template <int BITS>
 static void onesweep_launch(uint32_t tiles, const uint32_t* ik, const uint32_t* iv, uint32_t* ok, uint32_t* ov,
                             uint32_t n, int shift, const uint32_t* gstart, uint32_t* lookback, uint32_t* counter,
                             uint32_t* err, cudaStream_t st) {
-    // set on every launch: the attributes belong to the current device's context
-    cudaFuncSetAttribute(k_onesweep<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RsShape<BITS>::stage);
-    cudaFuncSetAttribute(k_onesweep<BITS>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    k_onesweep<BITS><<<tiles, kRsThreads, RsShape<BITS>::stage, st>>>(ik, iv, ok, ov, n, shift, gstart, lookback, counter, err);
+    if (n <= kRsSmallMax)
+        onesweep_launch_t<BITS, kRsIptSmall>(tiles, ik, iv, ok, ov, n, shift, gstart, lookback, counter, err, st);
+    else
+        onesweep_launch_t<BITS, kRsIptLarge<BITS>>(tiles, ik, iv, ok, ov, n, shift, gstart, lookback, counter, err, st);
 }
 
 template <int BITS>
@@ -363,7 +339,7 @@ static cudaError_t radix_impl(RadixScratch& s, uint32_t* ka, uint32_t* va, uint3
     constexpr int BINS = 1 << BITS;
     int passes = std::max(1, (key_bits + BITS - 1) / BITS);
     if (passes > kMaxPasses) return cudaErrorInvalidValue;
-    const uint32_t tiles = (n + RsShape<BITS>::tile - 1) / RsShape<BITS>::tile;
+    const uint32_t tiles = onesweep_tiles<BITS>(n);
     // [digit histograms][tile counters][lookback words], cleared together
     constexpr size_t kCounterWords = 32;  // the lookback rows start on a 128-byte line
     const size_t hw = ((size_t)passes * BINS + 31) / 32 * 32,
@@ -408,7 +384,8 @@ static cudaError_t radix_impl(RadixScratch& s, uint32_t* ka, uint32_t* va, uint3
 // (4 passes of 8-bit digits): about 1.35 MB that every GPU which loads the library keeps until the
 // process exits.
 constexpr uint32_t kNoAllocMaxN = 1u << 21;
-constexpr uint32_t kNoAllocTiles = (kNoAllocMaxN + RsShape<8>::tile - 1) / RsShape<8>::tile;
+constexpr uint32_t kNoAllocTiles = (kNoAllocMaxN + RsShape<8, kRsIptLarge<8>>::tile - 1) / RsShape<8, kRsIptLarge<8>>::tile;
+static_assert((kRsSmallMax + RsShape<8, kRsIptSmall>::tile - 1) / RsShape<8, kRsIptSmall>::tile <= kNoAllocTiles, "the no-allocation scratch holds the small tiles");
 constexpr uint32_t kNoAllocPasses = 4;
 constexpr size_t kNoAllocHistWords = kNoAllocPasses * 256;
 constexpr size_t kNoAllocCounterWords = 16;  // per-pass tile counters (padded)
@@ -1052,7 +1029,7 @@ extern "C" gpsb_status gpsb_sort_pairs_noalloc(uint32_t* keys_in, uint32_t* vals
         return capture_without_setup ? GPSB_ERR_STATE : GPSB_ERR_CUDA;
     }
     const int passes = (int)((key_bits + 7) / 8);
-    const uint32_t tiles = (n + RsShape<8>::tile - 1) / RsShape<8>::tile;
+    const uint32_t tiles = onesweep_tiles<8>(n);
     uint32_t* hist = base;
     uint32_t* counters = base + kNoAllocHistWords;
     uint32_t* err = err_dev;
