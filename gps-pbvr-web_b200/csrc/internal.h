@@ -95,9 +95,12 @@ inline size_t scan_scratch_bytes(uint32_t E, uint64_t lookback_words) {
 
 // ------------------------------------------------------------------ launchers (kernels.cu)
 void launch_geometry(const FrameConst& fc, const float4* splats, const float* sh, const float* lut, float4* rec,
-                     uint2* cdesc, float4* colour, cudaStream_t st);
+                     uint2* cdesc, float4* colour, const ScanScratch& sc, size_t scratch_bytes, cudaStream_t st);
+size_t count_scan_bytes(uint32_t n, uint32_t E);  // scratch that a batch's count scan needs zeroed
 void launch_count_scan(const FrameConst& fc, const uint2* cdesc, uint32_t first_seed, uint32_t E, const ScanScratch& sc,
-                       uint2* clist, unsigned long long* stats, uint32_t* err, cudaStream_t st);
+                       bool cleared, uint2* clist, unsigned long long* sub, unsigned long long* stats, uint32_t* err,
+                       cudaStream_t st);
+void launch_clear_accum(float4* accum, uint64_t P, unsigned long long* counter, cudaStream_t st);
 void launch_fast_bounds(uint32_t* out, cudaStream_t st);
 void launch_particles(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
                       const EnsTotal* etot, uint32_t first_seed, uint32_t E, unsigned long long* sub,

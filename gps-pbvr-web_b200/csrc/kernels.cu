@@ -8,11 +8,13 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "internal.h"
 
 #include "devmath.cuh"
+#include "pdl.cuh"
 
 // Resident blocks per SM the particle kernel is compiled for (register budget).
 #ifndef GPSB_FAST_MIN_BLOCKS
@@ -97,11 +99,22 @@ __device__ __forceinline__ float2 gps_limits(const FrameConst& f, float mx, floa
 // ============================================================================ geometry
 // Once per camera: projection, opacity clamp, per-method count descriptor and particle record,
 // and the view-dependent SH colour (prepare/prepare_gps/prepare_pbvr without the seed-dependent
-// Poisson draw, gps_splat.wgsl:535-642; splat_colour :210-251).
+// Poisson draw, gps_splat.wgsl:535-642; splat_colour :210-251). It also zeroes the scratch of the first
+// batch's count scan, which saves that batch a memset.
+//
+// The kernels of a frame (this one, k_count_scan, k_particles, k_resolve, k_features and the accumulator's
+// clear) are launched with programmatic stream serialisation and wait for the previous grid as their
+// first instruction, so each is resident when the one before it ends. With the clears inside kernels a frame of
+// one batch is four launches (10k splats, 256x256, one ensemble: 24.5 -> 18.5 us; frames
+// of milliseconds the same).
 __global__ void __launch_bounds__(128) k_geometry(FrameConst f, const float4* __restrict__ splats,
                                                    const float* __restrict__ sh, float4* __restrict__ rec,
-                                                   uint2* __restrict__ cdesc, float4* __restrict__ colour) {
+                                                   uint2* __restrict__ cdesc, float4* __restrict__ colour,
+                                                   uint64_t* __restrict__ scratch, uint32_t scratch_words) {
+    grid_dependency_wait();
+    launch_dependents();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t k = i; k < scratch_words; k += gridDim.x * blockDim.x) scratch[k] = 0ull;
     if (i >= f.N) return;
     float4 g0 = __ldg(&splats[4 * (size_t)i]);
     float4 g1 = __ldg(&splats[4 * (size_t)i + 1]);
@@ -267,10 +280,11 @@ __global__ void __launch_bounds__(128) k_geometry(FrameConst f, const float4* __
 }
 
 void launch_geometry(const FrameConst& fc, const float4* splats, const float* sh, const float* lut, float4* rec,
-                     uint2* cdesc, float4* colour, cudaStream_t st) {
+                     uint2* cdesc, float4* colour, const ScanScratch& sc, size_t scratch_bytes, cudaStream_t st) {
     (void)lut;
     if (fc.N == 0) return;
-    k_geometry<<<(fc.N + 127) / 128, 128, 0, st>>>(fc, splats, sh, rec, cdesc, colour);
+    launch_pdl(k_geometry, dim3((fc.N + 127) / 128), dim3(128), 0, st, fc, splats, sh, rec, cdesc, colour, (uint64_t*)sc.mem,
+               (uint32_t)(scratch_bytes / 8));
 }
 
 // ============================================================================ count + scan
@@ -299,10 +313,13 @@ __device__ __forceinline__ uint64_t lb_pack(uint64_t status, uint64_t sum, uint3
 // Bound: the draws of small means, one uniform per event (poisson): a thread draws for all its splats in
 // one loop, going on to its next splat when one is done, so a warp runs as long as its largest sum of counts
 // instead of the sum of each round's largest count (560k splats, far view, 64 ensembles: 1.06 -> 1.03 ms; mid view, 8: 0.156 -> 0.130).
+// The draws leave the memory idle, so the blocks also clear the batch's subpixels, an equal share each
+// (the same far view's scan 1032 -> 1062 us,
+// a memset of 83 us saved; 560k splats, 4 ensembles of 1280x720 2x2: a memset of 20 us saved).
 template <int ITEMS>
 __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const uint2* __restrict__ cdesc,
-                                                             uint32_t first_seed, uint32_t tiles_per_e,
-                                                             uint64_t* lookback, uint32_t* tile_counter,
+                                                             uint32_t first_seed, uint32_t tiles_per_e, uint32_t tiles,
+                                                             ull* __restrict__ sub, uint64_t sub_words, uint64_t* lookback, uint32_t* tile_counter,
                                                              uint2* __restrict__ clist, EnsTotal* etot, ull* stats,
                                                              uint32_t* err) {
     __shared__ uint32_t s_tile;
@@ -312,10 +329,20 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
     __shared__ uint32_t s_excl_nz;
     __shared__ ull s_stat[6];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    grid_dependency_wait();
+    launch_dependents();
+    {
+        const uint64_t pairs = sub_words / 2u, per = (pairs + gridDim.x - 1u) / gridDim.x, first = blockIdx.x * per;
+        const uint64_t end = first + per < pairs ? first + per : pairs;
+        for (uint64_t k = first + tid; k < end; k += kScanThreads)
+            reinterpret_cast<uint4*>(sub)[k] = make_uint4(gxc::kEmpty, gxc::kEmpty, gxc::kEmpty, gxc::kEmpty);
+        if (blockIdx.x == 0 && tid == 0 && (sub_words & 1u)) sub[sub_words - 1u] = ~0ull;
+    }
     if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
     if (tid < 6) s_stat[tid] = 0ull;
     __syncthreads();
     const uint32_t id = s_tile;
+    if (id >= tiles) return;  // a block that was only there to clear
     const uint32_t e = id / tiles_per_e, t = id % tiles_per_e;
     const uint32_t seed = first_seed + e;
     const uint32_t N = f.N, cap = f.cap;
@@ -499,21 +526,29 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
     }
 }
 
+// few tiles of eight splats a thread leave most SMs idle: one splat a thread (10k splats, one ensemble,
+// 5 blocks: 22 us; 40 blocks: 9 us)
+static bool scan_small(uint32_t n, uint32_t E) { return (uint64_t)((n + kScanTile - 1) / kScanTile) * E < kScanSmallTiles; }
+static uint32_t count_scan_tiles(uint32_t n, uint32_t E) {
+    return scan_small(n, E) ? (n + kScanThreads - 1) / kScanThreads : (n + kScanTile - 1) / kScanTile;
+}
+size_t count_scan_bytes(uint32_t n, uint32_t E) { return scan_scratch_bytes(E, (uint64_t)E * count_scan_tiles(n, E)); }
+
 void launch_count_scan(const FrameConst& fc, const uint2* cdesc, uint32_t first_seed, uint32_t E, const ScanScratch& sc,
-                       uint2* clist, unsigned long long* stats, uint32_t* err, cudaStream_t st) {
-    const uint32_t large = (fc.N + kScanTile - 1) / kScanTile;
-    // few tiles of eight splats a thread leave most SMs idle: one splat a thread (10k splats, one ensemble,
-    // 5 blocks: 22 us; 40 blocks: 9 us)
-    const bool small = (uint64_t)large * E < kScanSmallTiles;
-    const uint32_t tiles = small ? (fc.N + kScanThreads - 1) / kScanThreads : large;
-    cudaMemsetAsync(sc.mem, 0, scan_scratch_bytes(E, (uint64_t)E * tiles), st);
+                       bool cleared, uint2* clist, unsigned long long* sub, unsigned long long* stats, uint32_t* err,
+                       cudaStream_t st) {
+    if (!cleared) cudaMemsetAsync(sc.mem, 0, count_scan_bytes(fc.N, E), st);
     if (fc.N == 0 || E == 0) return;
-    if (small)
-        k_count_scan<1><<<tiles * E, kScanThreads, 0, st>>>(fc, cdesc, first_seed, tiles, sc.lookback(E), sc.counters(), clist,
-                                                            sc.totals(), stats, err);
-    else
-        k_count_scan<kScanItems><<<tiles * E, kScanThreads, 0, st>>>(fc, cdesc, first_seed, tiles, sc.lookback(E), sc.counters(),
-                                                                     clist, sc.totals(), stats, err);
+    const uint32_t per_e = count_scan_tiles(fc.N, E), tiles = per_e * E;
+    const uint64_t sub_words = (uint64_t)E * fc.W * fc.H * fc.S;
+    // with few tiles, more blocks that only clear: 32 KB each, up to two rounds of resident blocks
+    const uint32_t grid = std::max(tiles, (uint32_t)std::min<uint64_t>((sub_words + 4095u) / 4096u, 148u * 16u));
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, dim3(grid), dim3(kScanThreads), 0, st, fc, cdesc, first_seed, per_e, tiles, sub, sub_words,
+                   sc.lookback(E), sc.counters(), clist, sc.totals(), stats, err);
+    };
+    if (scan_small(fc.N, E)) go(k_count_scan<1>);
+    else go(k_count_scan<kScanItems>);
 }
 
 // ============================================================================ particles
@@ -913,6 +948,8 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     float* s_lut = reinterpret_cast<float*>(s_ring + (FM == 1 ? (kPT / 32) * kRing : 0));
     __shared__ uint32_t s_steps;
     const int tid = threadIdx.x, lane = tid & 31;
+    grid_dependency_wait();
+    launch_dependents();
     // particles per unit: max_steps * 32, fewer when warps would get less than four units each
     // (560k splats, far view, 4 ensembles: 0.775 ms; with one unit each 0.847), but at least two steps, as every
     // block that has a unit stages its tables (10k splats: 10.2 us; one step 12.9, four 11.6)
@@ -1219,7 +1256,8 @@ static void launch_particles_t(const FrameConst& fc, const float4* rec, const fl
         cudaFuncSetAttribute(k_particles<MC, FM, FL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (known) attr[dev] = smem;
     }
-    k_particles<MC, FM, FL><<<grid, kPT, smem, st>>>(fc, rec, lut, clist, etot, first_seed, E, (uint32_t)steps, sub, unit_counter, stats);
+    launch_pdl(k_particles<MC, FM, FL>, dim3(grid), dim3(kPT), smem, st, fc, rec, lut, clist, etot, first_seed, E,
+               (uint32_t)steps, sub, unit_counter, stats);
 }
 
 void launch_particles(const FrameConst& fc, const float4* rec, const float* lut, const uint2* clist,
@@ -1295,6 +1333,8 @@ void launch_primitive(const FrameConst& fc, const float4* rec, const uint2* cdes
 __global__ void __launch_bounds__(256) k_resolve(FrameConst f, const ull* __restrict__ sub,
                                                   const EnsTotal* __restrict__ etot, const float4* __restrict__ colour,
                                                   uint32_t E, float4* accum, ull* stats) {
+    grid_dependency_wait();
+    launch_dependents();
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t P = f.W * f.H;
     if (pix >= P) return;
@@ -1334,7 +1374,7 @@ void launch_resolve(const FrameConst& fc, const unsigned long long* sub, const E
                     uint32_t E, float4* accum, unsigned long long* stats, cudaStream_t st) {
     uint32_t P = fc.W * fc.H;
     if (P == 0 || E == 0) return;
-    k_resolve<<<(P + 255) / 256, 256, 0, st>>>(fc, sub, etot, colour, E, accum, stats);
+    launch_pdl(k_resolve, dim3((P + 255) / 256), dim3(256), 0, st, fc, sub, etot, colour, E, accum, stats);
 }
 
 // Denoiser features of the batch's ensembles (no counterpart in the reference, which has no
@@ -1344,6 +1384,8 @@ void launch_resolve(const FrameConst& fc, const unsigned long long* sub, const E
 __global__ void __launch_bounds__(256) k_features(FrameConst f, const ull* __restrict__ sub,
                                                    const EnsTotal* __restrict__ etot, const float4* __restrict__ colour,
                                                    uint32_t E, float* feat) {
+    grid_dependency_wait();
+    launch_dependents();
     uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t P = f.W * f.H;
     if (pix >= P) return;
@@ -1383,7 +1425,19 @@ void launch_features(const FrameConst& fc, const unsigned long long* sub, const 
                      uint32_t E, float* feat, cudaStream_t st) {
     const uint32_t P = fc.W * fc.H;
     if (P == 0 || E == 0) return;
-    k_features<<<(P + 255) / 256, 256, 0, st>>>(fc, sub, etot, colour, E, feat);
+    launch_pdl(k_features, dim3((P + 255) / 256), dim3(256), 0, st, fc, sub, etot, colour, E, feat);
+}
+
+// A new accumulation window: the accumulator and the window's counter to zero.
+__global__ void __launch_bounds__(256) k_clear_accum(float4* __restrict__ accum, uint64_t P, ull* counter) {
+    grid_dependency_wait();
+    launch_dependents();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint64_t k = i; k < P; k += gridDim.x * blockDim.x) accum[k] = make_float4(F_(0.0), F_(0.0), F_(0.0), F_(0.0));
+    if (i == 0) *counter = 0ull;
+}
+void launch_clear_accum(float4* accum, uint64_t P, unsigned long long* counter, cudaStream_t st) {
+    launch_pdl(k_clear_accum, dim3((uint32_t)std::min<uint64_t>((P + 255u) / 256u, 148u * 16u)), dim3(256), 0, st, accum, P, counter);
 }
 
 __global__ void k_add_stat(ull* stats, int word, ull v) { stats[word] += v; }

@@ -313,34 +313,36 @@ static uint32_t pick_batch(gpsb_renderer* r, uint32_t count) {
     return (uint32_t)std::min<uint64_t>(want, fit);
 }
 
-static gpsb_status geometry(gpsb_renderer* r, const FrameConst& f) {
+// Also zeroes the first scratch_bytes of the count scan's scratch.
+static gpsb_status geometry(gpsb_renderer* r, const FrameConst& f, size_t scratch_bytes) {
     if (r->n == 0) return GPSB_OK;
     StageScope sc(r, GPSB_STAGE_GEOMETRY);
     sc.kernels(1);
     launch_geometry(f, r->splats.as<float4>(), r->sh.as<float>(), r->lut.as<float>(), r->rec.as<float4>(),
-                    r->cdesc.as<uint2>(), r->colour.as<float4>(), r->stream);
+                    r->cdesc.as<uint2>(), r->colour.as<float4>(), ScanScratch{r->scan.p}, scratch_bytes, r->stream);
     CK(r, cudaGetLastError(), "geometry kernel");
     return GPSB_OK;
 }
 
-// One batch of E ensembles (seeds first_seed..) of the current camera into `accum`.
+// One batch of E ensembles (seeds first_seed..) of the current camera into `accum`. first: the geometry
+// kernel has just zeroed the count scan's scratch.
 static gpsb_status render_batch(gpsb_renderer* r, const FrameConst& f, bool particles, uint32_t first_seed, uint32_t E,
-                                float4* accum) {
+                                bool first, float4* accum) {
     uint64_t PS = sub_per_ensemble(r);
     ull_t* stats = r->stats.as<ull_t>();
-    {
+    if (!particles) {  // the count scan clears the subpixels and counts the ensembles itself
         StageScope sc(r, GPSB_STAGE_CLEAR);
-        sc.kernels(particles ? 0 : 1);
+        sc.kernels(1);
         CK(r, cudaMemsetAsync(r->sub.p, 0xFF, (size_t)E * PS * 8, r->stream), "clear subpixels");
-        if (!particles) launch_add_stat(stats, ST_ENSEMBLES, E, r->stream);  // the count scan counts its own
+        launch_add_stat(stats, ST_ENSEMBLES, E, r->stream);
     }
     const ScanScratch scan{r->scan.p};
     if (particles) {
         {
             StageScope sc(r, GPSB_STAGE_COUNT_SCAN);
             sc.kernels(1);
-            launch_count_scan(f, r->cdesc.as<uint2>(), first_seed, E, scan, r->clist.as<uint2>(), stats,
-                              r->err.as<uint32_t>(), r->stream);
+            launch_count_scan(f, r->cdesc.as<uint2>(), first_seed, E, scan, first, r->clist.as<uint2>(),
+                              r->sub.as<ull_t>(), stats, r->err.as<uint32_t>(), r->stream);
             CK(r, cudaGetLastError(), "count/scan kernel");
         }
         {
@@ -381,14 +383,14 @@ static gpsb_status render_camera(gpsb_renderer* r, const gpsb_camera* cam, const
                                  uint32_t count, float4* accum) {
     FrameConst f = make_frame(r, *cam, *p);
     bool particles = (p->path == GPSB_PATH_PARTICLE || p->method != GPSB_METHOD_GPS) && r->n > 0;
-    gpsb_status s = geometry(r, f);
+    const uint32_t B = pick_batch(r, count);
+    gpsb_status s = ensure_batch(r, B);
     if (s != GPSB_OK) return s;
-    uint32_t B = pick_batch(r, count);
-    s = ensure_batch(r, B);
+    s = geometry(r, f, particles ? count_scan_bytes(r->n, std::min(B, count)) : 0);
     if (s != GPSB_OK) return s;
     for (uint32_t done = 0; done < count;) {
         uint32_t E = std::min(B, count - done);
-        s = render_batch(r, f, particles, first_seed + done, E, accum);
+        s = render_batch(r, f, particles, first_seed + done, E, done == 0, accum);
         if (s != GPSB_OK) return s;
         done += E;
     }
@@ -758,10 +760,11 @@ gpsb_status gpsb_resize(gpsb_renderer* r, uint32_t w, uint32_t h, uint32_t spp_s
 gpsb_status gpsb_reset_accum(gpsb_renderer* r) {
     if (!r) return fail(nullptr, GPSB_ERR_INVALID_ARGUMENT, "null renderer");
     cudaSetDevice(r->device);
-    CK(r, cudaMemsetAsync(r->accum.p, 0, (size_t)r->W * r->H * 16, r->stream), "clear accum");
-    r->accumulated = 0;
     // the skip counter belongs to the history window (gps.rs:796-800)
-    CK(r, cudaMemsetAsync(r->stats.as<unsigned long long>() + ST_SKIPPED, 0, 8, r->stream), "clear skip counter");
+    launch_clear_accum(r->accum.as<float4>(), (uint64_t)r->W * r->H, r->stats.as<ull_t>() + ST_SKIPPED, r->stream);
+    CK(r, cudaGetLastError(), "clear accum");
+    r->total_launches += 1;
+    r->accumulated = 0;
     r->latest.skipped_ensembles = 0;
     return GPSB_OK;
 }
