@@ -1109,7 +1109,7 @@ gpsb_status gpsb_sort_pairs(gpsb_renderer* r, uint32_t* ki, uint32_t* vi, uint32
     if (n > (1u << 30)) return fail(r, GPSB_ERR_LIMIT, "at most 2^30 pairs");
     cudaSetDevice(r->device);
     cudaError_t e = radix_sort_pairs(r->prim_sort, ki, vi, ko, vo, n, (int)key_bits, r->sorted.digit_bits,
-                                     r->err.as<uint32_t>(), r->stream);
+                                     r->err.as<uint32_t>(), r->stream, false, true);
     if (e != cudaSuccess) return cuda_fail(r, e, "radix sort");
     r->total_launches += 2 + (key_bits + r->sorted.digit_bits - 1) / r->sorted.digit_bits;
     return GPSB_OK;

@@ -21,10 +21,10 @@ void radix_release(RadixScratch& s);
 // Stable ascending LSD sort of `n` pairs on the low `key_bits` bits with `digit_bits` (4, 6 or 8)
 // per pass. Sorted pairs end in (keys_out, vals_out); keys_in/vals_in are used as ping-pong
 // buffers and are clobbered. An even number of passes starts from a copy of the input in (keys_out,
-// vals_out); with `placed` the caller has put the input there.
+// vals_out); with `placed` the caller has put the input there. early: programmatic launches (sorted.cu).
 cudaError_t radix_sort_pairs(RadixScratch& s, uint32_t* keys_in, uint32_t* vals_in, uint32_t* keys_out,
                              uint32_t* vals_out, uint32_t n, int key_bits, int digit_bits, uint32_t* err,
-                             cudaStream_t st, bool placed = false);
+                             cudaStream_t st, bool placed = false, bool early = false);
 
 struct SortedState {
     uint32_t cap_n = 0, cap_entries = 0, W = 0, H = 0, tw = 16, th = 16;
