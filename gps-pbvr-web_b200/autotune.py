@@ -1,6 +1,6 @@
 """Autotuner of the renderer's launch shapes, per (Gaussian count, resolution, method, path).
 
-For the particle path it sweeps items per thread {8, 16, 24} x particle blocks per SM {4, 5, 6}
+For the particle path it sweeps the unit length (particle_items) {8, 16, 24} x particle blocks per SM {4, 5, 6}
 and times a short trajectory through the captured CUDA graph (gpsb_render_trajectory_graph); for
 the depth-sorted path (GPS) it sweeps radix digit width {4, 6, 8} x blend tiles {16x16, 32x8,
 32x32} and times render_sorted. Timing: CUDA events on the renderer's stream, median of `reps`

@@ -391,7 +391,7 @@ static cudaError_t radix_impl(RadixScratch& s, uint32_t* ka, uint32_t* va, uint3
 // budget through its own pool, or a real-time frame loop where a cudaMalloc would stall or is
 // forbidden) use gpsb_sort_pairs_noalloc. Its scratch (digit histograms, tile counters and the
 // lookback words) is this file-scope array, sized for kNoAllocMaxN pairs with up to 32-bit keys
-// (4 passes of 8-bit digits): about 1.35 MB that every GPU which loads the library keeps until the
+// (4 passes of 8-bit digits): about 1.25 MB that every GPU which loads the library keeps until the
 // process exits.
 constexpr uint32_t kNoAllocMaxN = 1u << 21;
 constexpr uint32_t kNoAllocTiles = (kNoAllocMaxN + RsShape<8, kRsIptLarge<8>>::tile - 1) / RsShape<8, kRsIptLarge<8>>::tile;

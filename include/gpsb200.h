@@ -125,7 +125,7 @@ enum {
     GPSB_STAGE_COUNT_SCAN = 1,
     GPSB_STAGE_PARTICLES = 2,
     GPSB_STAGE_RESOLVE = 3,
-    GPSB_STAGE_CLEAR = 4,
+    GPSB_STAGE_CLEAR = 4,     /* primitive path; the particle path clears in its count scan */
     GPSB_STAGE_PRIMITIVE = 5,
     GPSB_STAGE_SORTED = 6,
     GPSB_STAGE_COMPOSITE = 7,
@@ -353,7 +353,7 @@ gpsb_status gpsb_p0_sample(gpsb_renderer* r, uint32_t seed, uint32_t pixel_base,
  * stall or is not allowed. It allocates nothing: all four pointers are device memory of the
  * caller; the sorted pairs are written to keys_out/vals_out and keys_in/vals_in are overwritten
  * (they are the ping-pong buffer). Its scratch is a fixed array inside this library (about
- * 1.35 MB, held by every GPU that loads the library until the process exits), which limits n to
+ * 1.25 MB, held by every GPU that loads the library until the process exits), which limits n to
  * 2,097,152 pairs; larger n returns GPSB_ERR_LIMIT. Each call whose stream is not being captured
  * looks the array's device address up (cudaGetSymbolAddress, with the call's device current), so
  * a device reset in between is harmless; a call made while its stream is being captured uses the
