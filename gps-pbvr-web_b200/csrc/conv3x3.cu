@@ -519,6 +519,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3(const __grid_constant__ C
 //   wt[g][dx][c][s][n][e]  = w[n][(3 (2 - s) + dx) * cin + g G + 8 c + e]      (stacked, N <= 64)
 __global__ void k_conv3_arrange(const bf16* w, int cout, int cin, int kp, int N, int G, int groups, int stack,
                                 bf16* wt) {
+    grid_dependency_wait();
+    launch_dependents();
     const int CH = G / 8;
     const long total = (long)groups * 9 * CH * N * 8;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -911,8 +913,8 @@ int gpsb_dn_conv3_weights(const void* w, int cout, int cin, int kp, void* wt, vo
     const int N = n_of(cout), G = g_of(N, cin), groups = (cin + G - 1) / G;
     const long total = (long)groups * 9 * (G / 8) * N * 8;
     const int blocks = (int)((total + 255) / 256 < 1184 ? (total + 255) / 256 : 1184);
-    k_conv3_arrange<<<blocks, 256, 0, (cudaStream_t)stream>>>((const bf16*)w, cout, cin, kp, N, G, groups,
-                                                              3 * N <= 256 ? 1 : 0, (bf16*)wt);
+    launch_pdl(k_conv3_arrange, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, (const bf16*)w, cout, cin, kp, N, G, groups,
+               3 * N <= 256 ? 1 : 0, (bf16*)wt);
     return (int)cudaGetLastError();
 }
 

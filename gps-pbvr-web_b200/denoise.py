@@ -302,18 +302,17 @@ class Denoiser:
         return self.loss
 
     def zero_grad(self):
-        for q in self.p.values():
-            q["gw"].zero_()
-            q["gb"].zero_()
+        import torch
+        torch._foreach_zero_([q[k] for q in self.p.values() for k in ("gw", "gb")])
 
     def adam_step(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.t += 1
-        L, st = _L(), _stream()
-        for q in self.p.values():
-            _ck(L.gpsb_dn_adam(_p(q["w"]), _p(q["gw"]), _p(q["mw"]), _p(q["vw"]), q["w"].numel(), lr, b1, b2, eps,
-                               self.t, None, st), "adam")
-            _ck(L.gpsb_dn_adam(_p(q["b"]), _p(q["gb"]), _p(q["mb"]), _p(q["vb"]), q["b"].numel(), lr, b1, b2, eps,
-                               self.t, None, st), "adam")
+        sets = [(q["w"], q["gw"], q["mw"], q["vw"]) for q in self.p.values()]
+        sets += [(q["b"], q["gb"], q["mb"], q["vb"]) for q in self.p.values()]
+        ptr = C.c_void_p * len(sets)
+        w, g, m, v = (ptr(*[t[k].data_ptr() for t in sets]) for k in range(4))
+        n = (C.c_int * len(sets))(*[t[0].numel() for t in sets])
+        _ck(_L().gpsb_dn_adam_set(len(sets), w, g, m, v, n, lr, b1, b2, eps, self.t, _stream()), "adam")
         self.sync_weights()
 
     def train_step(self, x0, base, target, lr=1e-3):

@@ -477,6 +477,10 @@ int gpsb_dn_residual(const float* base, const float* r, int n, float* out, void*
 /* Adam step t (>= 1) on n fp32 weights w with gradient g and moments m, v; wb (optional) gets bf16 w. */
 int gpsb_dn_adam(float* w, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
                  int t, void* wb, void* stream);
+/* gpsb_dn_adam (without wb) for `count` tensors: host arrays of device pointers and sizes, read before the
+ * call returns. */
+int gpsb_dn_adam_set(int count, float* const* w, const float* const* g, float* const* m, float* const* v,
+                     const int* n, float lr, float b1, float b2, float eps, int t, void* stream);
 /* dst[r][c] = bf16(c < cols ? src[r*lds + c] : 0) for c < ldd. */
 int gpsb_dn_to_bf16(const float* src, int lds, int rows, int cols, void* dst, int ldd, void* stream);
 /* Denoiser input of a frame: accum (P float4: rgb sum, count) and feature sums (P x 8 floats of
