@@ -442,8 +442,8 @@ static void centroid_of(const gpsb_gaussian* g, size_t n, double* c) {
     for (int k = 0; k < 3; ++k) c[k] = c[k] / (double)n;
 }
 
-// Enqueues the copies of `parts` (destination, pageable source, bytes) through the pinned staging with the
-// worker threads, and calls `meanwhile` on this thread. Returns when every byte has been read.
+// Copies `parts` (destination, pageable source, bytes) through the pinned staging with the
+// worker threads, and calls `meanwhile` on this thread. Returns when every byte has arrived.
 struct UploadPart {
     char* dst;
     const char* src;
@@ -468,7 +468,7 @@ static cudaError_t staged_upload(gpsb_renderer* r, const UploadPart (&parts)[2],
             if (e != cudaSuccess) break;
             memcpy(stage, p.src + at, n);
             e = cudaMemcpyAsync(p.dst + at, stage, n, cudaMemcpyHostToDevice, r->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(done, r->stream);
+            if (e == cudaSuccess && (e = cudaEventRecord(done, r->stream)) != cudaSuccess) cudaStreamSynchronize(r->stream);
         }
         if (e != cudaSuccess) failed.store(e);
     };
@@ -481,7 +481,14 @@ static cudaError_t staged_upload(gpsb_renderer* r, const UploadPart (&parts)[2],
     meanwhile();
     if (started == 0) work(0);
     for (unsigned w = 0; w < started; ++w) threads[w].join();
-    return (cudaError_t)failed.load();
+    // The workers' copies are awaited through their events: the per-thread stream handle names another stream
+    // in each thread, which the caller's wait for its own would not cover.
+    cudaError_t e = (cudaError_t)failed.load();
+    for (cudaEvent_t done : r->upload.done) {
+        const cudaError_t landed = cudaEventSynchronize(done);
+        if (e == cudaSuccess) e = landed;
+    }
+    return e;
 }
 
 // ============================================================================== C ABI
