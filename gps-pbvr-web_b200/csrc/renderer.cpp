@@ -10,7 +10,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <string>
@@ -476,7 +475,7 @@ static cudaError_t staged_upload(gpsb_renderer* r, const UploadPart (&parts)[2],
     unsigned started = 0;
     try {
         for (; started < kUploadThreads; ++started) threads[started] = std::thread(work, started);
-    } catch (const std::system_error&) {  // fewer threads, or none, do the same work
+    } catch (...) {  // no thread or no memory for one: fewer threads, or none, do the same work
     }
     meanwhile();
     if (started == 0) work(0);

@@ -1,7 +1,7 @@
 // A CUDA runtime for host-logic tests on machines without a GPU, preloaded in front of libcudart: device memory
 // is host memory, kernels are counted and their pointer arguments looked at but never run, and copies from
 // pinned memory happen only when their stream or an event behind them is waited for, as the real ones may.
-// Allocations fail where the test asks for it. fake_* are the test's controls.
+// Allocations, the library's host ones too, fail where the test asks for it. fake_* are the test's controls.
 #include <cuda_runtime.h>
 #include <cxxabi.h>
 #include <dlfcn.h>
@@ -9,8 +9,10 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <utility>
@@ -87,10 +89,25 @@ cudaError_t launch(const void* f, void** args) {
     return cudaSuccess;
 }
 int encode_tensor_map() { return 0; }
+std::atomic<long> fail_new{-1};  // operator new calls of the renderer library until one fails
 }  // namespace
+
+void* operator new(size_t n) {
+    if (fail_new.load() >= 0) {
+        Dl_info info;
+        if (dladdr(__builtin_return_address(0), &info) && strstr(info.dli_fname, "libgpsb200") && fail_new.fetch_sub(1) == 0)
+            throw std::bad_alloc();
+    }
+    void* p = malloc(n ? n : 1);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
 
 extern "C" {
 // ---- controls
+void fake_fail_new(long n) { fail_new = n; }  // the library's n-th `new` from now on throws, once; < 0: none
 void fake_fail_malloc(long n) { fail_at = n < 0 ? -1 : mallocs + n; }  // the n-th allocation from now on fails, once
 long fake_mallocs() { return mallocs; }
 long fake_launches() { return launches; }
