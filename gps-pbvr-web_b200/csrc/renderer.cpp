@@ -205,6 +205,7 @@ static gpsb_status fail(gpsb_renderer* r, gpsb_status s, const std::string& msg)
 static gpsb_status cuda_fail(gpsb_renderer* r, cudaError_t e, const char* what) {
     char buf[256];
     snprintf(buf, sizeof buf, "%s: %s", what, cudaGetErrorString(e));
+    cudaGetLastError();  // reported here, not once more by the next call's check of its launches
     gpsb_status s = (e == cudaErrorMemoryAllocation) ? GPSB_ERR_OUT_OF_MEMORY : GPSB_ERR_CUDA;
     return fail(r, s, buf);
 }

@@ -1,0 +1,17 @@
+"""Growing a buffer set that runs out of device memory half-way (the runtime faked, fake_cudart.cpp): the call
+reports it, and the next, smaller call allocates what is missing before it launches anything. Every
+allocation of the growing call fails in turn; afterwards no kernel may get a null pointer."""
+from _fake_cuda import run
+
+
+def test_an_error_is_reported_once():
+    run("""
+r = PKG.GpsRenderer(64, 48, 1)
+r.set_gaussians(scene(4000))
+fake.fake_fail_malloc(1)
+assert "out of memory" in str(raises(r.set_gaussians, scene(100_000)))
+r.reset_accum()  # the old scene is still there
+r.render_ensembles(CAM, P, 1, 2)
+r.set_gaussians(scene(500))
+r.close()
+""")
