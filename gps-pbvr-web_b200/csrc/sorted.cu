@@ -855,7 +855,8 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
     (void)sm_count;
     const uint32_t n = f.N;
     cudaError_t e;
-    if (n > s.cap_n || !s.keys_a) {
+    if (n > s.cap_n) {
+        s.cap_n = 0;  // nothing is usable until the last allocation has succeeded
         void** bufs[] = {&s.keys_a, &s.vals_a, &s.keys_b, &s.vals_b, &s.offs};
         for (void** b : bufs) {
             if (*b) cudaFree(*b);

@@ -15,3 +15,27 @@ r.render_ensembles(CAM, P, 1, 2)
 r.set_gaussians(scene(500))
 r.close()
 """)
+
+
+def test_sorted_buffers():
+    run("""
+r = PKG.GpsRenderer(64, 48, 1)
+r.set_gaussians(scene(4000))
+r.render_sorted(CAM, P, 1)
+for k in range(1, 40):
+    r.set_gaussians(scene(4000 + 4000 * k))
+    fake.fake_fail_malloc(k)
+    e = raises(r.render_sorted, CAM, P, 1)
+    fake.fake_fail_malloc(-1)
+    if e is None:
+        break
+    assert "out of memory" in str(e)
+    r.set_gaussians(scene(500))
+    fake.fake_clear()
+    r.render_sorted(CAM, P, 1)
+    # without entries, as here, their lists are null and never read
+    bad = [x for x in nulls().split(";") if x and x not in ("gpsb::k_bin_ranges#0", "gpsb::k_blend<8, 8>#7")]
+    assert fake.fake_launches() > 5 and not bad, (k, bad)
+assert k > 5
+r.close()
+""")
