@@ -289,6 +289,7 @@ static gpsb_status alloc_frame(gpsb_renderer* r) {
 // Per-ensemble buffers for E ensembles of the current scene and resolution.
 static gpsb_status ensure_batch(gpsb_renderer* r, uint32_t E) {
     if (E <= r->batch_cap) return GPSB_OK;
+    r->batch_cap = 0;  // nothing is usable until the last allocation has succeeded
     uint64_t PS = sub_per_ensemble(r);
     uint32_t tiles = (r->n + kScanTile - 1) / kScanTile;
     CK(r, r->sub.ensure((size_t)E * PS * 8), "subpixel buffers");

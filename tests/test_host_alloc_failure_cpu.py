@@ -39,3 +39,25 @@ for k in range(1, 40):
 assert k > 5
 r.close()
 """)
+
+
+def test_batch_buffers():
+    run("""
+r = PKG.GpsRenderer(64, 48, 1)
+r.set_gaussians(scene(4000))
+r.render_ensembles(CAM, P, 1, 2)
+size = 2
+for k in range(1, 10):
+    size += 3
+    fake.fake_fail_malloc(k)
+    e = raises(r.render_ensembles, CAM, P, 1, size)
+    fake.fake_fail_malloc(-1)
+    if e is None:
+        break
+    assert "out of memory" in str(e)
+    fake.fake_clear()
+    r.render_ensembles(CAM, P, 1, 1)
+    assert fake.fake_launches() > 3 and not nulls(), (k, nulls())
+assert k > 2
+r.close()
+""")
