@@ -84,9 +84,11 @@ static gpsb_status dn_fail(gpsb_denoiser* d, gpsb_status s, const std::string& m
 #define DCK(d, call, what)                                                                              \
     do {                                                                                                \
         cudaError_t e_ = (call);                                                                        \
-        if (e_ != cudaSuccess)                                                                          \
+        if (e_ != cudaSuccess) {                                                                        \
+            cudaGetLastError(); /* reported here, not once more by the next check of a launch */        \
             return dn_fail(d, e_ == cudaErrorMemoryAllocation ? GPSB_ERR_OUT_OF_MEMORY : GPSB_ERR_CUDA, \
                            std::string(what) + ": " + cudaGetErrorString(e_));                         \
+        }                                                                                               \
     } while (0)
 #define DK(d, call, what) DCK(d, (cudaError_t)(call), what)
 
@@ -171,6 +173,7 @@ gpsb_status gpsb_denoiser_set_gate(gpsb_denoiser* d, float gate_limit) {
 static gpsb_status ensure_frame(gpsb_denoiser* d, uint32_t W, uint32_t H) {
     if (d->W == W && d->H == H && d->x.p) return GPSB_OK;
     drop_graph(d);
+    d->W = d->H = 0;  // nothing is usable until the last allocation has succeeded
     const size_t P = (size_t)W * H, P2 = P / 4, P4 = P / 16;
     const size_t bf = 2;
     struct {

@@ -127,7 +127,9 @@ cudaError_t cudaGetDeviceCount(int* n) { return *n = 1, cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
-cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { return *v = 148, cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+    return *v = a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 227 * 1024 : 148, cudaSuccess;  // else: multiprocessors
+}
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { return *f = *t = (size_t)8 << 30, cudaSuccess; }
 cudaError_t cudaGetLastError() {
     const cudaError_t e = last;

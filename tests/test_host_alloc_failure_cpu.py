@@ -61,3 +61,33 @@ for k in range(1, 10):
 assert k > 2
 r.close()
 """)
+
+
+def test_denoiser_buffers():
+    run("""
+from gps_pbvr_web_b200 import denoise
+net = denoise.NativeDenoiser()
+r = PKG.GpsRenderer(64, 48, 1)
+r.set_gaussians(scene(500))
+net.render(r, CAM, P, 1, ensembles=2, gate_limit=10.0)
+for k in range(1, 60):
+    w, h = 64 + 8 * k, 48
+    big = PKG.GpsRenderer(w, h, 1)
+    big.set_gaussians(scene(500))
+    big.render_ensembles(CAM, P, 1, 2)  # its own buffers are there
+    fake.fake_fail_malloc(k)
+    failed = False
+    try:
+        net.render(big, CAM, P, 1, ensembles=2, gate_limit=10.0)
+    except Exception as e:
+        assert "out of memory" in str(e), e
+        failed = True
+    fake.fake_fail_malloc(-1)
+    big.close()
+    if not failed:
+        break
+    fake.fake_clear()
+    net.render(r, CAM, P, 1, ensembles=2, gate_limit=10.0)  # the frame size of before
+    assert fake.fake_launches() > 20 and not nulls(), (k, nulls())
+assert k > 10
+""")
