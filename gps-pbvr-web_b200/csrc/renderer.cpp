@@ -286,6 +286,11 @@ static gpsb_status alloc_frame(gpsb_renderer* r) {
     return GPSB_OK;
 }
 
+// A resize that found no memory leaves the renderer without an accumulation buffer until one succeeds.
+static gpsb_status need_frame(gpsb_renderer* r) {
+    return r->accum.p ? GPSB_OK : fail(r, GPSB_ERR_STATE, "no frame buffer: the last resize failed");
+}
+
 // Per-ensemble buffers for E ensembles of the current scene and resolution.
 static gpsb_status ensure_batch(gpsb_renderer* r, uint32_t E) {
     if (E <= r->batch_cap) return GPSB_OK;
@@ -751,7 +756,7 @@ gpsb_status gpsb_resize(gpsb_renderer* r, uint32_t w, uint32_t h, uint32_t spp_s
     if (!r) return fail(nullptr, GPSB_ERR_INVALID_ARGUMENT, "null renderer");
     cudaSetDevice(r->device);
     spp_side = clamp_side(spp_side);
-    if (w == r->W && h == r->H && spp_side == r->side) return GPSB_OK;
+    if (w == r->W && h == r->H && spp_side == r->side && r->accum.p) return GPSB_OK;
     if (w == 0 || h == 0) return fail(r, GPSB_ERR_LIMIT, "width/height must be > 0");
     CK(r, cudaStreamSynchronize(r->stream), "synchronise");
     r->W = w;
@@ -768,6 +773,8 @@ gpsb_status gpsb_resize(gpsb_renderer* r, uint32_t w, uint32_t h, uint32_t spp_s
 gpsb_status gpsb_reset_accum(gpsb_renderer* r) {
     if (!r) return fail(nullptr, GPSB_ERR_INVALID_ARGUMENT, "null renderer");
     cudaSetDevice(r->device);
+    const gpsb_status s = need_frame(r);
+    if (s != GPSB_OK) return s;
     // the skip counter belongs to the history window (gps.rs:796-800)
     launch_clear_accum(r->accum.as<float4>(), (uint64_t)r->W * r->H, r->stats.as<ull_t>() + ST_SKIPPED, r->stream);
     CK(r, cudaGetLastError(), "clear accum");
@@ -793,6 +800,7 @@ gpsb_status gpsb_render_ensembles(gpsb_renderer* r, const gpsb_camera* cam, cons
     if (count == 0) return GPSB_OK;
     cudaSetDevice(r->device);
     gpsb_status s = check_params(r, cam, p);
+    if (s == GPSB_OK) s = need_frame(r);
     if (s != GPSB_OK) return s;
     s = render_camera(r, cam, p, first_seed, count, r->accum.as<float4>());
     if (s != GPSB_OK) return s;
@@ -902,6 +910,7 @@ gpsb_status gpsb_render_sorted(gpsb_renderer* r, const gpsb_camera* cam, const g
     cudaSetDevice(r->device);
     if (r->n == 0) return fail(r, GPSB_ERR_STATE, "empty scene");
     gpsb_status s = check_params(r, cam, p);
+    if (s == GPSB_OK) s = need_frame(r);
     if (s != GPSB_OK) return s;
     gpsb_params q = *p;
     q.method = GPSB_METHOD_GPS;  // gps.rs:935
@@ -940,6 +949,8 @@ gpsb_status gpsb_probe_demand(gpsb_renderer* r, const gpsb_camera* cam, const gp
 
 gpsb_status gpsb_read_accum(gpsb_renderer* r, float* out) {
     if (!r || !out) return fail(r, GPSB_ERR_INVALID_ARGUMENT, "null renderer or output");
+    const gpsb_status s = need_frame(r);
+    if (s != GPSB_OK) return s;
     cudaSetDevice(r->device);
     CK(r, cudaMemcpyAsync(out, r->accum.p, (size_t)r->W * r->H * 16, cudaMemcpyDeviceToHost, r->stream), "read accum");
     CK(r, cudaStreamSynchronize(r->stream), "synchronise");
@@ -1010,6 +1021,8 @@ gpsb_status gpsb_sync(gpsb_renderer* r) {
 gpsb_status gpsb_composite_rgba8(gpsb_renderer* r, const gpsb_params* p, uint32_t out_w, uint32_t out_h, uint8_t* out) {
     if (!r || !p || !out) return fail(r, GPSB_ERR_INVALID_ARGUMENT, "null argument");
     if (out_w == 0 || out_h == 0) return fail(r, GPSB_ERR_INVALID_ARGUMENT, "empty composite target");
+    const gpsb_status s = need_frame(r);
+    if (s != GPSB_OK) return s;
     cudaSetDevice(r->device);
     size_t bytes = (size_t)out_w * out_h * 4;
     CK(r, r->rgba8.ensure(bytes), "composite target");

@@ -1,6 +1,7 @@
 """Growing a buffer set that runs out of device memory half-way (the runtime faked, fake_cudart.cpp): the call
 reports it, and the next, smaller call allocates what is missing before it launches anything. Every
-allocation of the growing call fails in turn; afterwards no kernel may get a null pointer."""
+allocation of the growing call fails in turn; afterwards no kernel may get a null pointer. A frame buffer
+that could not be had is refused by every call that needs it."""
 from _fake_cuda import run
 
 
@@ -90,4 +91,26 @@ for k in range(1, 60):
     net.render(r, CAM, P, 1, ensembles=2, gate_limit=10.0)  # the frame size of before
     assert fake.fake_launches() > 20 and not nulls(), (k, nulls())
 assert k > 10
+""")
+
+
+def test_frame_buffer():
+    run("""
+r = PKG.GpsRenderer(64, 48, 1)
+r.set_gaussians(scene(500))
+r.render_ensembles(CAM, P, 1, 2)
+fake.fake_fail_malloc(1)
+assert "out of memory" in str(raises(r.resize, 128, 96, 1))
+fake.fake_clear()
+cam = PKG.OrbitCamera(distance=4.0).to_camera(128, 96)
+for call in (r.reset_accum, lambda: r.render_ensembles(cam, P, 1, 2), lambda: r.render_sorted(cam, P, 1),
+             lambda: r.composite(P), r.read_accum):
+    assert raises(call) is not None
+assert not nulls(), nulls()
+r.resize(128, 96, 1)  # the same size again: there is room now
+r.reset_accum()
+r.render_ensembles(cam, P, 1, 2)
+r.composite(P)
+assert not nulls(), nulls()
+r.close()
 """)
