@@ -279,10 +279,10 @@ static gpsb_status check_params(gpsb_renderer* r, const gpsb_camera* cam, const 
 
 static gpsb_status alloc_frame(gpsb_renderer* r) {
     uint64_t P = (uint64_t)r->W * r->H;
-    CK(r, r->accum.ensure(P * 16), "accum buffer");
-    CK(r, cudaMemsetAsync(r->accum.p, 0, P * 16, r->stream), "clear accum");
     r->batch_cap = 0;  // per-ensemble buffers depend on the resolution
     r->have_sorted = false;
+    CK(r, r->accum.ensure(P * 16), "accum buffer");
+    CK(r, cudaMemsetAsync(r->accum.p, 0, P * 16, r->stream), "clear accum");
     return GPSB_OK;
 }
 

@@ -103,9 +103,12 @@ fake.fake_fail_malloc(1)
 assert "out of memory" in str(raises(r.resize, 128, 96, 1))
 fake.fake_clear()
 cam = PKG.OrbitCamera(distance=4.0).to_camera(128, 96)
+own = np.zeros((128 * 96, 4), np.float32)
+OUT = own.ctypes.data
 for call in (r.reset_accum, lambda: r.render_ensembles(cam, P, 1, 2), lambda: r.render_sorted(cam, P, 1),
              lambda: r.composite(P), r.read_accum):
     assert raises(call) is not None
+r.render_trajectory([cam], P, 1, 2, OUT)  # into the caller's buffer
 assert not nulls(), nulls()
 r.resize(128, 96, 1)  # the same size again: there is room now
 r.reset_accum()
