@@ -356,11 +356,15 @@ static cudaError_t radix_impl(RadixScratch& s, uint32_t* ka, uint32_t* va, uint3
                  words = hw + kCounterWords + (size_t)passes * std::max(tiles, 1u) * BINS;
     cudaError_t e;
     if (words * 4 > s.bytes) {
+        // room for every smaller sort too, so that none of them allocates (it may be captured): just below the
+        // line between the tile sizes there are more tiles than just above it
+        const uint32_t most = std::max(tiles, onesweep_tiles<BITS>(std::min(n, kRsSmallMax)));
+        const size_t room = (hw + kCounterWords + (size_t)passes * std::max(most, 1u) * BINS) * 4;
         if (s.mem) cudaFree(s.mem);
         s.mem = nullptr;
         s.bytes = 0;
-        if ((e = cudaMalloc(&s.mem, words * 4)) != cudaSuccess) return e;
-        s.bytes = words * 4;
+        if ((e = cudaMalloc(&s.mem, room)) != cudaSuccess) return e;
+        s.bytes = room;
     }
     uint32_t* hist = (uint32_t*)s.mem;
     uint32_t* counters = hist + hw;
