@@ -167,14 +167,14 @@ __global__ void __launch_bounds__(256) k_relu_bwd_planes(const float* g, int ldg
     for (int i = threadIdx.x; i < kPix * kCh / 4; i += 256) {
         const int p = i / (kCh / 4), q = i - p * (kCh / 4);
         if (p0 + p < HW)
-            s4[p * (kPitch / 4) + q] = __ldg(reinterpret_cast<const float4*>(g + ((size_t)b * HW + p0 + p) * ldg + goff + c0) + q);
+            s4[p * (kPitch / 4) + q] = reinterpret_cast<const float4*>(g + ((size_t)b * HW + p0 + p) * ldg + goff + c0)[q];
     }
     __syncthreads();
     for (int i = threadIdx.x; i < kPix * kCh / 8; i += 256) {
         const int ch = i / kPix, p = i - ch * kPix;
         if (p0 + p >= HW) continue;
         uint4 m = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-        if (y) m = __ldg(&y[((size_t)b * (ldy / 8) + (yoff + c0) / 8 + ch) * HW + p0 + p]);
+        if (y) m = y[((size_t)b * (ldy / 8) + (yoff + c0) / 8 + ch) * HW + p0 + p];
         const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
         const float4 u = s4[p * (kPitch / 4) + ch * 2], v = s4[p * (kPitch / 4) + ch * 2 + 1];
         const float f[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256) k_bias_grad(const bf16* dz, int chunks, i
         for (int p = p0 + threadIdx.x; p < p1; p += 256) {
             uint32_t w[4];
             if (kVec) {
-                const uint4 q = __ldg(reinterpret_cast<const uint4*>(plane) + p);
+                const uint4 q = reinterpret_cast<const uint4*>(plane)[p];
                 w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
             } else {
                 const unsigned short* h = reinterpret_cast<const unsigned short*>(plane) + (size_t)p * 8;

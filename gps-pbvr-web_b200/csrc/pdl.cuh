@@ -3,7 +3,10 @@
 // set-up overlaps its tail. Such a kernel executes griddepcontrol.wait (which returns once the
 // previous grid has completed and its memory operations are visible) before it reads anything
 // earlier work wrote or writes anything earlier work reads, and griddepcontrol.launch_dependents
-// once its own dependents may be scheduled. Captured into a CUDA graph the dependency becomes a
+// once its own dependents may be scheduled. What the previous grid writes is read with plain loads of
+// pointers without __restrict__: the read-only path (__ldg) is for data nobody writes while the kernel
+// lives, and such a kernel lives from before its predecessor's end, unless that one never executes
+// launch_dependents (its dependents start once all its blocks have exited). Captured into a CUDA graph the dependency becomes a
 // programmatic edge.
 #pragma once
 #include <cuda_runtime.h>

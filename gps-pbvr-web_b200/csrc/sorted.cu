@@ -134,13 +134,20 @@ __global__ void k_radix_hist_scan(uint32_t* hist) {
 // input index: 388 us. A sort on its own launches its kernels with programmatic stream serialisation, so that
 // a pass is resident, its rows cleared, when the one before it ends (50k pairs 42 -> 34 us, 560k 54 -> 47, 4M
 // 122 -> 109). The sorts within a frame don't: frames one after another took 0.6 % longer.
+// A pass reads what the one before it writes, so the read-only path is open to it only if that one lets it in
+// after its last write. Large tiles do so (their dependents start when their blocks exit): plain loads cost them
+// 3 to 8 % (2^24 pairs, copies of the input included: 373 us; plain loads and early dependents 398). Small tiles
+// let theirs in at once and load plainly, which costs them nothing measurable (400k pairs: 57.5 us both ways).
+// All of a thread's keys are loaded before the first is ranked, as no load passes the ranking's barriers.
 template <int BITS, int IPT>
 __global__ void __launch_bounds__(kRsThreads, RsShape<BITS, IPT>::min_blocks)
-    k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
-               uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* __restrict__ gstart, uint32_t* lookback,
+    k_onesweep(const uint32_t* kin, const uint32_t* vin, uint32_t* __restrict__ kout,
+               uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* gstart, uint32_t* lookback,
                uint32_t* tile_counter, uint32_t* err) {
     constexpr int BINS = 1 << BITS;
     constexpr int kRsTile = RsShape<BITS, IPT>::tile;
+    constexpr bool kEarly = IPT == kRsIptSmall;  // dependents start before this pass has written
+    auto load = [](const uint32_t* p) { return kEarly ? *p : __ldg(p); };
     __shared__ uint32_t s_wpos[kRsWarps][BINS];  // each warp's digit counts, then the rank in the tile of its first key of a digit
     __shared__ uint32_t s_gbase[BINS];           // global position of the digit's first key of this tile, minus its rank
     // dynamic shared memory (RsShape::stage bytes): keys, then values, in digit order. Until the ranking ends
@@ -153,7 +160,7 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS, IPT>::min_blocks)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k = tid; k < kRsWarps * BINS; k += kRsThreads) s_stage[k] = (&s_wpos[0][0])[k] = 0u;
     grid_dependency_wait();
-    launch_dependents();
+    if (kEarly) launch_dependents();
     if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
     __syncthreads();
     const uint32_t t = s_tile;
@@ -199,16 +206,15 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS, IPT>::min_blocks)
     };
     if (whole) {
 #pragma unroll
-        for (int q = 0; q < IPT; ++q) {
-            key[q] = __ldg(kin + base + q * 32);
-            rank_key(q, (key[q] >> shift) & (BINS - 1), 0xffffffffu);
-        }
+        for (int q = 0; q < IPT; ++q) key[q] = load(kin + base + q * 32);
+#pragma unroll
+        for (int q = 0; q < IPT; ++q) rank_key(q, (key[q] >> shift) & (BINS - 1), 0xffffffffu);
     } else {
 #pragma unroll
         for (int q = 0; q < IPT; ++q) {
             const uint32_t idx = base + q * 32;
             const bool valid = idx < n;
-            key[q] = valid ? __ldg(&kin[idx]) : 0u;
+            key[q] = valid ? load(kin + idx) : 0u;
             rank_key(q, valid ? ((key[q] >> shift) & (BINS - 1)) : 0u, __ballot_sync(0xffffffffu, valid));
         }
     }
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS, IPT>::min_blocks)
         if (whole || idx < n) {
             rank[q] += cnts[(key[q] >> shift) & (BINS - 1)];
             s_key[rank[q]] = key[q];
-            key[q] = __ldg(&vin[idx]);
+            key[q] = load(vin + idx);
         }
     }
 #pragma unroll
