@@ -2,8 +2,8 @@
 
 For the particle path it sweeps the unit length (particle_items) {8, 16, 24} x particle blocks per SM {4, 5, 6}
 and times a short trajectory through the captured CUDA graph (gpsb_render_trajectory_graph); for
-the depth-sorted path (GPS) it sweeps radix digit width {4, 6, 8} x blend tiles {16x16, 32x8,
-32x32} and times render_sorted. Timing: CUDA events on the renderer's stream, median of `reps`
+the depth-sorted path (GPS) it sweeps radix digit width {4, 6, 8} x blend bins {16x16, 32x32,
+64x64} and times render_sorted. Timing: CUDA events on the renderer's stream, median of `reps`
 after one warm-up. The best shape per key is cached in a JSON file and applied with
 GpsRenderer.set_tuning.
 """
@@ -14,7 +14,8 @@ import statistics
 
 PARTICLE_SPACE = [{"particle_items": i, "particle_blocks_per_sm": b} for i in (8, 16, 24) for b in (4, 5, 6)]
 SORTED_SPACE = [{"sort_digit_bits": d, "blend_tile_w": w, "blend_tile_h": h}
-                for d in (4, 6, 8) for (w, h) in ((16, 16), (32, 8), (32, 32))]
+                for d in (4, 6, 8) for (w, h) in ((16, 16), (32, 32), (64, 64))]
+SORTED_BINS = 2  # meaning of the bin sizes; sorted entries of a cache without it are measured anew
 
 
 def key(n_splats, width, height, method, sorted_path):
@@ -77,9 +78,11 @@ def tuned(renderer, cams, params, n_splats, *, sorted_path=False, cache_path=Non
     w, h = renderer.size()
     k = key(n_splats, w, h, params.method, sorted_path)
     cache = load_cache(cache_path)
-    if k not in cache:
+    if k not in cache or (sorted_path and cache[k].get("bins") != SORTED_BINS):
         best, results = tune(renderer, cams, params, sorted_path=sorted_path, **kw)
         cache[k] = {"best": best, "ms": {json.dumps(s, sort_keys=True): ms for s, ms in results}}
+        if sorted_path:
+            cache[k]["bins"] = SORTED_BINS
         if cache_path:
             with open(cache_path, "w") as f:
                 json.dump(cache, f, indent=1, sort_keys=True)

@@ -1151,11 +1151,10 @@ gpsb_status gpsb_set_tuning(gpsb_renderer* r, const gpsb_tuning* t) {
     if (!r || !t) return fail(r, GPSB_ERR_INVALID_ARGUMENT, "null argument");
     if (t->sort_digit_bits && t->sort_digit_bits != 4 && t->sort_digit_bits != 6 && t->sort_digit_bits != 8)
         return fail(r, GPSB_ERR_INVALID_ARGUMENT, "sort_digit_bits must be 4, 6 or 8");
-    if (t->blend_tile_w || t->blend_tile_h) {
-        bool ok = (t->blend_tile_w == 16 && t->blend_tile_h == 16) || (t->blend_tile_w == 32 && t->blend_tile_h == 8) ||
-                  (t->blend_tile_w == 32 && t->blend_tile_h == 32);
-        if (!ok) return fail(r, GPSB_ERR_INVALID_ARGUMENT, "blend tiles must be 16x16, 32x8 or 32x32");
-    }
+    const uint32_t bw = t->blend_tile_w, bh = t->blend_tile_h;
+    const bool bin_auto = bw == GPSB_BLEND_TILE_AUTO && bh == GPSB_BLEND_TILE_AUTO;
+    if ((bw || bh) && !bin_auto && !(bw == 32 && bh == 8) && !(bw == bh && (bw == 16 || bw == 32 || bw == 64)))
+        return fail(r, GPSB_ERR_INVALID_ARGUMENT, "blend tiles must be 16x16, 32x8, 32x32, 64x64 or automatic");
     if (t->particle_items && t->particle_items != 8 && t->particle_items != 16 && t->particle_items != 24)
         return fail(r, GPSB_ERR_INVALID_ARGUMENT, "particle_items must be 8, 16 or 24");
     if (t->particle_blocks_per_sm > 32) return fail(r, GPSB_ERR_INVALID_ARGUMENT, "particle_blocks_per_sm must be 1..32");
@@ -1163,10 +1162,11 @@ gpsb_status gpsb_set_tuning(gpsb_renderer* r, const gpsb_tuning* t) {
     cudaSetDevice(r->device);
     CK(r, cudaStreamSynchronize(r->stream), "synchronise");
     if (t->sort_digit_bits) r->sorted.digit_bits = (int)t->sort_digit_bits;
-    if (t->blend_tile_w) {
-        if (r->sorted.tw != t->blend_tile_w || r->sorted.th != t->blend_tile_h) r->have_sorted = false;
-        r->sorted.tw = t->blend_tile_w;
-        r->sorted.th = t->blend_tile_h;
+    if (bw) {
+        const uint32_t tw = bin_auto ? 0 : bw, th = bin_auto ? 0 : bh;
+        if (r->sorted.tw != tw || r->sorted.th != th) r->have_sorted = false;
+        r->sorted.tw = tw;
+        r->sorted.th = th;
     }
     if (t->particle_items) r->particle_items = t->particle_items;
     if (t->particle_blocks_per_sm) r->particle_blocks_per_sm = t->particle_blocks_per_sm;
@@ -1183,8 +1183,8 @@ gpsb_status gpsb_set_tuning(gpsb_renderer* r, const gpsb_tuning* t) {
 gpsb_status gpsb_get_tuning(const gpsb_renderer* r, gpsb_tuning* out) {
     if (!r || !out) return GPSB_ERR_INVALID_ARGUMENT;
     out->sort_digit_bits = (uint32_t)r->sorted.digit_bits;
-    out->blend_tile_w = r->sorted.tw;
-    out->blend_tile_h = r->sorted.th;
+    out->blend_tile_w = r->sorted.tw ? r->sorted.tw : GPSB_BLEND_TILE_AUTO;
+    out->blend_tile_h = r->sorted.tw ? r->sorted.th : GPSB_BLEND_TILE_AUTO;
     out->particle_items = r->particle_items;
     out->particle_blocks_per_sm = r->particle_blocks_per_sm;
     out->ensemble_batch = r->ensemble_batch;

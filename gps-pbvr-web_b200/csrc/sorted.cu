@@ -885,15 +885,14 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
         if (!s.counted && (e = cudaEventCreateWithFlags(&s.counted, cudaEventDisableTiming)) != cudaSuccess) { *what = "event"; return e; }
         s.cap_n = n;
     }
-    // Bins of the blend: the tuned shape, and by default (16 x 16) the size with the lower time of the whole
+    // Bins of the blend: the tuned shape, and by default the size with the lower time of the whole
     // frame: large frames hold larger splats, where larger bins save more in entries than they cost in
     // records tested (560k splats, 1280x720: 32 x 32 0.44 ms, 64 x 64 0.51, 16 x 16 0.47; 6M splats,
     // 3840x2160: 64 x 64 2.3 ms, 32 x 32 2.9, 16 x 16 4.8). All are multiples of the blend's 8 x 8 regions.
     TileGeom tg;
     tg.tw = s.tw;
     tg.th = s.th;
-    if (s.tw == 16) tg.tw = tg.th = (uint64_t)f.W * f.H >= kBin64Pixels ? 64u : 32u;
-    else if (s.th == 8) tg.th = 16u;
+    if (!s.tw) tg.tw = tg.th = (uint64_t)f.W * f.H >= kBin64Pixels ? 64u : 32u;
     tg.tiles_x = (f.W + tg.tw - 1) / tg.tw;
     tg.tiles_y = (f.H + tg.th - 1) / tg.th;
     cudaMemsetAsync(stats + ST_PROBE, 0, 8, st);  // the probe reports the last view (sorted.rs:316-322)

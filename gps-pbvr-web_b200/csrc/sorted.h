@@ -27,7 +27,7 @@ cudaError_t radix_sort_pairs(RadixScratch& s, uint32_t* keys_in, uint32_t* vals_
                              cudaStream_t st, bool placed = false, bool early = false);
 
 struct SortedState {
-    uint32_t cap_n = 0, cap_entries = 0, W = 0, H = 0, tw = 16, th = 16;
+    uint32_t cap_n = 0, cap_entries = 0, W = 0, H = 0, tw = 0, th = 0;  // tw, th: the tuned bins, 0 automatic
     void* keys_a = nullptr;   // n u32
     void* vals_a = nullptr;
     void* keys_b = nullptr;   // sorted keys (the test hook)

@@ -18,6 +18,9 @@ import numpy as np
 from . import abi
 
 
+BLEND_TILE_AUTO = 1  # GPSB_BLEND_TILE_AUTO
+
+
 class GpsError(RuntimeError):
     """Err(String) of the reference renderer."""
 
@@ -492,7 +495,8 @@ class GpsRenderer:
                 "ms": {n: float(p.ms[i]) for i, n in enumerate(abi.STAGES)}, "total_launches": int(p.total_launches)}
 
     def set_tuning(self, **kw):
-        """sort_digit_bits, blend_tile_w, blend_tile_h, particle_items, particle_blocks_per_sm, ensemble_batch."""
+        """sort_digit_bits, blend_tile_w, blend_tile_h (both BLEND_TILE_AUTO: chosen per frame), particle_items,
+        particle_blocks_per_sm, ensemble_batch."""
         t = abi.TuningC()
         for k, v in kw.items():
             setattr(t, k, int(v))

@@ -304,10 +304,13 @@ gpsb_status gpsb_debug_particle_seeds(gpsb_renderer* r, uint32_t slot, uint64_t 
  * form). in_dev/out_dev: n floats of device memory. Synchronous (legacy default stream). */
 gpsb_status gpsb_debug_fmath(uint32_t which, const float* in_dev, float* out_dev, uint64_t n);
 
+/* Value of both blend_tile_w and blend_tile_h: the renderer chooses the bins of every frame. */
+#define GPSB_BLEND_TILE_AUTO 1u
+
 /* Launch-shape tuning (no reference counterpart). Zero fields keep the current value.
  *   sort_digit_bits        radix digit width of the depth sort: 4, 6 or 8 (default 8)
- *   blend_tile_w/h         screen bins of the sorted blend: 16x16 (default: bins chosen by the frame's
- *                          size), 32x8 (32x16 bins) or 32x32
+ *   blend_tile_w/h         screen bins of the sorted blend in pixels: 16x16, 32x8, 32x32 or 64x64, or
+ *                          GPSB_BLEND_TILE_AUTO for both (the default)
  *   particle_items         work units of the particle kernel: 8, 16 (default) or 24 times 256 particles
  *   particle_blocks_per_sm persistent grid of the particle kernel (default 5 per SM)
  *   ensemble_batch         most ensembles per device batch (default 64, at most 1024) */

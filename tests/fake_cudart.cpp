@@ -25,7 +25,10 @@ long mallocs = 0, fail_at = -1, launches = 0;
 size_t bytes_now = 0;
 thread_local cudaError_t last = cudaSuccess;
 std::string nulls, names;  // "kernel#argument;" of every null pointer passed, "kernel;" of every launch
-std::vector<size_t> sizes;
+std::string watch;  // kernel whose parameter `watch_arg` is kept
+int watch_arg = 0;
+unsigned char watched[64];
+size_t watch_bytes = 0;
 
 struct Copy {
     void* dst;
@@ -72,6 +75,7 @@ cudaError_t launch(const void* f, void** args) {
     const size_t open = sig.rfind('('), at = sig.find("gpsb::");
     std::string name = sig.substr(at == std::string::npos ? 0 : at, open == std::string::npos ? open : open - (at == std::string::npos ? 0 : at));
     names += name + ";";
+    if (watch_bytes && name == watch) memcpy(watched, args[watch_arg], watch_bytes);
     if (open == std::string::npos) return cudaSuccess;
     int arg = 0, depth = 0;
     std::string type;
@@ -120,6 +124,8 @@ size_t fake_pending() {
 }
 const char* fake_nulls() { return nulls.c_str(); }
 const char* fake_kernels() { return names.c_str(); }
+void fake_watch(const char* kernel, int arg, size_t bytes) { watch = kernel, watch_arg = arg, watch_bytes = bytes; }
+const void* fake_watched() { return watched; }
 void fake_clear() { nulls.clear(), names.clear(), launches = 0; }
 
 // ---- the runtime
