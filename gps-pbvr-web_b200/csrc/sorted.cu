@@ -451,7 +451,8 @@ static void* noalloc_scratch_address(cudaStream_t st, cudaError_t* err, bool* ca
 }
 
 // ============================================================================ sorted path
-constexpr uint64_t kBin64Pixels = 4ull << 20;  // frames from this size on use 64 x 64 bins
+constexpr uint64_t kBin64Pixels = 4ull << 20;  // frames from this size on may use 64 x 64 bins
+constexpr ull kMaxEntries = 1ull << 30;        // of the entry lists
 // Screen bins of the blend (tw x th pixels).
 struct TileGeom {
     uint32_t tw, th, tiles_x, tiles_y;
@@ -462,14 +463,26 @@ __device__ __forceinline__ uint32_t rect_tiles(uint2 r) {
     uint32_t w = (r.y & 0xFFFFu) - (r.x & 0xFFFFu) + 1u, h = (r.y >> 16) - (r.x >> 16) + 1u;
     return w * h;
 }
+// the rectangle in bins of twice the size
+__device__ __forceinline__ uint2 halved(uint2 r) { return make_uint2((r.x >> 1) & 0x7FFF7FFFu, (r.y >> 1) & 0x7FFF7FFFu); }
+__device__ __forceinline__ uint2 coarser(uint2 r) { return r.x == 0xFFFFFFFFu ? r : halved(r); }
+// Whether the frame's bins are doubled, from its numbers of entries with either size (decided on the device, where
+// the depth sort's result is counted, and on the host alike). Larger bins have fewer entries to write and sort,
+// but every region of 8 x 8 pixels tests four times the area's records: they win where splats cover several
+// bins. Whole frame, 32 / 64 pixels, against the ratio of their entries: 6M splats at 3840x2160, 2.62 / 2.08 ms at
+// 2.7 (distance 7), 2.42 / 2.02 at 2.36, 2.13 / 1.90 at 2.10, 1.64 / 2.09 at 1.85 (distance 20), 2.23 / 4.66 at
+// 1.4 (distance 60); 560k at 2560x1700: 0.82 / 0.79 at 2.47, 0.84 / 0.84 at 2.18, 0.73 / 0.76 at 1.94, 0.54 / 0.66
+// at 1.72. Frames below 4 Mpixel keep 32 pixels (560k at 1280x720, ratio 1.83: 0.44 / 0.51).
+__host__ __device__ inline bool double_bins(const ull* entries) { return entries[0] > 2u * entries[1] || entries[0] > kMaxEntries; }
 
-// sp_project (gps_splat.wgsl:737-777) + tile rectangle
+// sp_project (gps_splat.wgsl:737-777) + bin rectangle (kBoth: entries with bins of twice the size counted too)
+template <bool kBoth>
 __global__ void __launch_bounds__(128) k_sp_project(FrameConst f, TileGeom tg, const float4* __restrict__ splats,
                                                      const float* __restrict__ sh, uint32_t* keys, uint32_t* vals,
                                                      float4* rec, uint2* rect, ull* stats, ull* entries, int full) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     ull demand = 0;
-    uint32_t bins = 0;  // bins of the splat's rectangle; their sum sizes the entry lists
+    uint32_t bins = 0, bins2 = 0;  // bins of the splat's rectangle, and of twice the size; their sums size the entry lists
     if (i < f.N) {
         if (full) {
             keys[i] = 0xFFFFFFu;
@@ -525,16 +538,35 @@ __global__ void __launch_bounds__(128) k_sp_project(FrameConst f, TileGeom tg, c
                     const uint2 r = make_uint2((x0 / tg.tw) | ((y0 / tg.th) << 16), (x1 / tg.tw) | ((y1 / tg.th) << 16));
                     rect[i] = r;
                     bins = rect_tiles(r);
+                    if (kBoth) bins2 = rect_tiles(coarser(r));
                 }
             }
         }
     }
     for (int o = 16; o; o >>= 1) demand += __shfl_xor_sync(0xffffffffu, demand, o);
-    if ((threadIdx.x & 31) == 0 && demand) atomicAdd(&stats[ST_PROBE], demand);
-    if (full) {
-        ull b = bins;
-        for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-        if ((threadIdx.x & 31) == 0 && b) atomicAdd(entries, b);
+    if constexpr (!kBoth) {
+        if ((threadIdx.x & 31) == 0 && demand) atomicAdd(&stats[ST_PROBE], demand);
+        if (full) {
+            ull b = bins;
+            for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+            if ((threadIdx.x & 31) == 0 && b) atomicAdd(entries, b);
+        }
+    } else {
+        // one addition per block: a third one per warp made a frame of 6M splats 6 % longer. A frame has at most
+        // 2^25 bins (its accumulator bounds it), so a warp's fit 32 bits.
+        __shared__ ull s_sum[3][4];
+        const uint32_t b = __reduce_add_sync(0xffffffffu, bins), b2 = __reduce_add_sync(0xffffffffu, bins2);
+        if ((threadIdx.x & 31) == 0) {
+            s_sum[0][threadIdx.x >> 5] = demand;
+            s_sum[1][threadIdx.x >> 5] = b;
+            s_sum[2][threadIdx.x >> 5] = b2;
+        }
+        __syncthreads();
+        if (threadIdx.x < 3u) {
+            const ull* w = s_sum[threadIdx.x];
+            const ull sum = w[0] + w[1] + w[2] + w[3];
+            if (sum) atomicAdd(threadIdx.x ? entries + (threadIdx.x - 1u) : &stats[ST_PROBE], sum);
+        }
     }
 }
 
@@ -547,17 +579,19 @@ __device__ __forceinline__ uint32_t entry_splat(int g) {
     return blockIdx.x * kEbSplats + (threadIdx.x >> 5) * (32 * kEbGroups) + g * 32 + (threadIdx.x & 31);
 }
 __device__ __forceinline__ uint2 sorted_rect(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect, uint32_t j,
-                                             uint32_t n) {
-    return j < n ? rect[__ldg(&vals_sorted[j])] : make_uint2(0xFFFFFFFFu, 0u);  // unbinned splats have no rectangle
+                                             uint32_t n, bool twice) {
+    const uint2 r = j < n ? rect[__ldg(&vals_sorted[j])] : make_uint2(0xFFFFFFFFu, 0u);  // unbinned splats have no rectangle
+    return twice ? coarser(r) : r;
 }
 
-// entries of every block's splats
+// entries of every block's splats; choose: the bins may be doubled, by the numbers of entries
 __global__ void __launch_bounds__(kEbT) k_entry_sums(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect,
-                                                     uint32_t n, uint32_t* sums) {
+                                                     const ull* entries, bool choose, uint32_t n, uint32_t* sums) {
     __shared__ uint32_t s[kEbT / 32];
+    const bool twice = choose && double_bins(entries);
     uint32_t v = 0;
 #pragma unroll
-    for (int g = 0; g < kEbGroups; ++g) v += rect_tiles(sorted_rect(vals_sorted, rect, entry_splat(g), n));
+    for (int g = 0; g < kEbGroups; ++g) v += rect_tiles(sorted_rect(vals_sorted, rect, entry_splat(g), n, twice));
     v = __reduce_add_sync(0xffffffffu, v);
     if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
     __syncthreads();
@@ -597,13 +631,15 @@ __global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* sums, uint32_t nb)
 }
 // first entry of every sorted splat
 __global__ void __launch_bounds__(kEbT) k_entry_offsets(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect,
-                                                        const uint32_t* __restrict__ sums, uint32_t n, uint32_t* __restrict__ offs) {
+                                                        const uint32_t* __restrict__ sums, const ull* entries, bool choose, uint32_t n,
+                                                        uint32_t* __restrict__ offs) {
+    const bool twice = choose && double_bins(entries);
     __shared__ uint32_t s[kEbT / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t c[kEbGroups], v = 0;
 #pragma unroll
     for (int g = 0; g < kEbGroups; ++g) {
-        c[g] = rect_tiles(sorted_rect(vals_sorted, rect, entry_splat(g), n));
+        c[g] = rect_tiles(sorted_rect(vals_sorted, rect, entry_splat(g), n, twice));
         v += c[g];
     }
     v = __reduce_add_sync(0xffffffffu, v);
@@ -629,10 +665,12 @@ __global__ void __launch_bounds__(kEbT) k_entry_offsets(const uint32_t* __restri
 // one took 4.4 ms at 6M splats, 3840x2160, where some splats cover the whole frame; one warp per 32
 // splats 0.85 ms, as the nearest splats, neighbours in depth order, are the largest.)
 constexpr uint32_t kEwEntries = 512;
+template <bool kTwice>
 __global__ void __launch_bounds__(256) k_entries(const uint32_t* __restrict__ vals_sorted, const uint2* __restrict__ rect,
                                                  const uint32_t* __restrict__ offs, uint32_t n, uint32_t tiles_x, uint32_t m,
                                                  uint32_t* __restrict__ ekey, uint32_t* __restrict__ eval) {
     const uint32_t lane = threadIdx.x & 31u, upto = 0xFFFFFFFFu >> (31u - lane);
+    auto bins_of = [&](uint32_t splat) { return kTwice ? halved(rect[splat]) : rect[splat]; };  // a splat with entries
     const uint32_t first = ((blockIdx.x * 256u + threadIdx.x) >> 5) * kEwEntries;
     if (first >= m) return;
     const uint32_t last = m - first < kEwEntries ? m : first + kEwEntries;
@@ -648,7 +686,7 @@ __global__ void __launch_bounds__(256) k_entries(const uint32_t* __restrict__ va
     uint32_t j = lo;
     uint32_t co = __ldg(&offs[j]), nx = j + 1u < n ? __ldg(&offs[j + 1u]) : m;
     uint32_t id = __ldg(&vals_sorted[j]);
-    uint2 r = rect[id];
+    uint2 r = bins_of(id);
     for (uint32_t p = first; p < last; p += 32u) {
         uint32_t myid = id, o = co;
         uint2 mr = r;
@@ -666,7 +704,7 @@ __global__ void __launch_bounds__(256) k_entries(const uint32_t* __restrict__ va
             uint2 sr = make_uint2(0u, 0u);
             if (starts) {
                 sid = __ldg(&vals_sorted[jj]);
-                sr = rect[sid];
+                sr = bins_of(sid);
             }
             // the c-th starting splat of the mask serves this lane's entry
             const uint32_t c = __popc(bits & upto);
@@ -704,7 +742,7 @@ __global__ void __launch_bounds__(256) k_entries(const uint32_t* __restrict__ va
             nx = j + 1u < n ? __ldg(&offs[j + 1u]) : m;
             if (nx > co) {
                 id = __ldg(&vals_sorted[j]);
-                r = rect[id];
+                r = bins_of(id);
             }
         }
     }
@@ -885,36 +923,47 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
         if (!s.counted && (e = cudaEventCreateWithFlags(&s.counted, cudaEventDisableTiming)) != cudaSuccess) { *what = "event"; return e; }
         s.cap_n = n;
     }
-    // Bins of the blend: the tuned shape, and by default the size with the lower time of the whole
-    // frame: large frames hold larger splats, where larger bins save more in entries than they cost in
-    // records tested (560k splats, 1280x720: 32 x 32 0.44 ms, 64 x 64 0.51, 16 x 16 0.47; 6M splats,
-    // 3840x2160: 64 x 64 2.3 ms, 32 x 32 2.9, 16 x 16 4.8). All are multiples of the blend's 8 x 8 regions.
+    // Bins of the blend: the tuned shape, by default 32 x 32, doubled in large frames where that is the faster
+    // (double_bins). All are multiples of the blend's 8 x 8 regions.
     TileGeom tg;
     tg.tw = s.tw;
     tg.th = s.th;
-    if (!s.tw) tg.tw = tg.th = (uint64_t)f.W * f.H >= kBin64Pixels ? 64u : 32u;
-    tg.tiles_x = (f.W + tg.tw - 1) / tg.tw;
-    tg.tiles_y = (f.H + tg.th - 1) / tg.th;
+    if (!s.tw) tg.tw = tg.th = 32u;
+    const bool choose = !s.tw && (uint64_t)f.W * f.H >= kBin64Pixels;
+    auto count_bins = [&] {
+        tg.tiles_x = (f.W + tg.tw - 1) / tg.tw;
+        tg.tiles_y = (f.H + tg.th - 1) / tg.th;
+    };
+    count_bins();
     cudaMemsetAsync(stats + ST_PROBE, 0, 8, st);  // the probe reports the last view (sorted.rs:316-322)
-    if (full) cudaMemsetAsync(s.total, 0, 8, st);
-    k_sp_project<<<(n + 127) / 128, 128, 0, st>>>(f, tg, splats, sh, (uint32_t*)s.keys_a, (uint32_t*)s.vals_a,
-                                                  (float4*)s.rec, (uint2*)s.tiles, stats, (ull*)s.total, full ? 1 : 0);
+    if (full) cudaMemsetAsync(s.total, 0, 16, st);
+    auto project = full && choose ? k_sp_project<true> : k_sp_project<false>;
+    project<<<(n + 127) / 128, 128, 0, st>>>(f, tg, splats, sh, (uint32_t*)s.keys_a, (uint32_t*)s.vals_a, (float4*)s.rec,
+                                             (uint2*)s.tiles, stats, (ull*)s.total, full ? 1 : 0);
     if ((e = cudaGetLastError()) != cudaSuccess) { *what = "sp_project kernel"; return e; }
     if (!full) return cudaSuccess;
     // the number of bin entries sizes their buffers: it comes back while the depth sort runs
-    cudaMemcpyAsync(s.host_total, s.total, 8, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(s.host_total, s.total, 16, cudaMemcpyDeviceToHost, st);
     if ((e = cudaEventRecord(s.counted, st)) != cudaSuccess) { *what = "sorted path"; return e; }
     e = radix_sort_pairs(s.rs_keys, (uint32_t*)s.keys_a, (uint32_t*)s.vals_a, (uint32_t*)s.keys_b, (uint32_t*)s.vals_b, n, 24,
                          s.digit_bits, err, st);
     if (e != cudaSuccess) { *what = "depth sort"; return e; }
     const uint32_t nb = (n + kEbSplats - 1) / kEbSplats;
-    k_entry_sums<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, n, (uint32_t*)s.sums);
+    k_entry_sums<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, (ull*)s.total, choose, n, (uint32_t*)s.sums);
     k_scan_sums<<<1, 1024, 0, st>>>((uint32_t*)s.sums, nb);
-    k_entry_offsets<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, (uint32_t*)s.sums, n, (uint32_t*)s.offs);
+    k_entry_offsets<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, (uint32_t*)s.sums, (ull*)s.total, choose, n,
+                                          (uint32_t*)s.offs);
     if ((e = cudaEventSynchronize(s.counted)) != cudaSuccess) { *what = "sorted path"; return e; }
-    const ull total = *(ull*)s.host_total;
+    const ull* totals = (const ull*)s.host_total;
+    const bool twice = choose && double_bins(totals);
+    const ull total = totals[twice ? 1 : 0];
+    if (twice) {
+        tg.tw *= 2u;
+        tg.th *= 2u;
+        count_bins();
+    }
     const uint32_t n_tiles = tg.tiles_x * tg.tiles_y;
-    if (total > (1ull << 30)) { *what = "more than 2^30 tile entries"; return cudaErrorInvalidValue; }
+    if (total > kMaxEntries) { *what = "more than 2^30 tile entries"; return cudaErrorInvalidValue; }
     const uint32_t m = (uint32_t)total;
     if (m > s.cap_entries) {
         void** bufs[] = {&s.ent_key_a, &s.ent_val_a, &s.ent_key_b, &s.ent_val_b};
@@ -938,7 +987,8 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
         while ((1u << tbits) < n_tiles) ++tbits;
         // the entries start in the buffer from which the sort's passes end in (ent_key_b, ent_val_b)
         const bool even = ((tbits + 7) / 8) % 2 == 0;
-        k_entries<<<(m + 8 * kEwEntries - 1) / (8 * kEwEntries), 256, 0, st>>>(
+        auto entries = twice ? k_entries<true> : k_entries<false>;
+        entries<<<(m + 8 * kEwEntries - 1) / (8 * kEwEntries), 256, 0, st>>>(
             (uint32_t*)s.vals_b, (uint2*)s.tiles, (uint32_t*)s.offs, n, tg.tiles_x, m,
             (uint32_t*)(even ? s.ent_key_b : s.ent_key_a), (uint32_t*)(even ? s.ent_val_b : s.ent_val_a));
         e = radix_sort_pairs(s.rs_tiles, (uint32_t*)s.ent_key_a, (uint32_t*)s.ent_val_a, (uint32_t*)s.ent_key_b,

@@ -36,7 +36,7 @@ struct SortedState {
     void* tiles = nullptr;    // n x uint2: bin rectangle of the splat (packed), x all ones when it has none
     void* sums = nullptr;     // entries of each block of sorted splats, then their exclusive sums
     void* offs = nullptr;     // n u32 first entry of every splat, in sorted order
-    void* total = nullptr;    // u64 number of bin entries, and its copy on the host with the copy's event
+    void* total = nullptr;    // 2 u64: bin entries, and with bins of twice the size; their copy on the host with its event
     void* host_total = nullptr;
     cudaEvent_t counted = nullptr;
     void* ent_key_a = nullptr; void* ent_val_a = nullptr;   // bin entries (bin, splat id)

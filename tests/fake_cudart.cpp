@@ -29,6 +29,10 @@ std::string watch;  // kernel whose parameter `watch_arg` is kept
 int watch_arg = 0;
 unsigned char watched[64];
 size_t watch_bytes = 0;
+std::string poke;  // kernel that "writes" `poke_data` to its pointer parameter `poke_arg`
+int poke_arg = 0;
+unsigned char poke_data[64];
+size_t poke_bytes = 0;
 
 struct Copy {
     void* dst;
@@ -75,7 +79,9 @@ cudaError_t launch(const void* f, void** args) {
     const size_t open = sig.rfind('('), at = sig.find("gpsb::");
     std::string name = sig.substr(at == std::string::npos ? 0 : at, open == std::string::npos ? open : open - (at == std::string::npos ? 0 : at));
     names += name + ";";
-    if (watch_bytes && name == watch) memcpy(watched, args[watch_arg], watch_bytes);
+    const std::string base = name.substr(0, name.find('<'));  // any instance of a template
+    if (poke_bytes && (name == poke || base == poke)) memcpy(*(void**)args[poke_arg], poke_data, poke_bytes);
+    if (watch_bytes && (name == watch || base == watch)) memcpy(watched, args[watch_arg], watch_bytes);
     if (open == std::string::npos) return cudaSuccess;
     int arg = 0, depth = 0;
     std::string type;
@@ -125,6 +131,10 @@ size_t fake_pending() {
 const char* fake_nulls() { return nulls.c_str(); }
 const char* fake_kernels() { return names.c_str(); }
 void fake_watch(const char* kernel, int arg, size_t bytes) { watch = kernel, watch_arg = arg, watch_bytes = bytes; }
+void fake_poke(const char* kernel, int arg, const void* data, size_t bytes) {
+    poke = kernel, poke_arg = arg, poke_bytes = bytes;
+    memcpy(poke_data, data, bytes);
+}
 const void* fake_watched() { return watched; }
 void fake_clear() { nulls.clear(), names.clear(), launches = 0; }
 

@@ -41,6 +41,33 @@ for w, h in ((64, 48), (1280, 720), (2600, 1700)):
 """)
 
 
+def test_large_frames_choose_by_their_entries():
+    run("""
+fake.fake_watch.argtypes = [C.c_char_p, C.c_int, C.c_size_t]
+fake.fake_poke.argtypes = [C.c_char_p, C.c_int, C.c_void_p, C.c_size_t]
+fake.fake_watched.restype = C.POINTER(C.c_uint32 * 2)
+for w, h, choice in ((2600, 1700, True), (1280, 720, False)):
+    r = PKG.GpsRenderer(w, h, 1)
+    r.set_gaussians(scene(100))
+    cam = PKG.OrbitCamera(distance=4.0).to_camera(w, h)
+    # entries with 32 and with 64 pixels, the bins
+    for fine, coarse, side in ((10, 5, 32), (11, 5, 64), (3, 3, 32), (0, 0, 32), (40_000, 10_001, 64)):
+        both = (C.c_uint64 * 2)(fine, coarse if choice else 0)
+        fake.fake_poke(b"gpsb::k_sp_project", 9, both, 16)
+        for arg in (3, 4):
+            fake.fake_watch(b"gpsb::k_blend<8, 8>", arg, 4)
+            r.render_sorted(cam, P, 1)
+            assert fake.fake_watched().contents[0] == (side if choice else 32), (w, fine, coarse, arg)
+        fake.fake_watch(b"gpsb::k_entries", 5, 4)  # as many entries as that size has
+        r.render_sorted(cam, P, 1)
+        assert fine == 0 or fake.fake_watched().contents[0] == (coarse if choice and side == 64 else fine)
+    if choice:  # too many small bins, not too many large ones
+        fake.fake_poke(b"gpsb::k_sp_project", 9, (C.c_uint64 * 2)((1 << 30) + 1, (1 << 30) + 1), 16)
+        assert "2^30" in str(raises(r.render_sorted, cam, P, 1))
+    r.close()
+""")
+
+
 def test_old_cache_entries_are_measured_anew(tmp_path, monkeypatch):
     pkg = load_package()
     at = importlib.import_module(pkg.__name__ + ".autotune")
