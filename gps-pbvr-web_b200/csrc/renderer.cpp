@@ -917,11 +917,12 @@ gpsb_status gpsb_render_sorted(gpsb_renderer* r, const gpsb_camera* cam, const g
     FrameConst f = make_frame(r, *cam, q);
     std::string msg;
     cudaError_t e;
+    uint32_t launches = 0;
     {
         StageScope sc(r, GPSB_STAGE_SORTED);
-        sc.kernels(10);
         e = sorted_render(r->sorted, f, r->splats.as<float4>(), r->sh.as<float>(), r->accum.as<float4>(),
-                          r->stats.as<unsigned long long>(), r->err.as<uint32_t>(), r->sm_count, true, r->stream, &msg);
+                          r->stats.as<unsigned long long>(), r->err.as<uint32_t>(), &launches, true, r->stream, &msg);
+        sc.kernels(launches);
     }
     if (e != cudaSuccess) return cuda_fail(r, e, msg.c_str());
     r->have_sorted = true;
@@ -937,11 +938,12 @@ gpsb_status gpsb_probe_demand(gpsb_renderer* r, const gpsb_camera* cam, const gp
     FrameConst f = make_frame(r, *cam, *p);
     std::string msg;
     cudaError_t e;
+    uint32_t launches = 0;
     {
         StageScope sc(r, GPSB_STAGE_SORTED);
-        sc.kernels(1);
         e = sorted_render(r->sorted, f, r->splats.as<float4>(), r->sh.as<float>(), r->accum.as<float4>(),
-                          r->stats.as<unsigned long long>(), r->err.as<uint32_t>(), r->sm_count, false, r->stream, &msg);
+                          r->stats.as<unsigned long long>(), r->err.as<uint32_t>(), &launches, false, r->stream, &msg);
+        sc.kernels(launches);
     }
     if (e != cudaSuccess) return cuda_fail(r, e, msg.c_str());
     return GPSB_OK;
@@ -1132,7 +1134,7 @@ gpsb_status gpsb_sort_pairs(gpsb_renderer* r, uint32_t* ki, uint32_t* vi, uint32
     cudaError_t e = radix_sort_pairs(r->prim_sort, ki, vi, ko, vo, n, (int)key_bits, r->sorted.digit_bits,
                                      r->err.as<uint32_t>(), r->stream, false, true);
     if (e != cudaSuccess) return cuda_fail(r, e, "radix sort");
-    r->total_launches += 2 + (key_bits + r->sorted.digit_bits - 1) / r->sorted.digit_bits;
+    if (n) r->total_launches += radix_sort_launches((int)key_bits, r->sorted.digit_bits);
     return GPSB_OK;
 }
 

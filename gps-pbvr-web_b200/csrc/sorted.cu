@@ -898,9 +898,8 @@ static void blend_launch(const SortedState& s, const FrameConst& f, const TileGe
 }
 
 cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* splats, const float* sh, float4* accum,
-                          unsigned long long* stats, uint32_t* err, int sm_count, bool full, cudaStream_t st,
+                          unsigned long long* stats, uint32_t* err, uint32_t* launches, bool full, cudaStream_t st,
                           std::string* what) {
-    (void)sm_count;
     const uint32_t n = f.N;
     cudaError_t e;
     if (n > s.cap_n) {
@@ -941,6 +940,7 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
     project<<<(n + 127) / 128, 128, 0, st>>>(f, tg, splats, sh, (uint32_t*)s.keys_a, (uint32_t*)s.vals_a, (float4*)s.rec,
                                              (uint2*)s.tiles, stats, (ull*)s.total, full ? 1 : 0);
     if ((e = cudaGetLastError()) != cudaSuccess) { *what = "sp_project kernel"; return e; }
+    *launches = 1;
     if (!full) return cudaSuccess;
     // the number of bin entries sizes their buffers: it comes back while the depth sort runs
     cudaMemcpyAsync(s.host_total, s.total, 16, cudaMemcpyDeviceToHost, st);
@@ -949,6 +949,7 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
                          s.digit_bits, err, st);
     if (e != cudaSuccess) { *what = "depth sort"; return e; }
     const uint32_t nb = (n + kEbSplats - 1) / kEbSplats;
+    *launches += radix_sort_launches(24, s.digit_bits) + 3;
     k_entry_sums<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, (ull*)s.total, choose, n, (uint32_t*)s.sums);
     k_scan_sums<<<1, 1024, 0, st>>>((uint32_t*)s.sums, nb);
     k_entry_offsets<<<nb, kEbT, 0, st>>>((uint32_t*)s.vals_b, (uint2*)s.tiles, (uint32_t*)s.sums, (ull*)s.total, choose, n,
@@ -994,9 +995,11 @@ cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* spl
         e = radix_sort_pairs(s.rs_tiles, (uint32_t*)s.ent_key_a, (uint32_t*)s.ent_val_a, (uint32_t*)s.ent_key_b,
                              (uint32_t*)s.ent_val_b, m, tbits, 8, err, st, true);
         if (e != cudaSuccess) { *what = "tile sort"; return e; }
+        *launches += 1 + radix_sort_launches(tbits, 8);
     }
     k_bin_ranges<<<n_tiles / 4 + 1, 128, 0, st>>>((uint32_t*)s.ent_key_b, m, n_tiles, (uint32_t*)s.ranges);
     blend_launch<8, 8>(s, f, tg, accum, st);
+    *launches += 2;
     if ((e = cudaGetLastError()) != cudaSuccess) { *what = "blend kernel"; return e; }
     return cudaSuccess;
 }

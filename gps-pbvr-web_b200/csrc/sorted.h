@@ -26,6 +26,9 @@ cudaError_t radix_sort_pairs(RadixScratch& s, uint32_t* keys_in, uint32_t* vals_
                              uint32_t* vals_out, uint32_t n, int key_bits, int digit_bits, uint32_t* err,
                              cudaStream_t st, bool placed = false, bool early = false);
 
+// kernels of one such sort: the histogram, its scan and the passes
+inline uint32_t radix_sort_launches(int key_bits, int digit_bits) { return 2u + (uint32_t)((key_bits + digit_bits - 1) / digit_bits); }
+
 struct SortedState {
     uint32_t cap_n = 0, cap_entries = 0, W = 0, H = 0, tw = 0, th = 0;  // tw, th: the tuned bins, 0 automatic
     void* keys_a = nullptr;   // n u32
@@ -50,7 +53,7 @@ void sorted_release(SortedState& s);
 // Projects, sorts and blends (full = true, writes accum = (rgb, 1)) or only probes the GPS
 // particle demand into stats[ST_PROBE] (full = false).
 cudaError_t sorted_render(SortedState& s, const FrameConst& f, const float4* splats, const float* sh, float4* accum,
-                          unsigned long long* stats, uint32_t* err, int sm_count, bool full, cudaStream_t st,
+                          unsigned long long* stats, uint32_t* err, uint32_t* launches, bool full, cudaStream_t st,
                           std::string* what);
 cudaError_t sorted_read(SortedState& s, uint32_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st);
 
