@@ -284,16 +284,16 @@ def run_reference(args, rank, world):
 def algorithmic_bytes_per_launch(stage, writes, entries, E, n_splats, P):
     """Bytes one launch of `stage` must move (the roofline basis, one view of E ensembles):
     writes / entries = on-screen particle writes and compact-list entries of that launch."""
-    if stage == "particles":   # one 8-byte atomicMin per written particle, list entry + 192-byte record per entry
-        return 8.0 * writes + (8.0 + 192.0) * entries
+    if stage == "particles":   # one 8-byte atomicMin per written particle, list entry + 96 bytes of record per entry
+        return 8.0 * writes + (8.0 + 96.0) * entries
     if stage == "count_scan":  # 8-byte count descriptor per splat and ensemble, 8-byte list entry written, subpixels cleared
         return 8.0 * n_splats * E + 8.0 * entries + 8.0 * P * SIDE * SIDE * E
     if stage == "resolve":     # every subpixel word of every ensemble, accum read + write
         return 8.0 * P * SIDE * SIDE * E + 32.0 * P
     if stage == "clear":       # primitive path: every subpixel word of every ensemble
         return 8.0 * P * SIDE * SIDE * E
-    if stage == "geometry":    # splat + SH3 read, record + descriptor + colour written
-        return (64.0 + 180.0 + 192.0 + 8.0 + 16.0) * n_splats
+    if stage == "geometry":    # splat + SH3 read, 96 bytes of record + descriptor + colour written
+        return (64.0 + 180.0 + 96.0 + 8.0 + 16.0) * n_splats
     return 0.0
 
 
