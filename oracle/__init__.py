@@ -51,6 +51,7 @@ def _declare(L):
         ("o2_render_sorted", C.c_int, [P, U32, P, U32, P, U32, U32, U32, P, P, P, P, P, P]),
         ("o2_composite", C.c_int, [P, U32, U32, C.c_float, U32, U32, U32, P]),
         ("o2_fmath_eval", None, [C.c_int, P, P, SZ]),
+        ("o2_fast_edge_ex2", C.c_float, [C.c_float, C.c_int]),
         ("o2_fast_check", C.c_int, [P, U32, P, U32, P, U32, U32, U32, P, P, U32, U32, U32, C.c_int, P]),
     ]:
         f = getattr(L, name)
@@ -221,7 +222,7 @@ def o2_render_ensembles(splats, sh, sh_degree, lut, w, h, spp_side, cam17, param
 
 def o2_fast_check(splats, sh, sh_degree, lut, w, h, spp_side, cam17, params, first_seed, count, perturb_seed=0,
                   mode=0):
-    """The renderer's PBVR fast decisions restated with every approximation pushed to the edge of
+    """The renderer's PBVR fast decisions (its own code) with every approximation pushed to the edge of
     its assumed error bound (mode 0 random signs, 1 all +, 2 all -), against the exact path over
     every particle: returns (particles, decided, decided wrongly, points)."""
     import ctypes

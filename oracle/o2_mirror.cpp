@@ -598,8 +598,8 @@ struct Pipeline {
 // The renderer's PBVR fast decisions (gps-pbvr-web_b200/csrc/pbvr_fast.h) with every hardware
 // approximation replaced by the exact value pushed to the edge of the error bound the decisions
 // assume: lg2 by +-(kLogAbs + kLogRel |log|) / ln 2, the Box-Muller radius by +-kErMax, sin and cos
-// by +-kSinCos, ex2 by a relative +-kExpA, reciprocals by +-2^-23 relative (signs random per operand,
-// or all + / all -). Whenever the decision answers "not a point", "a point off screen" or "a point in
+// by +-kSinCos, ex2 by a relative +-(kExpA + kExpB |x ln 2|), the form the renderer checks on the GPU,
+// reciprocals by +-2^-23 relative (signs random per operand, or all + / all -). Whenever the decision answers "not a point", "a point off screen" or "a point in
 // this subpixel", the exact path (pbvr_eval) must agree, and the exact depth must lie within the
 // decision's bound: this checks the error propagation of the decisions on the CPU, independently of
 // the device's approximations (whose constants the renderer checks exhaustively on the GPU).
@@ -608,7 +608,7 @@ using gxf::kErMax;
 using gxf::kLogAbs;
 using gxf::kLogRel;
 using gxf::kSinCos;
-constexpr float kExpA = 6e-7f;
+constexpr float kExpA = 6e-7f, kExpB = 1.5e-7f;
 constexpr float kEdge = 0.999f;  // how far to the edge of each bound the perturbations go
 
 struct Perturb {
@@ -629,7 +629,10 @@ struct Perturb {
     float cos(float t) { return gx::cos(t) + sgn() * kSinCos * kEdge; }
     float sin(float t) { return gx::sin(t) + sgn() * kSinCos * kEdge; }
     float rcp(float x) { return (float)((1.0 / (double)x) * (1.0 + sgn() * 1.19e-7 * kEdge)); }
-    float ex2(float x) { return (float)(::exp2((double)x) * (1.0 + sgn() * (double)kExpA * kEdge)); }
+    float ex2(float x) {
+        const double rel = (double)kExpA + (double)kExpB * fabs((double)x) * 0.69314718055994530942;
+        return (float)(::exp2((double)x) * (1.0 + sgn() * rel * kEdge));
+    }
     float lg2(float v) {
         if (!(v > 0.0f)) return v == 0.0f ? -INFINITY : NAN;
         const double e = ::log((double)v);
@@ -963,7 +966,6 @@ int o2_composite(const float* accum, uint32_t W, uint32_t H, float exposure, uin
     return 0;
 }
 
-// Shared-function probes for the fmath tests: out[i] = f(in[i]) for f in {exp, log, sin, cos}.
 // The fast-decision check (fastcheck above) over every particle of `count` ensembles of a PBVR
 // frame: out[0] particles, out[1] decided without an on-screen write, out[2] decided wrongly,
 // out[3] points among the particles. mode: 0 random perturbation signs (seeded by perturb_seed),
@@ -1035,6 +1037,10 @@ int o2_fast_check(const gpsb_gaussian* g, uint32_t n, const float* sh, uint32_t 
     return 0;
 }
 
+// The check's stand-in for ex2, pushed up (mode 1) or down (mode 2) to the edge of its bound.
+float o2_fast_edge_ex2(float x, int mode) { return fastcheck::Perturb{1u, mode}.ex2(x); }
+
+// Shared-function probes for the fmath tests: out[i] = f(in[i]) for f in {exp, log, sin, cos}.
 void o2_fmath_eval(int which, const float* in, float* out, size_t n) {
     for (size_t i = 0; i < n; ++i) {
         float x = in[i];
