@@ -211,10 +211,10 @@ __global__ void __launch_bounds__(kRsThreads, RsShape<BITS, IPT>::min_blocks)
         for (int q = 0; q < IPT; ++q) rank_key(q, (key[q] >> shift) & (BINS - 1), 0xffffffffu);
     } else {
 #pragma unroll
+        for (int q = 0; q < IPT; ++q) key[q] = base + q * 32 < n ? load(kin + base + q * 32) : 0u;
+#pragma unroll
         for (int q = 0; q < IPT; ++q) {
-            const uint32_t idx = base + q * 32;
-            const bool valid = idx < n;
-            key[q] = valid ? load(kin + idx) : 0u;
+            const bool valid = base + q * 32 < n;
             rank_key(q, valid ? ((key[q] >> shift) & (BINS - 1)) : 0u, __ballot_sync(0xffffffffu, valid));
         }
     }
