@@ -72,6 +72,10 @@ struct Mufu {
     __device__ __forceinline__ float rcp(float x) const { return mufu(x, 3); }
     __device__ __forceinline__ float ex2(float x) const { return mufu(x, 1); }
     __device__ __forceinline__ float lg2(float x) const { return mufu(x, 0); }
+    __device__ __forceinline__ bool every(bool b) const { return b; }
+};
+struct MufuWarp : Mufu {  // for a whole warp that decides together
+    __device__ __forceinline__ bool every(bool b) const { return __all_sync(0xffffffffu, b); }
 };
 
 // ---------------------------------------------------------------- fast decisions (GPS): position bound
@@ -934,7 +938,9 @@ constexpr bool kStageTabs = MC == 1 || FM != 1;
 //
 // MC: 0 GPS, 1 PBVR, 2 ScreenOccupancy; FM: fast decisions (0 off, 1 on, 2 validate: exact always,
 // disagreements counted), template parameters so each variant gets its own register allocation.
-// FL: the PBVR flags known at compile time (never ViewConditioned), or -1: read from f.
+// FL: the PBVR flags known at compile time, or -1: read from f, or kViewConditioned: read from f, that method
+// (the other two never are; with fast decisions only).
+constexpr int kViewConditioned = -2;
 template <int MC, int FM, int FL = -1>
 __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS : GPSB_PARTICLE_MIN_BLOCKS)
     k_particles(FrameConst f, const float4* __restrict__ rec, const float* __restrict__ lut, const uint2* clist,
@@ -998,7 +1004,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
     const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);  // lanes up to this one
     uint2* ring = s_ring + (size_t)(tid >> 5) * kRing;
     const uint32_t flags = FL >= 0 ? (uint32_t)FL : f.flags;
-    const bool vc = FL >= 0 ? false : f.method == 3u;
+    const bool vc = FM == 2 ? f.method == 3u : FL == kViewConditioned;  // of the decisions
     uint32_t points = 0, writes = 0, exact_runs = 0, mismatch = 0;
     // the first unit is the warp's own number, the next ones come from the counter (a call with no more units
     // than warps asks it nothing: thousands of warps queue up on one word)
@@ -1124,7 +1130,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                         ++writes;
                     }
                 } else if (MC == 1) {
-                    Mufu ap;
+                    MufuWarp ap;
                     gxf::Point P;
                     a = gxf::decide(ap, f.ff, flags, vc, keep, rs, q, P);
                     if (act && a == 3u) {
@@ -1190,7 +1196,7 @@ __global__ void __launch_bounds__(kPT, MC == 1 && FM == 1 ? GPSB_FAST_MIN_BLOCKS
                         if (i != curq) load_fast(i);
                         Mufu ap;
                         gxf::Point P;
-                        a = gxf::decide(ap, f.ff, f.flags, f.method == 3u, keep, rs, q, P);
+                        a = gxf::decide(ap, f.ff, f.flags, vc, keep, rs, q, P);
                         uint32_t xc;
                         float z;
                         x = pbvr_eval(f, T, rx, R, xc, z);
@@ -1285,6 +1291,8 @@ void launch_particles(const FrameConst& fc, const float4* rec, const float* lut,
         launch_particles_t<1, 1, kJR>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, items, st);
     else if (pbvr && fm == 1u && fc.flags == (uint32_t)kJ)
         launch_particles_t<1, 1, kJ>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, items, st);
+    else if (fc.method == 3u && fm == 1u)
+        launch_particles_t<1, 1, kViewConditioned>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid, items, st);
     else if (fc.method == 0u) method(std::integral_constant<int, 0>());
     else if (fc.method == 4u) method(std::integral_constant<int, 2>());
     else method(std::integral_constant<int, 1>());

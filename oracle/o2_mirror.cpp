@@ -628,6 +628,7 @@ struct Perturb {
     }
     float cos(float t) { return gx::cos(t) + sgn() * kSinCos * kEdge; }
     float sin(float t) { return gx::sin(t) + sgn() * kSinCos * kEdge; }
+    bool every(bool b) { return b; }
     float rcp(float x) { return (float)((1.0 / (double)x) * (1.0 + sgn() * 1.19e-7 * kEdge)); }
     float ex2(float x) {
         const double rel = (double)kExpA + (double)kExpB * fabs((double)x) * 0.69314718055994530942;
