@@ -79,7 +79,11 @@ struct EnsTotal {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr uint32_t kScanSmallTiles = 2 * 148;  // below this many tiles a batch is scanned with one splat a thread
+// Below this many tiles a batch is scanned with one splat a thread: more blocks draw, but the lookback's chain
+// has eight times the links. One ensemble at 1280x720, one / eight splats a thread, GPS and ScreenOccupancy:
+// 10k splats (5 tiles) 9 / 22 us of scan, 100k (49) 20 / 27 and 20 / 23, 200k (98) 22 / 30 and 22 / 25, 250k (123)
+// 26 / 29 and 25 / 25, 300k (147) 31 / 29 and 29 / 25, 560k (274) 42 / 33 and 40 / 29.
+constexpr uint32_t kScanSmallTiles = 128;
 
 // Scratch of a batch's count scan and particle kernels, cleared by one memset per batch: [64 bytes of counters:
 // scan tiles, particle units][EnsTotal of each ensemble][lookback words].

@@ -531,8 +531,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(FrameConst f, const
     }
 }
 
-// few tiles of eight splats a thread leave most SMs idle: one splat a thread (10k splats, one ensemble,
-// 5 blocks: 22 us; 40 blocks: 9 us)
+// few tiles of eight splats a thread leave most SMs idle: one splat a thread
 static bool scan_small(uint32_t n, uint32_t E) { return (uint64_t)((n + kScanTile - 1) / kScanTile) * E < kScanSmallTiles; }
 static uint32_t count_scan_tiles(uint32_t n, uint32_t E) {
     return scan_small(n, E) ? (n + kScanThreads - 1) / kScanThreads : (n + kScanTile - 1) / kScanTile;
