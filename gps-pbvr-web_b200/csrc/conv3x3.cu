@@ -635,7 +635,10 @@ static cudaError_t launch(const bf16* x, int ldx, int xoff, int cin, const Param
 // in the registers of eight warps: the tensor core drops the low bits of what it adds to a growing
 // accumulator, about half a unit in the last place a step, so a chain per CTA (hundreds of steps) would
 // lose 1e-5 of the result. The sums are added to dw once.
-// Pixels and rows outside the image are TMA's zero fill in both operands.
+// Pixels and rows outside the image are TMA's zero fill in both operands. A K-step's pixels past the image's last
+// column have dY = 0 but, for dx = 0, the last column itself in X, which may be inf or NaN: where the width is
+// not a multiple of 16, that one K-step's dx = 0 operand is a small tile of its own, fetched through a map that
+// ends one pixel earlier. Rows past the last are not multiplied at all.
 // Roles: lane 0 of warp 0 issues the TMA boxes (one per operand and stage), lane 0 of warp 1 the MMAs,
 // warps 2-9 (two per tensor-memory lane quarter, each half of the columns) keep the sums. Waits are
 // bounded as in k_conv3.
@@ -653,33 +656,35 @@ struct DwCfg {
     static constexpr int FLUSH = 24 / R;                      // units between read-backs: 168 K-steps at most
     static constexpr int N = CHX == 1 ? 32 : 24 * CHX;        // one MMA's columns (24 used of 32 for one plane)
     static constexpr int XB = (R + 2) * CHX * kRow, YB = R * CHY * kDwSeg * 16;  // room for the operands of a stage
-    static constexpr int STAGE = YB + XB;
+    static constexpr int EB = (R + 2) * CHX * 256;                               // and for the edge tile of X
+    static constexpr int STAGE = YB + XB + EB;
     static constexpr int S = 2;
-    // rows past cout read up to (16 - CHY) planes past the last dY row, the 25th..32nd column one X row
-    // past the last: both stay within the stage behind them or this slack
-    static constexpr size_t SLACK = 4096;
-    static_assert((16 - CHY) * kDwSeg * 16 <= XB + 4096, "reads past the last dY plane");
-    static constexpr size_t SMEM = (size_t)S * STAGE + SLACK + 1024;
-    static_assert(STAGE % 128 == 0 && SMEM <= 227 * 1024, "shared memory of one CTA");
+    // rows past cout read up to (16 - CHY) planes past the last dY row, the 25th..32nd column (one plane only) one
+    // X row past the last: both stay within the stage behind them or this slack
+    static constexpr size_t SLACK = CHX == 1 ? 4096 : 0;
+    static_assert((16 - CHY) * kDwSeg * 16 <= XB + EB + SLACK, "reads past the last dY plane");
+    static constexpr size_t SMEM = (size_t)S * STAGE + SLACK;
+    static_assert(YB % 128 == 0 && XB % 128 == 0 && EB % 128 == 0 && SMEM + 1024 <= 227 * 1024, "shared memory of one CTA (1024 static)");
     static_assert(3 * N <= 512 && 3 * N % 32 == 0, "tensor-memory columns, halved in units of 16");
 };
 
 struct DwParams {
     float* dw;  // [cout][kp], k = tap * cin + ci
-    int cout, kp, cin, groups, splits, units, segs, rowblocks, W;
+    int cout, kp, cin, groups, splits, units, segs, rowblocks, W, H;
     int seg, xpx;  // pixels of a segment and of the staged X row (seg + 16), multiples of 16
+    int edge, ex;  // whether the last segment's last K-step has an edge tile, and where it starts (8-byte elements)
     uint32_t* err;
 };
 
 template <int CHX, int CHY>
 __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant__ CUtensorMap ymap,
-                                                          const __grid_constant__ CUtensorMap xmap, const DwParams p) {
+                                                          const __grid_constant__ CUtensorMap xmap,
+                                                          const __grid_constant__ CUtensorMap emap, const DwParams p) {
     using C = DwCfg<CHX, CHY>;
-    extern __shared__ __align__(1024) uint8_t s_raw[];
+    extern __shared__ __align__(128) uint8_t base[];
     __shared__ __align__(8) uint64_t s_full[C::S], s_empty[C::S], s_acc_full, s_acc_empty, s_drain;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s_tmem)), "r"(512u)
@@ -720,10 +725,12 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant
                     fail();
                     break;
                 }
-                bar_expect(&s_full[stage], (uint32_t)(C::R * CHY * p.seg * 16 + (C::R + 2) * CHX * p.xpx * 16));
+                const bool edge = p.edge && seg == p.segs - 1;
+                bar_expect(&s_full[stage], (uint32_t)(C::R * CHY * p.seg * 16 + (C::R + 2) * CHX * p.xpx * 16 + (edge ? C::EB : 0)));
                 const uint32_t st = saddr(base + (size_t)stage * C::STAGE);
                 tma_load4(st, &ymap, 2 * p.seg * seg, 0, rb * C::R, b, &s_full[stage]);
                 tma_load4(st + C::YB, &xmap, 2 * (p.seg * seg - 1), g * CHX, rb * C::R - 1, b, &s_full[stage]);
+                if (edge) tma_load4(st + C::YB + C::XB, &emap, p.ex, g * CHX, rb * C::R - 1, b, &s_full[stage]);
                 armed |= 1u << stage;
                 if (++stage == C::S) {
                     stage = 0;
@@ -764,20 +771,23 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int left = p.W - ((split + i * p.splits) % p.segs) * p.seg;
+                const int u = split + i * p.splits, seg = u % p.segs, y0 = (u / p.segs) % p.rowblocks * C::R;
+                const int left = p.W - seg * p.seg, rows = p.H - y0 < C::R ? p.H - y0 : C::R;
                 const int steps = ((left < p.seg ? left : p.seg) + 15) / 16;
+                const int edge = p.edge && seg == p.segs - 1 ? steps - 1 : -1;  // the K-step with the edge tile
                 const uint32_t st = saddr(base + (size_t)stage * C::STAGE);
                 // leading byte offset: the next 8 pixels; stride byte offset: the next 8 channels
-                const uint64_t a0 = desc(st, 128, sy), b0 = desc(st + C::YB, 128, sx);
+                const uint64_t a0 = desc(st, 128, sy), b0 = desc(st + C::YB, 128, sx), e0 = desc(st + C::YB + C::XB, 128, 256);
 #pragma unroll 1
-                for (int r = 0; r < C::R; ++r) {
+                for (int r = 0; r < rows; ++r) {
 #pragma unroll 1
                     for (int k = 0; k < steps; ++k) {
                         const uint64_t ad = a0 + (uint64_t)(r * CHY * (int)(sy / 16) + k * 16);
                         const uint64_t bd = b0 + (uint64_t)(r * CHX * (int)(sx / 16) + k * 16);
+                        const uint64_t bl = k == edge ? e0 + (uint64_t)(r * CHX * 16) : bd;  // dx = 0
 #pragma unroll
                         for (int dx = 0; dx < 3; ++dx)
-                            umma::mma_bf16(tmem + (uint32_t)(dx * C::N), ad, bd + (uint64_t)dx, id, !fresh);
+                            umma::mma_bf16(tmem + (uint32_t)(dx * C::N), ad, dx == 0 ? bl : bd + (uint64_t)dx, id, !fresh);
                         fresh = false;
                     }
                 }
@@ -850,12 +860,12 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-// (2 W, plane, H, B) view of channels [off, off + c) of a chunk-planar tensor of ld channels, as 8-byte
-// elements; boxes of px pixels x planes x rows
-static CUresult planes_map(CUtensorMap* map, const bf16* x, int ld, int off, int c, int B, int H, int W, int px, int planes,
-                           int rows) {
+// (2 w, plane, H, B) view of the first w columns of channels [off, off + c) of a chunk-planar tensor of ld channels
+// and width W, as 8-byte elements; boxes of px pixels x planes x rows
+static CUresult planes_map(CUtensorMap* map, const bf16* x, int ld, int off, int c, int B, int H, int W, int w, int px,
+                           int planes, int rows) {
     const cuuint64_t plane = (cuuint64_t)W * H * 16;
-    const cuuint64_t dims[4] = {(cuuint64_t)W * 2, (cuuint64_t)((c + 7) / 8), (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t dims[4] = {(cuuint64_t)w * 2, (cuuint64_t)((c + 7) / 8), (cuuint64_t)H, (cuuint64_t)B};
     const cuuint64_t strides[3] = {plane, (cuuint64_t)W * 16, plane * (cuuint64_t)(ld / 8)};
     const cuuint32_t box[4] = {(cuuint32_t)(2 * px), (cuuint32_t)planes, (cuuint32_t)rows, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
@@ -873,9 +883,15 @@ static cudaError_t launch_dw(const bf16* dy, int ldy, const bf16* x, int ldx, in
     q.seg = ((q.W + q.segs - 1) / q.segs + 15) / 16 * 16;
     q.segs = (q.W + q.seg - 1) / q.seg;
     q.xpx = q.seg + 16;
-    CUtensorMap ymap, xmap;
-    if (planes_map(&ymap, dy, ldy, 0, q.cout, B, H, q.W, q.seg, CHY, Cf::R) != CUDA_SUCCESS ||
-        planes_map(&xmap, x, ldx, xoff, q.cin, B, H, q.W, q.xpx, CHX, Cf::R + 2) != CUDA_SUCCESS)
+    // the edge tile: 16 pixels from the one before the last K-step's first, through a map without the last column
+    // (of a single column every pixel lies past the map's end)
+    q.H = H;
+    q.edge = q.W % 16 != 0;
+    q.ex = q.W == 1 ? 2 * 16 : 2 * (q.W / 16 * 16 - 1);
+    CUtensorMap ymap, xmap, emap;
+    if (planes_map(&ymap, dy, ldy, 0, q.cout, B, H, q.W, q.W, q.seg, CHY, Cf::R) != CUDA_SUCCESS ||
+        planes_map(&xmap, x, ldx, xoff, q.cin, B, H, q.W, q.W, q.xpx, CHX, Cf::R + 2) != CUDA_SUCCESS ||
+        planes_map(&emap, x, ldx, xoff, q.cin, B, H, q.W, q.W == 1 ? 1 : q.W - 1, 16, CHX, Cf::R + 2) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     q.rowblocks = (H + Cf::R - 1) / Cf::R;
     q.units = q.segs * q.rowblocks * B;
@@ -888,7 +904,7 @@ static cudaError_t launch_dw(const bf16* dy, int ldy, const bf16* x, int ldx, in
     if (q.splits <= 0) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(k_conv_dw<CHX, CHY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cf::SMEM);
     if (e != cudaSuccess) return e;
-    k_conv_dw<CHX, CHY><<<q.groups * q.splits, kDwThreads, Cf::SMEM, st>>>(ymap, xmap, q);
+    k_conv_dw<CHX, CHY><<<q.groups * q.splits, kDwThreads, Cf::SMEM, st>>>(ymap, xmap, emap, q);
     return cudaGetLastError();
 }
 
