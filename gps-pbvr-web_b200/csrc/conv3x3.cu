@@ -141,6 +141,24 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, volatile 
     }
     return false;
 }
+// What the producer had issued when it ended: the stage after its last copy, that stage's phase, a bit per stage used.
+struct Issued {
+    int stage;
+    uint32_t phase, armed;
+};
+// Waits (bounded) until every stage's last copy has landed, which its transaction count alone completes: a block
+// that gave a wait up must not exit before.
+__device__ __forceinline__ void drain_copies(uint64_t* full, int stages, Issued q) {
+    for (int k = 0; k < stages; ++k) {
+        if (--q.stage < 0) {
+            q.stage = stages - 1;
+            q.phase ^= 1u;
+        }
+        if (q.armed & (1u << q.stage))
+            for (uint32_t i = 0; i < kSpin && !bar_test(&full[q.stage], q.phase); ++i) {
+            }
+    }
+}
 __device__ __forceinline__ void bar_arrive(uint64_t* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
 }
@@ -235,6 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3(const __grid_constant__ C
     __shared__ __align__(8) uint64_t s_full[C::S], s_empty[C::S], s_acc_full[2], s_acc_empty[2], s_drain[2], s_wbar;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
+    __shared__ Issued s_issued;
     __shared__ __align__(16) float s_bias[N];  // bias of the N accumulator columns (0 past cout)
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -325,26 +344,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3(const __grid_constant__ C
                     }
                 }
             }
-            if (s_abort) {
-                // let this CTA's copies land before the CTA can exit: every stage's last armed phase
-                // (and the resident weights' barrier) completes by its transaction count alone
-                if (p.resident) {
-                    for (uint32_t i = 0; i < kSpin && !bar_test(&s_wbar, 0); ++i) {
-                    }
-                }
-                int st2 = stage;
-                uint32_t ph2 = phase;
-                for (int k = 0; k < C::S; ++k) {
-                    if (--st2 < 0) {
-                        st2 = C::S - 1;
-                        ph2 ^= 1u;
-                    }
-                    if (armed & (1u << st2)) {
-                        for (uint32_t i = 0; i < kSpin && !bar_test(&s_full[st2], ph2); ++i) {
-                        }
-                    }
-                }
-            }
+            s_issued = Issued{stage, phase, armed};
         }
         __syncwarp();
     } else if (warp < kEpiWarp0) {
@@ -509,6 +509,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3(const __grid_constant__ C
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (s_abort && tid == 0) {
+        if (p.resident)
+            for (uint32_t i = 0; i < kSpin && !bar_test(&s_wbar, 0); ++i) {
+            }
+        drain_copies(s_full, C::S, s_issued);
+    }
+    __syncwarp();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * kAccCols) : "memory");
 }
@@ -685,6 +692,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant
     __shared__ __align__(8) uint64_t s_full[C::S], s_empty[C::S], s_acc_full, s_acc_empty, s_drain;
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
+    __shared__ Issued s_issued;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s_tmem)), "r"(512u)
@@ -737,17 +745,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant
                     phase ^= 1u;
                 }
             }
-            if (!ok) {  // this CTA's copies land before it can exit
-                for (int k = 0; k < C::S; ++k) {
-                    if (--stage < 0) {
-                        stage = C::S - 1;
-                        phase ^= 1u;
-                    }
-                    if (armed & (1u << stage))
-                        for (uint32_t i = 0; i < kSpin && !bar_test(&s_full[stage], phase); ++i) {
-                        }
-                }
-            }
+            s_issued = Issued{stage, phase, armed};
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -857,6 +855,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_conv_dw(const __grid_constant
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (s_abort && tid == 0) drain_copies(s_full, C::S, s_issued);
+    __syncwarp();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
