@@ -976,7 +976,7 @@ int gpsb_dn_conv3(const void* x, int ldx, int xoff, int cin, int B, int H, int W
 int gpsb_dn_conv_dw(const void* dy, int ldy, const void* x, int ldx, int xoff, int cin, int B, int H, int W, int cout,
                     int kp, float* dw, void* stream, uint32_t* err) {
     if (cin % 8 || ldx % 8 || xoff % 8 || ldy % 8 || kp < 9 * cin || cout < 1 || cout > 128) return (int)cudaErrorInvalidValue;
-    if (cin < 1 || B < 1 || H < 1 || W < 1) return (int)cudaSuccess;
+    if (cin < 1 || B < 1 || H < 1 || W < 1) return (int)cudaErrorInvalidConfiguration;  // an empty grid
     if (!dy || !x || !dw || cout > ldy || xoff < 0 || xoff + cin > ldx ||
         ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 15u))
         return (int)cudaErrorInvalidValue;

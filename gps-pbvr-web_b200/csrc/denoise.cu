@@ -571,7 +571,8 @@ int gpsb_dn_pool2_bwd_add(const float* g, int B, int h, int w, int C, float* acc
 }
 int gpsb_dn_bias_grad(const void* dz, int ld, int B, int HW, int C, float* db, void* stream) {
     if (C > 256 || ld % 8 || C > ld) return (int)cudaErrorInvalidValue;
-    if (C < 1 || B < 1 || HW < 1) return (int)cudaSuccess;
+    if (B < 1 || HW < 1) return (int)cudaErrorInvalidConfiguration;  // an empty grid
+    if (C < 1) return (int)cudaSuccess;
     // about four blocks per SM, each at least 2048 pixels
     const long planes = (long)((C + 7) / 8) * B;
     const int want = (int)((148 * 4 + planes - 1) / planes), most = (HW + 2047) / 2048;
@@ -587,7 +588,8 @@ int gpsb_dn_bias_grad(const void* dz, int ld, int B, int HW, int C, float* db, v
 int gpsb_dn_l1(const float* base, const float* r, const float* target, int M, float* loss_sum, void* dr, float scale,
                void* stream) {
     const int blocks = grid_of(M) < 148 * 4 ? grid_of(M) : 148 * 4;
-    if (blocks > 0) k_l1<<<blocks, 256, 0, (cudaStream_t)stream>>>(base, r, target, M, loss_sum, (bf16*)dr, scale);
+    if (blocks <= 0) return (int)cudaErrorInvalidConfiguration;  // an empty grid
+    k_l1<<<blocks, 256, 0, (cudaStream_t)stream>>>(base, r, target, M, loss_sum, (bf16*)dr, scale);
     return (int)cudaGetLastError();
 }
 int gpsb_dn_residual(const float* base, const float* r, int n, float* out, void* stream) {

@@ -247,6 +247,11 @@ cudaError_t cudaEventElapsedTime(float* t, cudaEvent_t, cudaEvent_t) { return *t
 
 cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) { return memset(a, 0, sizeof *a), cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t) { return launch(f, args); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { return launch(f, args); }
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3 block, void** args, size_t, cudaStream_t) {
+    if (!grid.x || !grid.y || !grid.z || !block.x || !block.y || !block.z) return set(cudaErrorInvalidConfiguration);
+    return launch(f, args);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) {
+    return cudaLaunchKernel(f, c->gridDim, c->blockDim, args, c->dynamicSmemBytes, c->stream);
+}
 }
