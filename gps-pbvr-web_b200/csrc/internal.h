@@ -80,10 +80,12 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 // Below this many tiles a batch is scanned with one splat a thread: more blocks draw, but the lookback's chain
-// has eight times the links. One ensemble at 1280x720, one / eight splats a thread, GPS and ScreenOccupancy:
-// 10k splats (5 tiles) 9 / 22 us of scan, 100k (49) 20 / 27 and 20 / 23, 200k (98) 22 / 30 and 22 / 25, 250k (123)
-// 26 / 29 and 25 / 25, 300k (147) 31 / 29 and 29 / 25, 560k (274) 42 / 33 and 40 / 29.
-constexpr uint32_t kScanSmallTiles = 128;
+// has eight times the links. Whole frames at 320x180, us with one / eight splats a thread, GPS, Extinction and
+// ScreenOccupancy: 50k splats, 1 ensemble (25 tiles) 39 / 57, 89 / 116, 85 / 100; 200k, 1 (98) 85 / 93, 149 / 170,
+// 115 / 123; 200k, 2 (196) 122 / 124, 236 / 247, 195 / 197; 50k, 8 (200) 115 / 125, 235 / 250, 193 / 198; 560k, 1
+// (274) 151 / 148, 319 / 327, 270 / 266; 300k, 2 (294) 140 / 135, 318 / 321, 269 / 263; 200k, 4 (392) 163 / 151,
+// 408 / 401, 348 / 334; 560k, 4 (1096) 299 / 245, 964 / 921, 885 / 826.
+constexpr uint32_t kScanSmallTiles = 240;
 
 // Scratch of a batch's count scan and particle kernels, cleared by one memset per batch: [64 bytes of counters:
 // scan tiles, particle units][EnsTotal of each ensemble][lookback words].
