@@ -149,8 +149,8 @@ struct Point {
 // 0 not a point, 1 a point off screen, 2 undecided, 3 a point on screen or within e of its edge (at P).
 // vc: the ViewConditioned draw against `keep` comes first (exact), and where ap.every(dropped) says so
 // (every lane of a warp) nothing else is computed, as from far away almost no particle is kept: 560k splats,
-// 1280x720, 4 ensembles, distance 60 (0.3 % kept) 12.7 -> 6.9 ms (the exact path of each lane, left at its draw,
-// takes 10.4), 20: 13.4 -> 9.5, 7: 14.0 -> 13.4, 2.5: 11.4 -> 11.6. Otherwise straight-line code: the lanes of a
+// 1280x720, 4 ensembles, distance 60 (0.3 % kept) 12.7 -> 6.8 ms (the exact path of each lane, left at its draw,
+// takes 10.4), 20: 13.4 -> 9.5, 7: 13.9 -> 13.3, 2.5: 10.5 both, with 2x2 subpixels 11.2 -> 11.3. Otherwise straight-line code: the lanes of a
 // warp rarely agree on an early exit.
 template <class A>
 GX_HD uint32_t decide(A& ap, const Frame& F, uint32_t flags, bool vc, float keep, uint32_t st, const float* q, Point& P) {
