@@ -1284,7 +1284,7 @@ void launch_particles(const FrameConst& fc, const float4* rec, const float* lut,
         else go(mc, std::integral_constant<int, 0>());
     };
     // the two common flag sets of the fast PBVR decisions, compiled with the flags known (ViewConditioned, 560k
-    // splats, 1280x720, 4 ensembles, jitter and radial, read / known: distance 2.5 10.71 / 10.53 ms, 20 9.64 / 9.49)
+    // splats, 1280x720, 4 ensembles, jitter and radial, read / known: distance 2.5 10.71 / 10.57 ms, 20 9.64 / 9.50)
     constexpr int kJR = (int)(FLAG_JITTER | FLAG_RADIAL), kJ = (int)FLAG_JITTER;
     auto known = [&](auto fl) {
         launch_particles_t<1, 1, decltype(fl)::value>(fc, rec, lut, clist, etot, first_seed, E, sub, unit_counter, stats, grid,

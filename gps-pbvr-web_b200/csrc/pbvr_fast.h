@@ -128,12 +128,13 @@ GX_HD void make_record(const Frame& F, const float* rot0, const float* rot1, con
     }
 }
 
-// One Box-Muller pair from two consecutive states of the stream, in the order of the exact path (cosine part,
-// sine part).
+// One Box-Muller pair from the stream, drawn in the order of the exact path (cosine part, sine part).
 template <class A>
-GX_HD bool pair(A& ap, uint32_t s1, uint32_t s2, float& c, float& s) {
-    const float u1 = (float)(s1 >> 8u) * (1.0f / 16777216.0f);
-    const float t = (float)(s2 >> 8u) * (gxc::kTwoPi * (1.0f / 16777216.0f));  // = RN(2 pi u2)
+GX_HD bool pair(A& ap, uint32_t& st, float& c, float& s) {
+    st = gx::pcg(st);
+    const float u1 = (float)(st >> 8u) * (1.0f / 16777216.0f);
+    st = gx::pcg(st);
+    const float t = (float)(st >> 8u) * (gxc::kTwoPi * (1.0f / 16777216.0f));  // = RN(2 pi u2)
     float x;
     const float r = ap.radius(u1, x);
     c = r * ap.cos(t);
@@ -150,20 +151,20 @@ struct Point {
 // vc: the ViewConditioned draw against `keep` comes first (exact), and where ap.every(dropped) says so
 // (every lane of a warp) nothing else is computed, as from far away almost no particle is kept: 560k splats,
 // 1280x720, 4 ensembles, distance 60 (0.3 % kept) 12.7 -> 6.8 ms (the exact path of each lane, left at its draw,
-// takes 10.4), 20: 13.4 -> 9.5, 7: 13.9 -> 13.3, 2.5: 10.5 both, with 2x2 subpixels 11.2 -> 11.3. Otherwise straight-line code: the lanes of a
-// warp rarely agree on an early exit.
+// takes 10.4), 20: 13.4 -> 9.5, 7: 13.9 -> 13.3, 2.5: 10.6 both, with 2x2 subpixels 11.2 -> 11.4. Otherwise
+// straight-line code: the lanes of a warp rarely agree on an early exit.
 template <class A>
 GX_HD uint32_t decide(A& ap, const Frame& F, uint32_t flags, bool vc, float keep, uint32_t st, const float* q, Point& P) {
-    const uint32_t s1 = gx::pcg(st), s2 = gx::pcg(s1), s3 = gx::pcg(s2), s4 = gx::pcg(s3);
-    st = s4;
     bool drop = false;
     if (vc) {
-        drop = gx::next_u(&st) >= keep;
+        uint32_t s = gx::pcg(gx::pcg(gx::pcg(gx::pcg(st))));  // past the two pairs
+        drop = gx::next_u(&s) >= keep;
         if (ap.every(drop)) return 0u;
     }
     float uz, uy, ux, jy;
-    bool ok = pair(ap, s1, s2, uz, uy);
-    ok &= pair(ap, s3, s4, ux, jy);  // jy is the pair's spare, used by the jitter
+    bool ok = pair(ap, st, uz, uy);
+    ok &= pair(ap, st, ux, jy);  // jy is the pair's spare, used by the jitter
+    if (vc) st = gx::pcg(st);
     const float X = gx::fma_(q[3], uz, gx::fma_(q[2], uy, gx::fma_(q[1], ux, q[0])));
     const float Y = gx::fma_(q[7], uz, gx::fma_(q[6], uy, gx::fma_(q[5], ux, q[4])));
     const float Z = gx::fma_(q[11], uz, gx::fma_(q[10], uy, gx::fma_(q[9], ux, q[8])));
@@ -173,9 +174,7 @@ GX_HD uint32_t decide(A& ap, const Frame& F, uint32_t flags, bool vc, float keep
     float sx = gx::fma_(X, iz, F.kcx), sy = gx::fma_(Y, iz, F.kcy);
     if (flags & kJitter) {
         float jx, js;
-        const uint32_t s = gx::pcg(st);
-        st = gx::pcg(s);
-        sure &= pair(ap, s, st, jx, js);
+        sure &= pair(ap, st, jx, js);
         sx = gx::fma_(F.sd, jx, sx);
         sy = gx::fma_(F.sd, jy, sy);
     }
